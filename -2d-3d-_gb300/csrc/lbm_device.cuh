@@ -168,6 +168,11 @@ __device__ __forceinline__ T pull_thermal(const Geo& g, int a, int i, int j, int
     return pull_thermal_w<QT, T>(g, a, i, j, k, c, load, [&](int, int d, long long cc) { return load(d, cc); });
 }
 
+// A row that touches no y face and, in 3D, no z face.
+__host__ __device__ __forceinline__ bool row_off_faces(const Geo& g, int j, int k) {
+    return j > 0 && j < g.ny - 1 && (g.nz == 1 || (k > 0 && k < g.nz - 1));
+}
+
 // Row launches.  Interior rows (0 < j < ny-1, and 0 < k < nz-1 in 3D): block (bx, j-1, k-1)
 // holds cells i = bx*blockDim.x + t of row (j, k), so warps start at row starts and every
 // access of a warp is one contiguous run; only x can take a pull source outside the lattice

@@ -515,7 +515,9 @@ namespace fxa {
 // g: geometry whose thermal wall terms are deviations (wall term - 2 wT Tref).
 // PATH: 0 = any cell (the boundary rule where a pull leaves the lattice), 1 = a cell known to
 // touch no face (fixed-offset pulls only), 2 = a face cell (boundary path only), 3 = a cell of
-// an interior row (only x can leave the lattice: pull_flow_xrow / pull_thermal_xrow).
+// an interior row (only x can leave the lattice: pull_flow_xrow / pull_thermal_xrow), 4 = a cell
+// of any row: PATH 3's loads on an interior row, the boundary path's on the others (a warp holds
+// cells of one row, so the choice does not diverge, and only the loads are inside it).
 // I: index type of the cell's own accesses and of PATH 3's pulls (int when every array
 // index fits in 32 bits: half the address arithmetic; the values do not depend on it).
 template <int D, bool FIRST, int PATH = 0, class I = long long>
@@ -537,7 +539,7 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const Fi
         tdev = q60(A.T[c]) - Qb(X.tref);
     } else {
         q60 ts = Qb(0);
-        if (PATH == 3) {
+        if (PATH == 3 || (PATH == 4 && row_off_faces(g, j, k))) {
             auto lf = [&](int a, I cc) { return ldq(fin, a * ni + cc); };
             auto lg = [&](int a, I cc) { return ldq(gin, a * ni + cc); };
 #pragma unroll
@@ -583,7 +585,8 @@ __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const
     q60 d[Q], e[QT], ep[QT], rho, P[3], U[3], B[3], tdev;
     const bool inner = PATH == 1 || (PATH == 0 && aa_inner(g, i, j, k));
     auto lf = [&](int a, long long cc) { return ldq(fin, a * n + cc); };
-    if (PATH == 3) {
+    const bool inrow = PATH == 3 || (PATH == 4 && row_off_faces(g, j, k));
+    if (inrow) {
         auto lfi = [&](int a, I cc) { return ldq(fin, a * ni + cc); };
 #pragma unroll
         for (int a = 0; a < Q; ++a) d[a] = pull_flow_xrow<Q, q60>(g, a, i, ci, lfi);
@@ -603,7 +606,7 @@ __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const
         B[2] = D == 3 ? q60(A.Bz[c]) : Qb(0);
     } else {
         q60 ts = Qb(0);
-        if (PATH == 3) {
+        if (inrow) {
             auto lg = [&](int a, I cc) { return ldq(gin, a * ni + cc); };
 #pragma unroll
             for (int a = 0; a < QT; ++a) {
