@@ -13,9 +13,8 @@ namespace lbm {
 
 using namespace fxa;
 
-// Resident blocks per SM asked of the interior flow kernel: 5 (96 registers, no spill) ran
-// the kernel 8% faster on GB300 than 4 (124 registers) at 256^3 and 384^3, where the warps
-// wait on their loads (long-scoreboard stalls) at half the issue rate; 6 spills.
+// Resident blocks per SM asked of the flow kernels: 5 (96 registers).  GB300, flow half at 128^3 /
+// 256^3: 4 blocks 157 / 1163 us, 5 blocks 146 / 1071 us, 6 blocks (120 B of spill) 145 / 1077 us.
 #ifndef LBM_XFLOW_MIN_BLOCKS
 #define LBM_XFLOW_MIN_BLOCKS 5
 #endif
@@ -223,7 +222,7 @@ __global__ void __launch_bounds__(NT, XfBlocks<NT>::value) k_xfused(Geo g, PhysX
                 for (int jt = j0 - 1; jt <= j1; ++jt) {
                     if (jt < 0 || jt >= ny) continue;
                     const long long c = (long long)i + (long long)nx * ((long long)jt + (long long)ny * pp);
-                    q60 d[Q], e[QT], ep[QT], rho, P[3], U[3], B[3];
+                    q60 d[Q], e[QT], ep[QT], rho, P[3], U[3], B[3], Fl;
                     q60 tdev = Qb(0);
                     if (aa_inner(g, i, jt, pp)) {
 #pragma unroll
@@ -242,7 +241,7 @@ __global__ void __launch_bounds__(NT, XfBlocks<NT>::value) k_xfused(Geo g, PhysX
                             tdev = tdev + e[a];
                         }
                     }
-                    macro<3>(d, tdev, X, rho, P, U);
+                    macro<3>(d, tdev, X, rho, P, U, Fl);
                     B[0] = Qb(F.bin0[c]);
                     B[1] = Qb(F.bin1[c]);
                     B[2] = Qb(F.bin2[c]);
@@ -293,7 +292,7 @@ __global__ void __launch_bounds__(NT, XfBlocks<NT>::value) k_xfused(Geo g, PhysX
             if (act && q >= z0 && q < z1) {
                 for (int j = j0; j < j1; ++j) {
                     const long long c = (long long)i + (long long)nx * ((long long)j + (long long)ny * q);
-                    q60 d[Q], dp[Q], rho, P[3], U[3];
+                    q60 d[Q], dp[Q], rho, P[3], U[3], Fl;
                     if (aa_inner(g, i, j, q)) {
 #pragma unroll
                         for (int a = 0; a < Q; ++a) d[a] = ldq(F.fin, a * n + c - lat_off<Q>(g, a));
@@ -301,9 +300,9 @@ __global__ void __launch_bounds__(NT, XfBlocks<NT>::value) k_xfused(Geo g, PhysX
 #pragma unroll
                         for (int a = 0; a < Q; ++a) d[a] = pull_flow<Q, q60>(g, a, i, j, q, c, lf);
                     }
-                    macro<3>(d, Qb(tst[((q & 1) * TY + (j - j0)) * NT + i]), X, rho, P, U);
+                    macro<3>(d, Qb(tst[((q & 1) * TY + (j - j0)) * NT + i]), X, rho, P, U, Fl);
                     const q60 tnew = Qb((long long)tacc[((q % 3) * TY + (j - j0)) * NT + i]);
-                    collide_3d(d, rho, P, U, tnew, X, dp);
+                    collide_trt_3d(d, rho, P, U, Fl, tnew, X, dp);
 #pragma unroll
                     for (int a = 0; a < Q; ++a) F.fout[a * n + c] = dp[a].s();
                 }

@@ -20,7 +20,8 @@
 //  * Products are 64 x 64 -> 128-bit integer multiplies: of two q60 values (equilibria, the
 //    force, B = u T, 1/rho by Newton's iteration), or of a q60 value with a constant scaled by
 //    2^64 (relaxation rates over the row norms).  Each rounds once, down, by < 2^-60.
-//  * The collision adds the relaxation update in moment space to the populations:
+//  * The first step's collision adds the relaxation update in moment space to the populations
+//    (every further one works on even and odd parts of opposite directions, collide_trt):
 //      f_post = f + M^-1 delta,  delta_i = -s_i (m_i - meq_i) + source_i,
 //    with M^-1 = M^T D^-1 because the rows of the reference's moment matrices are orthogonal
 //    (D holds their squared norms: the reference's divisors 19, 2394, 252, 10, 40, 36, 72, 12,
@@ -122,24 +123,36 @@ __device__ __forceinline__ q60 mulk(q60 a, long long K) {
 #endif
 }
 
-// 1/rho for rho in (1/2, 4): an FP32 reciprocal of the leading bits (24 correct bits), then
-// two Newton steps r <- r + r (1 - rho r) in q60 (48, then beyond 60 bits).
+// Product of two q60 numbers below 2 in magnitude that were scaled by 4 beforehand (sh2), rounded
+// down to q60: the high word of 4a * 4b is the product's bits 60..123, so no low word is needed.
+__device__ __forceinline__ q60 sh2(q60 a) { return Qb((long long)(a.u << 2)); }
+__device__ __forceinline__ q60 mul4(q60 a4, q60 b4) {
+#ifdef __CUDA_ARCH__
+    return Qb(__mul64hi(a4.s(), b4.s()));
+#else
+    return Qb((long long)(((__int128)a4.s() * (__int128)b4.s()) >> 64));
+#endif
+}
+
+// 1/rho for rho in (1/2, 4): an FP32 reciprocal of the leading bits (24 correct bits), then two
+// steps of Newton's iteration r <- r + r (1 - rho r).  The first needs its residual to 2^-52 only
+// and the second's residual fits 32 bits, so both corrections are single 32 x 32 -> 64-bit
+// products; only rho r of the second step is a full product.
 __device__ __forceinline__ q60 recip(q60 rho) {
     float x = (float)(int)(rho.s() >> 32) * 0x1p-28f;
     x = x < 0.5f ? 0.5f : (x > 4.0f ? 4.0f : x);
 #ifdef __CUDA_ARCH__
-    const float r0 = __frcp_rn(x);
-    q60 r = Qb((long long)__float2int_rz(r0 * 0x1p30f) << 30);
+    const unsigned r0 = __float2uint_rz(__frcp_rn(x) * 0x1p30f);
 #else
-    const float r0 = 1.0f / x;
-    q60 r = Qb((long long)(int)(r0 * 0x1p30f) << 30);
+    const unsigned r0 = (unsigned)((1.0f / x) * 0x1p30f);
 #endif
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const q60 e = Qb(kOne) - mul(rho, r);
-        r = r + mul(r, e);
-    }
-    return r;
+    // rho r0 with r0 in units of 2^-30
+    const unsigned long long t = (((rho.u >> 32) * r0) << 2) + (((rho.u & 0xFFFFFFFFULL) * r0) >> 30);
+    const q60 e1 = Qb(kOne) - Qb((long long)t);
+    const q60 r1 = Qb((long long)((unsigned long long)r0 << 30)) +
+                   Qb(((long long)(int)r0 * (long long)(int)(e1.s() >> 8)) >> 22);
+    const q60 e2 = Qb(kOne) - mul(rho, r1);
+    return r1 + Qb(((long long)(int)(r1.s() >> 30) * (long long)(int)e2.s()) >> 30);
 }
 
 __device__ __forceinline__ double quiet_nan() {
@@ -180,6 +193,10 @@ struct PhysX {
     long long x12_n, x12_s;    // -Spi/24, -(1 - Spi/2)/24
     long long x13_n, x13_s;    // -Snu/4, (1 - Snu/2)/4 (times u F_y, w F_y)
     long long m_n;             // -Sm/8
+    // steady-state collision in even and odd parts (collide_trt): rates over the weights
+    long long s36, s72;        // 3D Snu/36 (axis), 2D Snu/18 (axis); Snu/72 (diagonals)
+    long long sq12, sqg;       // Sq/12; 3D Sq/120, 2D Sq/24 (times F_y minus the lagged force)
+    long long h12, h6;         // 1/12, 1/6 (3D 1/12): force and v F_y shares
     // 2D flow
     long long e2_n, e2_s;      // -Snu/36, (6 - 3 Snu)/36
     long long q2_n, q2_s;      // -Sq/12, -(1 - Sq/2)/12
@@ -243,6 +260,12 @@ inline bool make_physx(const lbm_params& p, const lbm_constants& c, PhysX& X) {
         ok = ok && fx_const(Snu / 4, 0, X.x7_n) && fx_const((2 - Snu) / 4, 0, X.x7_s);
         ok = ok && fx_const((1 - Snu / 2) / 4, 0, X.x8_s);
     }
+    // collide_trt needs one rate for the even moments and one for the odd ones, as
+    // commondata sets them (2DRB.F90:83-84, 3DRB.F90:92-97)
+    if (d3) ok = ok && c.Se == c.Snu && c.Seps == c.Snu && c.Spi == c.Snu && c.Sm == c.Sq;
+    ok = ok && fx_const(d3 ? Snu / 36 : Snu / 18, 0, X.s36) && fx_const(Snu / 72, 0, X.s72);
+    ok = ok && fx_const(Sq / 12, 0, X.sq12) && fx_const(d3 ? Sq / 120 : Sq / 24, 0, X.sqg);
+    ok = ok && fx_const(1.0L / 12, 0, X.h12) && fx_const(d3 ? 1.0L / 12 : 1.0L / 6, 0, X.h6);
     const long double Qk = c.Qk, Qnu = c.Qnu, SG = c.SG;
     // a_T of the thermal equilibrium moment: -3/4 (3D), -2/3 (2D), paraA in the legacy scheme
     const long double aT = p.legacy_thermal ? (long double)c.paraA : (d3 ? -0.75L : -2.0L / 3);
@@ -270,29 +293,165 @@ namespace fxa {
 // 2D: the force stored by the collision, lag = F_y), u = P / rho.
 // ------------------------------------------------------------------------------------
 template <int D>
-__device__ __forceinline__ void macro(const q60* d, q60 lag, const PhysX& X, q60& rho, q60* P, q60* U) {
+__device__ __forceinline__ void macro(const q60* d, q60 lag, const PhysX& X, q60& rho, q60* P, q60* U, q60& F) {
     if (D == 2) {
         rho = Qb(kOne) + d[0] + d[1] + d[2] + d[3] + d[4] + d[5] + d[6] + d[7] + d[8];
-        P[0] = d[1] - d[3] + d[5] - d[6] - d[7] + d[8];
-        P[1] = d[2] - d[4] + d[5] + d[6] - d[7] - d[8] + half(lag);
+        const q60 r5 = d[5] - d[7], r8 = d[8] - d[6];
+        F = lag;
+        P[0] = d[1] - d[3] + r5 + r8;
+        P[1] = d[2] - d[4] + r5 - r8 + half(F);
         P[2] = Qb(0);
     } else {
         q60 s = d[0];
 #pragma unroll
         for (int a = 1; a < 19; ++a) s = s + d[a];
         rho = Qb(kOne) + s;
-        const q60 Fy = mul(rho, mulk<0>(lag, X.gb));
-        P[0] = d[1] - d[2] + d[7] - d[8] + d[9] - d[10] + d[11] - d[12] + d[13] - d[14];
-        P[1] = d[3] - d[4] + d[7] + d[8] - d[9] - d[10] + d[15] - d[16] + d[17] - d[18] + half(Fy);
-        P[2] = d[5] - d[6] + d[11] + d[12] - d[13] - d[14] + d[15] + d[16] - d[17] - d[18];
+        F = mul(rho, mulk<0>(lag, X.gb));
+        const q60 r7 = d[7] - d[10], r9 = d[9] - d[8], r11 = d[11] - d[14], r13 = d[13] - d[12], r15 = d[15] - d[18],
+                  r17 = d[17] - d[16];
+        P[0] = d[1] - d[2] + r7 + r9 + r11 + r13;
+        P[1] = d[3] - d[4] + r7 - r9 + r15 + r17 + half(F);
+        P[2] = d[5] - d[6] + r11 - r13 + r15 - r17;
     }
-    const q60 r = recip(rho);
-    U[0] = mul(P[0], r);
-    U[1] = mul(P[1], r);
-    U[2] = D == 3 ? mul(P[2], r) : Qb(0);
+    const q60 r = sh2(recip(rho));
+    U[0] = mul4(sh2(P[0]), r);
+    U[1] = mul4(sh2(P[1]), r);
+    U[2] = D == 3 ? mul4(sh2(P[2]), r) : Qb(0);
 }
 
 // ------------------------------------------------------------------------------------
+// Steady-state collision (both dimensions): the MRT collision with Guo forcing below, for rho, P
+// and U of this cell's own macro step.  All even moments relax at one rate s (Snu) and all odd
+// ones at one rate q (Sq), and the equilibrium moments are those of the quadratic equilibrium,
+// so the relaxation acts on the even and odd parts of each pair of opposite directions a, -a
+// of weight w (two relaxation times):
+//   even: s/2 (d_a + d_-a - 2 feq+ + S+) with S+ = w (-3 v F + 9 (e.u) e_y F), times 1/w:
+//         s w/2 ((d_a + d_-a)/w - (2 dr - 3 rho u^2 + 3 v F) - 9 ((e.P)(e.u) - (e.u) e_y F));
+//   odd:  q/2 (d_a - d_-a - 6 w e.j), j = sum e d: the momentum itself is conserved.
+// What the force adds does not depend on the rates: S+, and 3 w e_y F to the odd parts, but for
+// the q/60 (F - F_lag)-sized share of the odd fourth-order moment whose equilibrium holds the
+// lagged force (sqg).  The rest population takes minus the sum of the even changes and the axis
+// pairs minus the diagonal pairs' odd changes, so mass and momentum are conserved to the last bit.
+// Against the moment-space form: 19 instead of 30 products with constants in 3D, a third of the
+// macro step's products (recip, mul4) and half the additions.  GB300, flow half of the step at
+// 256^3: 1.07 ms instead of 1.17 (85% instead of 78% of the copy rate on its 368 B per cell), so
+// that the half is bound by HBM where it waited on its own instructions before.
+// ------------------------------------------------------------------------------------
+__device__ __forceinline__ q60 collide_trt_2d(const q60* d, q60 rho, const q60* P, const q60* U, q60 F, q60 tdev,
+                                              const PhysX& X, q60* dp) {
+    const q60 dr = rho - Qb(kOne);
+    const q60 Fy = mul(rho, mulk<0>(tdev, X.gb));
+    const q60 u4 = sh2(U[0]), v4 = sh2(U[1]), p4 = sh2(P[0]), F4 = sh2(Fy);
+    const q60 ruu = mul4(p4, u4), rvv = mul4(sh2(P[1]), v4), ruv = mul4(p4, v4);
+    const q60 vF = mul4(v4, F4), uF = mul4(u4, F4);
+    const q60 base = 2 * dr - 3 * (ruu + rvv - vF);
+    const q60 bx = base + 9 * ruu, by = base + 9 * (rvv - vF), bxy = bx + by - base, cxy = 9 * (2 * ruv - uF);
+    const q60 h = mulk<0>(vF, X.h6), u1 = Qb(uF.s() >> 2);
+    const q60 e1 = mulk<0>(9 * (d[1] + d[3]) - bx, X.s36) + 2 * h;
+    const q60 e2 = mulk<0>(9 * (d[2] + d[4]) - by, X.s36) - 4 * h;
+    const q60 e5 = mulk<0>(36 * (d[5] + d[7]) - bxy - cxy, X.s72) - h - u1;
+    const q60 e6 = mulk<0>(36 * (d[6] + d[8]) - bxy + cxy, X.s72) - h + u1;
+    const q60 jx = P[0], jy = P[1] - half(F);
+    const q60 k5 = mulk<0>(6 * (d[5] - d[7]) - (jx + jy), X.sq12), k8 = mulk<0>(6 * (d[8] - d[6]) - (jx - jy), X.sq12);
+    const q60 b = mulk<0>(Fy, X.h12), G = mulk<0>(Fy - F, X.sqg);
+    const q60 y1 = half(Fy - 4 * b) - 2 * G, yd = b + G;
+    const q60 o1 = -(k5 + k8), o2 = k8 - k5 - y1, o5 = k5 - yd, o8 = k8 + yd;
+    dp[0] = d[0] + 2 * (e1 + e2 + e5 + e6);
+    dp[1] = d[1] - e1 - o1;
+    dp[3] = d[3] - e1 + o1;
+    dp[2] = d[2] - e2 - o2;
+    dp[4] = d[4] - e2 + o2;
+    dp[5] = d[5] - e5 - o5;
+    dp[7] = d[7] - e5 + o5;
+    dp[8] = d[8] - e6 - o8;
+    dp[6] = d[6] - e6 + o8;
+    return Fy;
+}
+
+__device__ __forceinline__ void collide_trt_3d(const q60* d, q60 rho, const q60* P, const q60* U, q60 F, q60 tdev,
+                                               const PhysX& X, q60* dp) {
+    const q60 dr = rho - Qb(kOne);
+    const q60 Fy = mul(rho, mulk<0>(tdev, X.gb));
+    const q60 u4 = sh2(U[0]), v4 = sh2(U[1]), w4 = sh2(U[2]), F4 = sh2(Fy);
+    const q60 vF = mul4(v4, F4), uF = mul4(u4, F4), wF = mul4(w4, F4);
+    q60 bx, by, bz, base, cxy, cyz, cxz;
+    {
+        const q60 px = sh2(P[0]), py = sh2(P[1]), pz = sh2(P[2]);
+        const q60 xx = mul4(px, u4), yy = mul4(py, v4) - vF, zz = mul4(pz, w4);
+        base = 2 * dr - 3 * (xx + yy + zz);
+        bx = base + 9 * xx;
+        by = base + 9 * yy;
+        bz = base + 9 * zz;
+        cxy = 9 * (2 * mul4(px, v4) - uF);
+        cyz = 9 * (2 * mul4(py, w4) - wF);
+        cxz = 18 * mul4(px, w4);
+    }
+    const q60 h = mulk<0>(vF, X.h12), h2 = 2 * h, u1 = Qb(uF.s() >> 2), w1 = Qb(wF.s() >> 2);
+    const q60 b = mulk<0>(Fy, X.h12);
+    const q60 jx = P[0], jy = P[1] - half(F), jz = P[2];
+    const q60 G = mulk<0>(Fy - F, X.sqg);
+    const q60 yd = b + G;
+    q60 ox, oy = half(Fy - 8 * b) - 4 * G, oz, es;
+    {  // xy diagonals: 7 and 10, 9 and 8
+        const q60 bb = bx + by - base;
+        const q60 e7 = mulk<0>(36 * (d[7] + d[10]) - bb - cxy, X.s72) - h2 - u1;
+        const q60 e9 = mulk<0>(36 * (d[9] + d[8]) - bb + cxy, X.s72) - h2 + u1;
+        const q60 k7 = mulk<0>(6 * (d[7] - d[10]) - (jx + jy), X.sq12);
+        const q60 k9 = mulk<0>(6 * (d[9] - d[8]) - (jx - jy), X.sq12);
+        es = e7 + e9;
+        ox = k7 + k9;
+        oy = oy + k7 - k9;
+        const q60 o7 = k7 - yd, o9 = k9 + yd;
+        dp[7] = d[7] - e7 - o7;
+        dp[10] = d[10] - e7 + o7;
+        dp[9] = d[9] - e9 - o9;
+        dp[8] = d[8] - e9 + o9;
+    }
+    {  // xz diagonals: 11 and 14, 13 and 12
+        const q60 bb = bx + bz - base;
+        const q60 e11 = mulk<0>(36 * (d[11] + d[14]) - bb - cxz, X.s72) + h;
+        const q60 e13 = mulk<0>(36 * (d[13] + d[12]) - bb + cxz, X.s72) + h;
+        const q60 k11 = mulk<0>(6 * (d[11] - d[14]) - (jx + jz), X.sq12);
+        const q60 k13 = mulk<0>(6 * (d[13] - d[12]) - (jx - jz), X.sq12);
+        es = es + e11 + e13;
+        ox = ox + k11 + k13;
+        oz = k11 - k13;
+        dp[11] = d[11] - e11 - k11;
+        dp[14] = d[14] - e11 + k11;
+        dp[13] = d[13] - e13 - k13;
+        dp[12] = d[12] - e13 + k13;
+    }
+    {  // yz diagonals: 15 and 18, 17 and 16
+        const q60 bb = by + bz - base;
+        const q60 e15 = mulk<0>(36 * (d[15] + d[18]) - bb - cyz, X.s72) - h2 - w1;
+        const q60 e17 = mulk<0>(36 * (d[17] + d[16]) - bb + cyz, X.s72) - h2 + w1;
+        const q60 k15 = mulk<0>(6 * (d[15] - d[18]) - (jy + jz), X.sq12);
+        const q60 k17 = mulk<0>(6 * (d[17] - d[16]) - (jy - jz), X.sq12);
+        es = es + e15 + e17;
+        oy = oy + k15 + k17;
+        oz = oz + k15 - k17;
+        const q60 o15 = k15 - yd, o17 = k17 - yd;
+        dp[15] = d[15] - e15 - o15;
+        dp[18] = d[18] - e15 + o15;
+        dp[17] = d[17] - e17 - o17;
+        dp[16] = d[16] - e17 + o17;
+    }
+    // axis pairs: odd changes -ox, -oy, -oz
+    const q60 e1 = mulk<0>(18 * (d[1] + d[2]) - bx, X.s36) + h2;
+    const q60 e3 = mulk<0>(18 * (d[3] + d[4]) - by, X.s36) - 2 * h2;
+    const q60 e5 = mulk<0>(18 * (d[5] + d[6]) - bz, X.s36) + h2;
+    dp[0] = d[0] + 2 * (es + e1 + e3 + e5);
+    dp[1] = d[1] - e1 + ox;
+    dp[2] = d[2] - e1 - ox;
+    dp[3] = d[3] - e3 + oy;
+    dp[4] = d[4] - e3 - oy;
+    dp[5] = d[5] - e5 + oz;
+    dp[6] = d[6] - e5 - oz;
+}
+
+// ------------------------------------------------------------------------------------
+// First step after `initial` or a state load: rho and U are the loaded ones, which need not be
+// those of the populations, so the collision keeps the reference's moment space.
 // D2Q9 MRT collision with Guo forcing (2DRB.F90:688-759), F = (0, F_y).  rho, P = rho u, U,
 // tdev = T - Tref; returns F_y (the force the reference stores, 2DRB.F90:718-719).
 // ------------------------------------------------------------------------------------
@@ -526,7 +685,7 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const Fi
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     const I ni = (I)g.ncell, ci = (I)c;
-    q60 d[Q], dp[Q], rho, P[3], U[3], tdev;
+    q60 d[Q], dp[Q], rho, P[3], U[3], F = Qb(0), tdev;
     if (FIRST) {
 #pragma unroll
         for (int a = 0; a < Q; ++a) d[a] = q60(A.f[a * n + c]) - Qb(X.w[a]);
@@ -563,13 +722,15 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const Fi
             for (int a = 0; a < QT; ++a) ts = ts + pull_thermal<QT, q60>(g, a, i, j, k, c, lg);
         }
         tdev = ts;
-        macro<D>(d, Qb(A.xlag[ci]), X, rho, P, U);
+        macro<D>(d, Qb(A.xlag[ci]), X, rho, P, U, F);
     }
     if (D == 2) {
-        const q60 Fy = collide_2d(d, rho, P, U, tdev, X, dp);
+        const q60 Fy = FIRST ? collide_2d(d, rho, P, U, tdev, X, dp) : collide_trt_2d(d, rho, P, U, F, tdev, X, dp);
         A.xlag[ci] = Fy.s();
-    } else {
+    } else if (FIRST) {
         collide_3d(d, rho, P, U, tdev, X, dp);
+    } else {
+        collide_trt_3d(d, rho, P, U, F, tdev, X, dp);
     }
 #pragma unroll
     for (int a = 0; a < Q; ++a) fout[a * ni + ci] = dp[a].s();
@@ -582,7 +743,7 @@ __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     const I ni = (I)g.ncell, ci = (I)c;
-    q60 d[Q], e[QT], ep[QT], rho, P[3], U[3], B[3], tdev;
+    q60 d[Q], e[QT], ep[QT], rho, P[3], U[3], B[3], F, tdev;
     const bool inner = PATH == 1 || (PATH == 0 && aa_inner(g, i, j, k));
     auto lf = [&](int a, long long cc) { return ldq(fin, a * n + cc); };
     const bool inrow = PATH == 3 || (PATH == 4 && row_off_faces(g, j, k));
@@ -632,7 +793,7 @@ __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const
         B[1] = Qb(A.xb1[ci]);
         B[2] = D == 3 ? Qb(A.xb2[ci]) : Qb(0);
     }
-    macro<D>(d, D == 2 ? Qb(A.xlag[ci]) : tdev, X, rho, P, U);
+    macro<D>(d, D == 2 ? Qb(A.xlag[ci]) : tdev, X, rho, P, U, F);
     if (D == 2) {
         collideT_2d(e, U, tdev, B, X, ep);
     } else {
@@ -658,7 +819,7 @@ __device__ __forceinline__ void materialize_cell(const Geo& g, const PhysX& X, c
                                                  int k) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    q60 d[Q], rho, P[3], U[3];
+    q60 d[Q], rho, P[3], U[3], F;
     auto lf = [&](int a, long long cc) { return ldq(fin, a * n + cc); };
     auto lg = [&](int a, long long cc) { return ldq(gin, a * n + cc); };
     q60 ts = Qb(0);
@@ -674,7 +835,7 @@ __device__ __forceinline__ void materialize_cell(const Geo& g, const PhysX& X, c
         A.g[a * n + c] = to_double(e + Qb(X.wt[a]));
     }
     const q60 lag = Qb(A.xlag[c]);
-    macro<D>(d, lag, X, rho, P, U);
+    macro<D>(d, lag, X, rho, P, U, F);
     const long long lim = kOne / 2;
     const bool bad = rho.s() <= lim || rho.s() >= 4 * kOne || U[0].s() > lim || U[0].s() < -lim ||
                      U[1].s() > lim || U[1].s() < -lim || U[2].s() > lim || U[2].s() < -lim;
