@@ -13,6 +13,7 @@
 
 #include "lbm_fast.h"
 #include "lbm_fast_cells.cuh"
+#include "lbm_fast_duo.cuh"
 #include "lbm_fast_pairs.cuh"
 
 namespace lbm {
@@ -28,6 +29,7 @@ static FastArgs<S> args_for(const FastState& F, int bin, int bout, int lin, int 
     a.lag_in = F.L[lin];
     a.lag_out = F.L[lout];
     a.tick = F.tick;
+    a.ticks = F.tick;
     return a;
 }
 
@@ -85,6 +87,26 @@ __global__ void __launch_bounds__(128, (OneCellBlocks<S, true>::value)) k_fast_t
     int i, j, k;
     if (!fcell_i<I>(g, c, i, j, k)) return;
     thermal_cell_2k<D, FIRST, S, true, I>(g, P, A, fin, gin, gout, c, i, j, k);
+}
+
+// Two cells per thread, 32 apart (lbm_fast_duo.cuh): the default of the steady-state step.  Six
+// (flow) and seven (thermal) resident blocks per SM: 80 and 72 registers.  GB300, us per step at
+// 256^3 with 5 / 6 / 7 / 8 blocks of both: FP32 818 / 814 / 814 / 824, FP16 659 / 630 / 642 / 660.
+// Against one cell per thread with branches in its pulls: 256^3 FP32 979 / 810 (6.5 TB/s on 313 B
+// per cell: bound by HBM), FP16 955 / 607; 96^3 FP16 89 / 34; 2D 2050x1025 FP32 75 / 63.
+template <int D, class S>
+__global__ void __launch_bounds__(128, 6) k_fast_flow_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
+                                                       const S* __restrict__ gin, S* __restrict__ fout) {
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+    const unsigned long long tick = sizeof(S) == 2 || one ? flow_tick(A.ticks, one) : 0ULL;
+    flow_duo_2k<D, S>(g, P, A, fin, gin, fout, duo_cells(g), tick);
+}
+template <int D, class S>
+__global__ void __launch_bounds__(128, 7) k_fast_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
+                                                          const S* __restrict__ gin, S* __restrict__ gout) {
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+    const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
+    thermal_duo_2k<D, S>(g, P, A, fin, gin, gout, duo_cells(g), tick);
 }
 
 // Paired form of the two kernels (lbm_fast_pairs.cuh): thread (x, y) of a block holds the
@@ -169,19 +191,27 @@ __global__ void __launch_bounds__(128) k_fast_thermal_facerows(Geo g, PhysF P, F
     thermal_cell_2k<D, false, S, false>(g, P, A, fin, gin, gout, c, i, j, k);
 }
 
-// idx32: every array index fits in 32 bits.  Measured on GB300 (256^3 and 384^3): 32-bit
-// indices speed up both FP16 kernels (2%) and the FP32 thermal kernel (1-1.5%); the FP32
-// flow kernel takes 64 registers instead of 56 with them and runs 5-6% slower, so it keeps
-// 64-bit indices.
+// One cell per thread: the first step (module arrays), and lattices whose indices need 64 bits.
+// idx32: every array index fits in 32 bits.
 template <int D, bool FIRST, class S>
 static void one_cell_step(bool idx32, unsigned blocks, const Geo& g, const PhysF& pf, const FastArgs<S>& Af,
                           const FastArgs<S>& At, const S* fin, const S* gin, S* fout, S* gout, cudaStream_t s, bool fl,
                           bool th) {
-    const bool flow32 = idx32 && sizeof(S) == 2;
-    if (fl && flow32) k_fast_flow<D, FIRST, S, int><<<blocks, 128, 0, s>>>(g, pf, Af, fin, gin, fout);
-    else if (fl) k_fast_flow<D, FIRST, S, long long><<<blocks, 128, 0, s>>>(g, pf, Af, fin, gin, fout);
-    if (th && idx32) k_fast_thermal<D, FIRST, S, int><<<blocks, 128, 0, s>>>(g, pf, At, fout, gin, gout);
-    else if (th) k_fast_thermal<D, FIRST, S, long long><<<blocks, 128, 0, s>>>(g, pf, At, fout, gin, gout);
+    if (FIRST && idx32) {
+        if (fl) k_fast_flow<D, FIRST, S, int><<<blocks, 128, 0, s>>>(g, pf, Af, fin, gin, fout);
+        if (th) k_fast_thermal<D, FIRST, S, int><<<blocks, 128, 0, s>>>(g, pf, At, fout, gin, gout);
+        return;
+    }
+    if (fl) k_fast_flow<D, FIRST, S, long long><<<blocks, 128, 0, s>>>(g, pf, Af, fin, gin, fout);
+    if (th) k_fast_thermal<D, FIRST, S, long long><<<blocks, 128, 0, s>>>(g, pf, At, fout, gin, gout);
+}
+
+template <int D, class S>
+static void duo_step(const Geo& g, const PhysF& pf, const FastArgs<S>& Af, const FastArgs<S>& At, const S* fin,
+                     const S* gin, S* fout, S* gout, cudaStream_t s, bool fl, bool th) {
+    const unsigned nb2 = (unsigned)((g.ncell + 255) / 256);
+    if (fl) k_fast_flow_duo<D, S><<<nb2, 128, 0, s>>>(g, pf, Af, fin, gin, fout);
+    if (th) k_fast_thermal_duo<D, S><<<nb2, 128, 0, s>>>(g, pf, At, fout, gin, gout);
 }
 
 template <int D, class S>
@@ -275,6 +305,7 @@ static inline unsigned nb(long long n, int bs) { return (unsigned)((n + bs - 1) 
 
 PhysF fast_physf(const FastState& F, const PhysC& P) {
     PhysF pf = to_physf(P);
+    steady_constants(P, F.dim, pf);
     pf.sr = (F.sr && F.precision == LBM_FP16) ? 1 : 0;
     return pf;
 }
@@ -283,13 +314,9 @@ void fast_tick(FastState& F, cudaStream_t s) { k_tick<<<1, 1, 0, s>>>(F.tick); }
 
 int fast_allocate(FastState& F, const lbm_params& p, const Geo& g, const AllocFn& alloc) {
     F.precision = p.precision;
-    // Measured on GB300 (3D cubes 128^3 and 384^3; 2D 256 x 128 to 4096 x 2048): with the
-    // boundary tests confined to the face cells, one cell per thread is the fastest form
-    // for 3D in both storage types (FP16 17.3 G cell updates/s at 384^3 against 13.0 G for
-    // the staged rows) and for 2D FP16; 2D FP32 is fastest with two cells per thread.  The
-    // staged and paired forms stay selectable (LBM_OPT_STAGED, LBM_OPT_PAIRS).
+    // x-adjacent pairs and staged rows on request (LBM_OPT_PAIRS, LBM_OPT_STAGED)
     F.tma = false;
-    F.pairs = p.dim == 2 && p.precision == LBM_FP32;
+    F.pairs = false;
     F.dim = p.dim;
     F.q = p.dim == 3 ? 19 : 9;
     F.qt = p.dim == 3 ? 7 : 5;
@@ -308,8 +335,8 @@ int fast_allocate(FastState& F, const lbm_params& p, const Geo& g, const AllocFn
     }
     if ((st = alloc((void**)&F.err, sizeof(int))) != LBM_OK) return st;
     if (cudaMemset(F.err, 0, sizeof(int)) != cudaSuccess) return LBM_ERR_CUDA;
-    if ((st = alloc((void**)&F.tick, sizeof(unsigned long long))) != LBM_OK) return st;
-    if (cudaMemset(F.tick, 0, sizeof(unsigned long long)) != cudaSuccess) return LBM_ERR_CUDA;
+    if ((st = alloc((void**)&F.tick, 2 * sizeof(unsigned long long))) != LBM_OK) return st;
+    if (cudaMemset(F.tick, 0, 2 * sizeof(unsigned long long)) != cudaSuccess) return LBM_ERR_CUDA;
     F.sr = p.precision == LBM_FP16;
     if (F.aa) {
         // one array each, which is also the module array; the lag fields are read and
@@ -405,7 +432,8 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
     const unsigned blocks = nb(g.ncell, 128);
     const bool paired = F.pairs && g.nx % 2 == 0;
     const bool rows = F.rows && !paired && row_launch_supported(g);
-    const bool idx32 = !F.wide && (long long)F.q * g.ncell < (1LL << 31);
+    const bool idx32 = !F.wide && (long long)F.q * g.ncell < (1LL << 31) - 64;
+    bool ticked = false;  // the step's kernels advance the step counter themselves
     dim3 pgrid, pblock;
     pair_launch(g, pgrid, pblock);
     F.ahead = false;
@@ -427,8 +455,11 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
                 if (th) k_fast_thermal_pair<2, S><<<pgrid, pblock, 0, s>>>(g, pf, At, fout, gin, gout);
             } else if (rows) {
                 rows_step<2, S>(g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
+            } else if (idx32) {
+                duo_step<2, S>(g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
+                ticked = true;
             } else {
-                one_cell_step<2, false, S>(idx32, blocks, g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
+                one_cell_step<2, false, S>(false, blocks, g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
             }
         } else {
             if (first) {
@@ -438,13 +469,16 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
                 if (th) k_fast_thermal_pair<3, S><<<pgrid, pblock, 0, s>>>(g, pf, At, fout, gin, gout);
             } else if (rows) {
                 rows_step<3, S>(g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
+            } else if (idx32) {
+                duo_step<3, S>(g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
+                ticked = true;
             } else {
-                one_cell_step<3, false, S>(idx32, blocks, g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
+                one_cell_step<3, false, S>(false, blocks, g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
             }
         }
     });
     if (part != 0) {
-        fast_tick(F, s);
+        if (!ticked) fast_tick(F, s);
         F.cur = nxt;
         F.fused_valid = true;
     }

@@ -41,9 +41,9 @@ struct FastState {
     bool ahead = false;         // single-kernel phase: F[cur^1] already holds f_post_{N+1}
     bool single_kernel = false; // one-launch fused step (lbm_fused.cu); off: the two-kernel step is faster today
     int kchunk = 16;            // z planes per block of the fused kernel (3D)
-    // Form of the non-first two-kernel step, chosen by fast_allocate from GB300 timings:
-    // one cell per thread, except two cells per thread for 2D FP32; staged rows
-    // (lbm_fast_tma.cu) on request.
+    // Form of the non-first two-kernel step: two cells per thread with packed arithmetic
+    // (lbm_fast_duo.cuh) where 32-bit indices fit; x-adjacent pairs, staged rows
+    // (lbm_fast_tma.cu) or row launches on request.
     bool pairs = false;
     bool tma = false;
     bool rows = false;          // interior-row and face-row launches (LBM_OPT_ROWS)
@@ -55,7 +55,7 @@ struct FastState {
     AAState AA;
     // FP16 storage rounds new populations stochastically (lbm_fast_math.cuh, storeS), with
     // random bits keyed on this device step counter (steps since initial; continuation
-    // records keep it).
+    // records keep it).  tick[1]: its copy for the thermal kernels of lbm_fast_duo.cuh.
     bool sr = false;
     unsigned long long* tick = nullptr;
 };

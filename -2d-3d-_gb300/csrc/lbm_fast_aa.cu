@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(128) k_aa_flow_p(Geo g, PhysF P, FastArgs<S> A
     if (!aa_pair_cell(g, c0, i0, j, k)) return;
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    float d0[Q], d1[Q];
+    f2 d[Q];
     if (ODD) {
         auto lf = [&](int b, long long cc) { return ldA(f, Lat<Q>::opp(b) * n + cc); };
         auto w0 = [&](int ax, int b, long long) {
@@ -304,56 +304,36 @@ __global__ void __launch_bounds__(128) k_aa_flow_p(Geo g, PhysF P, FastArgs<S> A
 #pragma unroll
         for (int a = 0; a < Q; ++a) {
             const float2 v = swp_pull2<Q, false, S, true>(g, f, a, i0, j, k, c0, n, lf, w0, w1);
-            d0[a] = v.x;
-            d1[a] = v.y;
+            d[a] = make_f2(v.x, v.y);
         }
     } else {
 #pragma unroll
         for (int a = 0; a < Q; ++a) {
             const float2 v = ld2<S, true>(f, a * n + c0);
-            d0[a] = v.x;
-            d1[a] = v.y;
+            d[a] = make_f2(v.x, v.y);
         }
     }
-    float ts0 = 0.0f, ts1 = 0.0f;
+    f2 ts = make_f2(0.0f, 0.0f);
     if (gpar) {
         auto lg = [&](int b, long long cc) { return ldS(gs, Lat<QT>::opp(b) * n + cc); };
         auto wd = [&](int, int b, long long cc) { return lg(b, cc); };
 #pragma unroll
         for (int a = 0; a < QT; ++a) {
             const float2 e = swp_pull2<QT, true, S, false>(g, gs, a, i0, j, k, c0, n, lg, wd, wd);
-            ts0 += e.x;
-            ts1 += e.y;
+            ts = vadd(ts, make_f2(e.x, e.y));
         }
     } else {
 #pragma unroll
         for (int a = 0; a < QT; ++a) {
             const float2 e = loc_thermal2<QT, S, false>(g, gs, a, i0, j, k, c0, n, graw != 0);
-            ts0 += e.x;
-            ts1 += e.y;
+            ts = vadd(ts, make_f2(e.x, e.y));
         }
     }
     const float2 lag = ld2<float, true>(A.lag_in, c0);
-    float dp0[Q], dp1[Q], Fy0, Fy1;
-    {
-        const float T = ts0 + P.Tref;
-        float dr, rho, u, v, w = 0.0f, Fm;
-        fmacro<D>(d0, lag.x, P, dr, rho, u, v, w, Fm);
-        Fy0 = rho * P.gBeta * (T - P.Tref);
-        if (D == 2) fcollide_2d(d0, dr, rho, u, v, Fy0, P, dp0);
-        else fcollide_3d(d0, dr, rho, u, v, w, Fy0, P, dp0);
-    }
-    {
-        const float T = ts1 + P.Tref;
-        float dr, rho, u, v, w = 0.0f, Fm;
-        fmacro<D>(d1, lag.y, P, dr, rho, u, v, w, Fm);
-        Fy1 = rho * P.gBeta * (T - P.Tref);
-        if (D == 2) fcollide_2d(d1, dr, rho, u, v, Fy1, P, dp1);
-        else fcollide_3d(d1, dr, rho, u, v, w, Fy1, P, dp1);
-    }
-    if (D == 2) stf2(A.lag_out, c0, Fy0, Fy1);
+    const f2 Fy = steady_flow<D>(d, steady_lag<D>(make_f2(lag.x, lag.y), P), ts, P);
+    if (D == 2) stf2(A.lag_out, c0, f2_lo(Fy), f2_hi(Fy));
     S h0[Q], h1[Q];
-    round_pair<Q>(dp0, dp1, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 0), sr_seed(*A.tick, c0 + 1, 0));
+    round_pair<Q>(d, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 0), sr_seed(*A.tick, c0 + 1, 0));
     if (ODD) {
 #pragma unroll
         for (int a = 0; a < Q; ++a) push2<Q, false, S>(g, f, a, i0, j, k, c0, n, h0[a], h1[a]);
@@ -371,25 +351,22 @@ __global__ void __launch_bounds__(128) k_aa_thermal_p(Geo g, PhysF P, FastArgs<S
     if (!aa_pair_cell(g, c0, i0, j, k)) return;
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    float d0[Q], d1[Q], G0[QT], G1[QT];
+    f2 d[Q], e[QT];
     if (fpar) {
         auto lf = [&](int b, long long cc) { return ldS(fs, Lat<Q>::opp(b) * n + cc); };
         auto wd = [&](int, int b, long long cc) { return lf(b, cc); };
 #pragma unroll
         for (int a = 0; a < Q; ++a) {
             const float2 v = swp_pull2<Q, false, S, false>(g, fs, a, i0, j, k, c0, n, lf, wd, wd);
-            d0[a] = v.x;
-            d1[a] = v.y;
+            d[a] = make_f2(v.x, v.y);
         }
     } else {
 #pragma unroll
         for (int a = 0; a < Q; ++a) {
             const float2 v = ld2<S, false>(fs, a * n + c0);
-            d0[a] = v.x;
-            d1[a] = v.y;
+            d[a] = make_f2(v.x, v.y);
         }
     }
-    float ts0 = 0.0f, ts1 = 0.0f;
     if (ODD) {
         auto lg = [&](int b, long long cc) { return ldA(gg, Lat<QT>::opp(b) * n + cc); };
         auto w0 = [&](int ax, int b, long long) {
@@ -400,53 +377,19 @@ __global__ void __launch_bounds__(128) k_aa_thermal_p(Geo g, PhysF P, FastArgs<S
         };
 #pragma unroll
         for (int a = 0; a < QT; ++a) {
-            const float2 e = swp_pull2<QT, true, S, true>(g, gg, a, i0, j, k, c0, n, lg, w0, w1);
-            G0[a] = e.x + wT<QT>(P, a) * P.Tref;
-            G1[a] = e.y + wT<QT>(P, a) * P.Tref;
-            ts0 += G0[a];
-            ts1 += G1[a];
+            const float2 v = swp_pull2<QT, true, S, true>(g, gg, a, i0, j, k, c0, n, lg, w0, w1);
+            e[a] = make_f2(v.x, v.y);
         }
     } else {
 #pragma unroll
         for (int a = 0; a < QT; ++a) {
-            const float2 e = loc_thermal2<QT, S, true>(g, gg, a, i0, j, k, c0, n, graw != 0);
-            G0[a] = e.x + wT<QT>(P, a) * P.Tref;
-            G1[a] = e.y + wT<QT>(P, a) * P.Tref;
-            ts0 += G0[a];
-            ts1 += G1[a];
+            const float2 v = loc_thermal2<QT, S, true>(g, gg, a, i0, j, k, c0, n, graw != 0);
+            e[a] = make_f2(v.x, v.y);
         }
     }
-    const float2 bx = ld2<float, true>(A.Bin0, c0), by = ld2<float, true>(A.Bin1, c0);
-    const float2 bz = D == 3 ? ld2<float, true>(A.Bin2, c0) : make_float2(0.0f, 0.0f);
-    const float2 lag = D == 2 ? ld2<float, true>(A.lag_in, c0) : make_float2(0.0f, 0.0f);
-    float GP0[QT], GP1[QT];
-    float Bx0 = bx.x, By0 = by.x, Bz0 = bz.x, Bx1 = bx.y, By1 = by.y, Bz1 = bz.y;
-    {
-        float dr, rho, u, v, w, Fy;
-        fmacro<D>(d0, D == 2 ? lag.x : ts0, P, dr, rho, u, v, w, Fy);
-        if (D == 2) fcollideT_2d(G0, u, v, ts0, Bx0, By0, P, GP0);
-        else fcollideT_3d(G0, u, v, w, ts0, Bx0, By0, Bz0, P, GP0);
-    }
-    {
-        float dr, rho, u, v, w, Fy;
-        fmacro<D>(d1, D == 2 ? lag.y : ts1, P, dr, rho, u, v, w, Fy);
-        if (D == 2) fcollideT_2d(G1, u, v, ts1, Bx1, By1, P, GP1);
-        else fcollideT_3d(G1, u, v, w, ts1, Bx1, By1, Bz1, P, GP1);
-    }
-    stf2(A.Bout0, c0, Bx0, Bx1);
-    stf2(A.Bout1, c0, By0, By1);
-    if (D == 3) {
-        stf2(A.Bout2, c0, Bz0, Bz1);
-        stf2(A.lag_out, c0, ts0, ts1);
-    }
-    float e0[QT], e1[QT];
+    thermal_pair_end<D, S>(P, A, d, e, c0);
     S h0[QT], h1[QT];
-#pragma unroll
-    for (int a = 0; a < QT; ++a) {
-        e0[a] = GP0[a] - wT<QT>(P, a) * P.Tref;
-        e1[a] = GP1[a] - wT<QT>(P, a) * P.Tref;
-    }
-    round_pair<QT>(e0, e1, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 1), sr_seed(*A.tick, c0 + 1, 1));
+    round_pair<QT>(e, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 1), sr_seed(*A.tick, c0 + 1, 1));
     if (ODD) {
 #pragma unroll
         for (int a = 0; a < QT; ++a) push2<QT, true, S>(g, gg, a, i0, j, k, c0, n, h0[a], h1[a]);

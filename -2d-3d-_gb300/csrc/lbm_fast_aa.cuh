@@ -29,7 +29,7 @@ __device__ __forceinline__ void aa_flow_cell(const Geo& g, const PhysF& P, const
                                              long long c, int i, int j, int k) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    float d[Q], dp[Q], dr, rho, u, v, w = 0.0f, T;
+    float d[Q], Fy;
     const bool inner = aa_inner(g, i, j, k);  // no boundary rule on any pull or push
     if (ODD && inner) {
 #pragma unroll
@@ -46,12 +46,14 @@ __device__ __forceinline__ void aa_flow_cell(const Geo& g, const PhysF& P, const
         for (int a = 0; a < Q; ++a) d[a] = ldA(f, a * n + c);
     }
     if (FIRST) {
-        rho = A.rho[c];
-        dr = rho - 1.0f;
-        u = A.u[c];
-        v = A.v[c];
-        if (D == 3) w = A.w[c];
-        T = A.T[c];
+        const float rho = A.rho[c], u = A.u[c], v = A.v[c], w = D == 3 ? A.w[c] : 0.0f;
+        const float dr = rho - 1.0f;
+        float dp[Q];
+        Fy = rho * P.gBeta * (A.T[c] - P.Tref);
+        if (D == 2) fcollide_2d(d, dr, rho, u, v, Fy, P, dp);
+        else fcollide_3d(d, dr, rho, u, v, w, Fy, P, dp);
+#pragma unroll
+        for (int a = 0; a < Q; ++a) d[a] = dp[a];
     } else {
         float ts = 0.0f;
         if (gpar && inner) {
@@ -69,21 +71,13 @@ __device__ __forceinline__ void aa_flow_cell(const Geo& g, const PhysF& P, const
 #pragma unroll
             for (int a = 0; a < QT; ++a) ts += aa_local_thermal<QT, float>(g, a, i, j, k, c, graw != 0, lg);
         }
-        T = ts + P.Tref;
-        float Fy;
-        fmacro<D>(d, A.lag_in[c], P, dr, rho, u, v, w, Fy);
+        Fy = steady_flow<D>(d, steady_lag<D>(A.lag_in[c], P), ts, P);
     }
-    const float Fy = rho * P.gBeta * (T - P.Tref);
-    if (D == 2) {
-        A.lag_out[c] = Fy;
-        fcollide_2d(d, dr, rho, u, v, Fy, P, dp);
-    } else {
-        fcollide_3d(d, dr, rho, u, v, w, Fy, P, dp);
-    }
+    if (D == 2) A.lag_out[c] = Fy;
     // rounded by source cell and direction (the two-buffer kernels' bits); the push only
     // routes the stored value
     S hs[Q];
-    round_cell<Q>(dp, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
+    round_cell<Q>(d, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
     if (ODD && inner) {
 #pragma unroll
         for (int a = 0; a < Q; ++a) f[a * n + c + lat_off<Q>(g, a)] = hs[a];
@@ -104,7 +98,7 @@ __device__ __forceinline__ void aa_thermal_cell(const Geo& g, const PhysF& P, co
                                                 int graw, long long c, int i, int j, int k) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    float d[Q], G[QT], GP[QT];
+    float d[Q];
     const bool inner = aa_inner(g, i, j, k);  // no boundary rule on any pull or push
     if (fpar && inner) {
 #pragma unroll
@@ -136,41 +130,14 @@ __device__ __forceinline__ void aa_thermal_cell(const Geo& g, const PhysF& P, co
 #pragma unroll
         for (int a = 0; a < QT; ++a) e[a] = aa_local_thermal<QT, float>(g, a, i, j, k, c, graw != 0, lg);
     }
-    float Tprev;
     if (FIRST) {
         // the module array holds each value rounded to the storage type
 #pragma unroll
-        for (int a = 0; a < QT; ++a) G[a] = roundS<S>(e[a]) + wT<QT>(P, a) * P.Tref;
-        Tprev = A.T[c];
-    } else {
-        float ts = 0.0f;
-#pragma unroll
-        for (int a = 0; a < QT; ++a) {
-            G[a] = e[a] + wT<QT>(P, a) * P.Tref;
-            ts += G[a];
-        }
-        Tprev = ts;
+        for (int a = 0; a < QT; ++a) e[a] = roundS<S>(e[a]);
     }
-    float dr, rho, u, v, w, Fy;
-    fmacro<D>(d, D == 2 ? A.lag_in[c] : Tprev, P, dr, rho, u, v, w, Fy);
-    if (D == 2) {
-        float Bx = A.Bin0[c], By = A.Bin1[c];
-        fcollideT_2d(G, u, v, Tprev, Bx, By, P, GP);
-        A.Bout0[c] = Bx;
-        A.Bout1[c] = By;
-    } else {
-        float Bx = A.Bin0[c], By = A.Bin1[c], Bz = A.Bin2[c];
-        fcollideT_3d(G, u, v, w, Tprev, Bx, By, Bz, P, GP);
-        A.Bout0[c] = Bx;
-        A.Bout1[c] = By;
-        A.Bout2[c] = Bz;
-        A.lag_out[c] = Tprev;
-    }
-    float ev[QT];
+    thermal_cell_end<D, FIRST, S>(P, A, d, e, c);
     S hs[QT];
-#pragma unroll
-    for (int a = 0; a < QT; ++a) ev[a] = GP[a] - wT<QT>(P, a) * P.Tref;
-    round_cell<QT>(ev, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
+    round_cell<QT>(e, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
     if (ODD && inner) {
 #pragma unroll
         for (int a = 0; a < QT; ++a) gg[a * n + c + lat_off<QT>(g, a)] = hs[a];

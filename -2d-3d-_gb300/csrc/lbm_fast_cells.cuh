@@ -26,6 +26,7 @@ struct FastArgs {
     const float* lag_in;
     float* lag_out;
     const unsigned long long* tick;  // the lattice's step counter (stochastic rounding)
+    unsigned long long* ticks;       // the counter and its copy for the thermal kernel (lbm_fast_duo.cuh)
 };
 
 // Flow collision of step n: f_post_n from f_post_{n-1} (or the module arrays when FIRST).
@@ -41,8 +42,9 @@ __device__ __forceinline__ void flow_cell_2k(const Geo& g, const PhysF& P, const
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     const I ni = (I)g.ncell, ci = (I)c;
-    float d[Q], dp[Q], dr, rho, u, v, w = 0.0f, T;
+    float d[Q], Fy;
     if (FIRST) {
+        float dp[Q], dr, rho, u, v, w = 0.0f;
 #pragma unroll
         for (int a = 0; a < Q; ++a) d[a] = ldS(A.fref, a * ni + ci);
         rho = A.rho[ci];
@@ -50,11 +52,13 @@ __device__ __forceinline__ void flow_cell_2k(const Geo& g, const PhysF& P, const
         u = A.u[ci];
         v = A.v[ci];
         if (D == 3) w = A.w[ci];
-        T = A.T[ci];
+        Fy = rho * P.gBeta * (A.T[ci] - P.Tref);
+        if (D == 2) fcollide_2d(d, dr, rho, u, v, Fy, P, dp);
+        else fcollide_3d(d, dr, rho, u, v, w, Fy, P, dp);
+#pragma unroll
+        for (int a = 0; a < Q; ++a) d[a] = dp[a];
     } else {
-        // loads only in the branch: the arithmetic after it is one sequence for every cell,
-        // so FMA contraction rounds it as in the paired and staged kernels
-        float ts = 0.0f;
+        float ts = 0.0f;  // sum of the thermal deviations
         if (INNER && aa_inner(g, i, j, k)) {  // no pull off the faces needs a boundary rule
 #pragma unroll
             for (int a = 0; a < Q; ++a) d[a] = ldS(fin, a * ni + ci - (I)lat_off<Q>(g, a));
@@ -68,21 +72,42 @@ __device__ __forceinline__ void flow_cell_2k(const Geo& g, const PhysF& P, const
 #pragma unroll
             for (int a = 0; a < QT; ++a) ts += pull_thermal<QT, float>(g, a, i, j, k, c, lg);
         }
-        T = ts + P.Tref;  // sum of deviations + Tref * sum(wT)
-        float Fy;
-        fmacro<D>(d, A.lag_in[ci], P, dr, rho, u, v, w, Fy);
+        Fy = steady_flow<D>(d, steady_lag<D>(A.lag_in[ci], P), ts, P);
     }
-    const float Fy = rho * P.gBeta * (T - P.Tref);
-    if (D == 2) {
-        A.lag_out[ci] = Fy;
-        fcollide_2d(d, dr, rho, u, v, Fy, P, dp);
-    } else {
-        fcollide_3d(d, dr, rho, u, v, w, Fy, P, dp);
-    }
+    if (D == 2) A.lag_out[ci] = Fy;
     S hs[Q];
-    round_cell<Q>(dp, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
+    round_cell<Q>(d, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
 #pragma unroll
     for (int a = 0; a < Q; ++a) fout[a * ni + ci] = hs[a];
+}
+
+// Thermal collision of one cell from its streamed flow and thermal deviations (e, in place), with
+// B_prev and the 3D T lag (T_{n-1}).  FIRST: T is the module's, which a state load may have set
+// apart from the populations.
+template <int D, bool FIRST, class S>
+__device__ __forceinline__ void thermal_cell_end(const PhysF& P, const FastArgs<S>& A, const float* d, float* e,
+                                                 long long c) {
+    constexpr int QT = D == 2 ? 5 : 7;
+    float B[3] = {A.Bin0[c], A.Bin1[c], D == 3 ? A.Bin2[c] : 0.0f}, T;
+    if (FIRST) {
+        float G[QT], GP[QT], dr, rho, u, v, w, Fy;
+#pragma unroll
+        for (int a = 0; a < QT; ++a) G[a] = e[a] + wT<QT>(P, a) * P.Tref;
+        T = A.T[c];
+        fmacro<D>(d, D == 2 ? A.lag_in[c] : T, P, dr, rho, u, v, w, Fy);
+        if (D == 2) fcollideT_2d(G, u, v, T, B[0], B[1], P, GP);
+        else fcollideT_3d(G, u, v, w, T, B[0], B[1], B[2], P, GP);
+#pragma unroll
+        for (int a = 0; a < QT; ++a) e[a] = GP[a] - wT<QT>(P, a) * P.Tref;
+    } else {
+        T = steady_thermal<D>(d, e, D == 2 ? A.lag_in[c] : 0.0f, B, P);
+    }
+    A.Bout0[c] = B[0];
+    A.Bout1[c] = B[1];
+    if (D == 3) {
+        A.Bout2[c] = B[2];
+        A.lag_out[c] = T;
+    }
 }
 
 // Streaming, boundary and macro of the flow, and thermal collision of step n.
@@ -94,7 +119,7 @@ __device__ __forceinline__ void thermal_cell_2k(const Geo& g, const PhysF& P, co
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     const I ni = (I)g.ncell, ci = (I)c;
-    float d[Q], G[QT], GP[QT];
+    float d[Q], e[QT];
     const bool inner = INNER && aa_inner(g, i, j, k);  // no pull needs a boundary rule
     auto lf = [&](int a, long long cc) { return ldS(fin, a * n + cc); };
     if (inner) {
@@ -104,49 +129,20 @@ __device__ __forceinline__ void thermal_cell_2k(const Geo& g, const PhysF& P, co
 #pragma unroll
         for (int a = 0; a < Q; ++a) d[a] = pull_flow<Q, float>(g, a, i, j, k, c, lf);
     }
-    float Tprev;
     if (FIRST) {
 #pragma unroll
-        for (int a = 0; a < QT; ++a) G[a] = ldS(A.gref, a * ni + ci) + wT<QT>(P, a) * P.Tref;
-        Tprev = A.T[ci];
+        for (int a = 0; a < QT; ++a) e[a] = ldS(A.gref, a * ni + ci);
     } else if (inner) {
-        float ts = 0.0f;
 #pragma unroll
-        for (int a = 0; a < QT; ++a) {
-            G[a] = ldS(gin, a * ni + ci - (I)lat_off<QT>(g, a)) + wT<QT>(P, a) * P.Tref;
-            ts += G[a];
-        }
-        Tprev = ts;
+        for (int a = 0; a < QT; ++a) e[a] = ldS(gin, a * ni + ci - (I)lat_off<QT>(g, a));
     } else {
         auto lg = [&](int a, long long cc) { return ldS(gin, a * n + cc); };
-        float ts = 0.0f;
 #pragma unroll
-        for (int a = 0; a < QT; ++a) {
-            G[a] = pull_thermal<QT, float>(g, a, i, j, k, c, lg) + wT<QT>(P, a) * P.Tref;
-            ts += G[a];
-        }
-        Tprev = ts;
+        for (int a = 0; a < QT; ++a) e[a] = pull_thermal<QT, float>(g, a, i, j, k, c, lg);
     }
-    float dr, rho, u, v, w, Fy;
-    fmacro<D>(d, D == 2 ? A.lag_in[ci] : Tprev, P, dr, rho, u, v, w, Fy);
-    if (D == 2) {
-        float Bx = A.Bin0[ci], By = A.Bin1[ci];
-        fcollideT_2d(G, u, v, Tprev, Bx, By, P, GP);
-        A.Bout0[ci] = Bx;
-        A.Bout1[ci] = By;
-    } else {
-        float Bx = A.Bin0[ci], By = A.Bin1[ci], Bz = A.Bin2[ci];
-        fcollideT_3d(G, u, v, w, Tprev, Bx, By, Bz, P, GP);
-        A.Bout0[ci] = Bx;
-        A.Bout1[ci] = By;
-        A.Bout2[ci] = Bz;
-        A.lag_out[ci] = Tprev;
-    }
-    float ev[QT];
+    thermal_cell_end<D, FIRST, S>(P, A, d, e, c);
     S hs[QT];
-#pragma unroll
-    for (int a = 0; a < QT; ++a) ev[a] = GP[a] - wT<QT>(P, a) * P.Tref;
-    round_cell<QT>(ev, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
+    round_cell<QT>(e, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
 #pragma unroll
     for (int a = 0; a < QT; ++a) gout[a * ni + ci] = hs[a];
 }
@@ -165,26 +161,15 @@ __device__ __forceinline__ void flow_cell_row(const Geo& g, const PhysF& P, cons
     const long long n = g.ncell;
     auto lf = [&](int a, long long cc) { return ldS(fin, a * n + cc); };
     auto lg = [&](int a, long long cc) { return ldS(gin, a * n + cc); };
-    float d[Q], dp[Q], dr, rho, u, v, w = 0.0f, T;
-    {
-        float ts = 0.0f;
+    float d[Q], ts = 0.0f;
 #pragma unroll
-        for (int a = 0; a < Q; ++a) d[a] = pull_flow_xrow<Q, float>(g, a, i, c, lf);
+    for (int a = 0; a < Q; ++a) d[a] = pull_flow_xrow<Q, float>(g, a, i, c, lf);
 #pragma unroll
-        for (int a = 0; a < QT; ++a) ts += pull_thermal_xrow<QT, float>(g, a, i, c, lg);
-        T = ts + P.Tref;
-        float Fy;
-        fmacro<D>(d, A.lag_in[c], P, dr, rho, u, v, w, Fy);
-    }
-    const float Fy = rho * P.gBeta * (T - P.Tref);
-    if (D == 2) {
-        A.lag_out[c] = Fy;
-        fcollide_2d(d, dr, rho, u, v, Fy, P, dp);
-    } else {
-        fcollide_3d(d, dr, rho, u, v, w, Fy, P, dp);
-    }
+    for (int a = 0; a < QT; ++a) ts += pull_thermal_xrow<QT, float>(g, a, i, c, lg);
+    const float Fy = steady_flow<D>(d, steady_lag<D>(A.lag_in[c], P), ts, P);
+    if (D == 2) A.lag_out[c] = Fy;
     S hs[Q];
-    round_cell<Q>(dp, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
+    round_cell<Q>(d, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
 #pragma unroll
     for (int a = 0; a < Q; ++a) fout[a * n + c] = hs[a];
 }
@@ -197,39 +182,14 @@ __device__ __forceinline__ void thermal_cell_row(const Geo& g, const PhysF& P, c
     const long long n = g.ncell;
     auto lf = [&](int a, long long cc) { return ldS(fin, a * n + cc); };
     auto lg = [&](int a, long long cc) { return ldS(gin, a * n + cc); };
-    float d[Q], G[QT], GP[QT];
+    float d[Q], e[QT];
 #pragma unroll
     for (int a = 0; a < Q; ++a) d[a] = pull_flow_xrow<Q, float>(g, a, i, c, lf);
-    float Tprev;
-    {
-        float ts = 0.0f;
 #pragma unroll
-        for (int a = 0; a < QT; ++a) {
-            G[a] = pull_thermal_xrow<QT, float>(g, a, i, c, lg) + wT<QT>(P, a) * P.Tref;
-            ts += G[a];
-        }
-        Tprev = ts;
-    }
-    float dr, rho, u, v, w, Fy;
-    fmacro<D>(d, D == 2 ? A.lag_in[c] : Tprev, P, dr, rho, u, v, w, Fy);
-    if (D == 2) {
-        float Bx = A.Bin0[c], By = A.Bin1[c];
-        fcollideT_2d(G, u, v, Tprev, Bx, By, P, GP);
-        A.Bout0[c] = Bx;
-        A.Bout1[c] = By;
-    } else {
-        float Bx = A.Bin0[c], By = A.Bin1[c], Bz = A.Bin2[c];
-        fcollideT_3d(G, u, v, w, Tprev, Bx, By, Bz, P, GP);
-        A.Bout0[c] = Bx;
-        A.Bout1[c] = By;
-        A.Bout2[c] = Bz;
-        A.lag_out[c] = Tprev;
-    }
-    float ev[QT];
+    for (int a = 0; a < QT; ++a) e[a] = pull_thermal_xrow<QT, float>(g, a, i, c, lg);
+    thermal_cell_end<D, false, S>(P, A, d, e, c);
     S hs[QT];
-#pragma unroll
-    for (int a = 0; a < QT; ++a) ev[a] = GP[a] - wT<QT>(P, a) * P.Tref;
-    round_cell<QT>(ev, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
+    round_cell<QT>(e, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
 #pragma unroll
     for (int a = 0; a < QT; ++a) gout[a * n + c] = hs[a];
 }

@@ -88,38 +88,6 @@ __device__ __forceinline__ void round_cell(const float* v, __half* h, bool sr, u
         }
     }
 }
-// The same for two cells (paired forms): value a of each cell takes the bits it takes in
-// round_cell.
-template <int Q>
-__device__ __forceinline__ void round_pair(const float* v0, const float* v1, float* h0, float* h1, bool, unsigned,
-                                           unsigned) {
-#pragma unroll
-    for (int a = 0; a < Q; ++a) {
-        h0[a] = v0[a];
-        h1[a] = v1[a];
-    }
-}
-template <int Q>
-__device__ __forceinline__ void round_pair(const float* v0, const float* v1, __half* h0, __half* h1, bool sr,
-                                           unsigned seed0, unsigned seed1) {
-#pragma unroll
-    for (int j = 0; 2 * j < Q; ++j) {
-        const unsigned w0 = sr ? sr_word(seed0, j) : 0u, w1 = sr ? sr_word(seed1, j) : 0u;
-#pragma unroll
-        for (int a = 2 * j; a < 2 * j + 2 && a < Q; ++a) {
-            if (sr) {
-                const unsigned r0 = (a & 1) ? w0 >> 16 : w0 & 0xFFFFu, r1 = (a & 1) ? w1 >> 16 : w1 & 0xFFFFu;
-                const unsigned d = cvt_rs_f16x2(v1[a], v0[a], (r1 << 16) | r0);
-                h0[a] = lo_half(d);
-                h1[a] = hi_half(d);
-            } else {
-                h0[a] = __float2half_rn(v0[a]);
-                h1[a] = __float2half_rn(v1[a]);
-            }
-        }
-    }
-}
-
 // Rest weights (D2Q9 2DRB.F90:506-512, D3Q19 3DRB.F90:669-671).
 template <int Q>
 __host__ __device__ constexpr double wrest(int a) {
@@ -134,6 +102,14 @@ struct PhysF {
     float omegaT0, omegaT1, geqc;
     int use_g, legacy;
     int sr;  // FP16 storage: stochastic rounding of the new populations (round_cell, round_pair)
+    // steady-state collisions in even and odd parts (steady_flow, steady_thermal), s = Snu,
+    // q = Sq; rounded once on the host (steady_constants)
+    float ce, co;               // (1 - s)/2, (1 - q)/2
+    float kd, kt, kx, kv;       // density, trace and axis shares, v F share of the axis terms
+    float kc, kf;               // s/4, 1/4 - s/8: cross terms rho u v and u F
+    float q12, sqg;             // q/12; q/120 (3D), q/24 (2D)
+    float te, ta;               // 1 - Qnu; Qnu a_T, a_T T the equilibrium of the even moment
+    float to, tb, tg;           // (1 - Qk)/2, Qk/2, SG/2
 };
 
 inline PhysF to_physf(const PhysC& P) {
@@ -148,6 +124,27 @@ inline PhysF to_physf(const PhysC& P) {
     return F;
 }
 
+// The constants of the steady-state collisions.  All even flow moments relax at Snu and all odd
+// ones at Sq (commondata sets Se = Seps = Spi = Snu and Sm = Sq, 3DRB.F90:92-97).
+inline void steady_constants(const PhysC& P, int dim, PhysF& F) {
+    const double s = P.Snu, q = P.Sq, m = dim == 3 ? 1.0 : 2.0;
+    F.ce = (float)(0.5 * (1.0 - s));
+    F.co = (float)(0.5 * (1.0 - q));
+    F.kd = (float)(m * s / 18.0);
+    F.kt = (float)(m * s / 12.0);
+    F.kx = (float)(m * s / 4.0);
+    F.kv = (float)(-m / 6.0);
+    F.kc = (float)(s / 4.0);
+    F.kf = (float)(0.25 - s / 8.0);
+    F.q12 = (float)(q / 12.0);
+    F.sqg = (float)(dim == 3 ? q / 120.0 : q / 24.0);
+    F.te = (float)(1.0 - P.Qnu);
+    F.ta = (float)(P.Qnu * (P.legacy ? P.paraA : (dim == 3 ? -0.75 : -2.0 / 3.0)));
+    F.to = (float)(0.5 * (1.0 - P.Qk));
+    F.tb = (float)(0.5 * P.Qk);
+    F.tg = (float)(0.5 * P.SG);
+}
+
 // Thermal wall terms for deviations: e_a = -e_opp + 2 wT (Tw - Tref).
 inline Geo dev_geo(const Geo& g, const PhysC& P) {
     Geo d = g;
@@ -159,7 +156,299 @@ inline Geo dev_geo(const Geo& g, const PhysC& P) {
 }
 
 // ------------------------------------------------------------------------------------
-// per-cell arithmetic (FP32, deviations)
+// Arithmetic of one cell (float) or of two cells at once (f2: GB300's packed FP32 operations,
+// two results per issued instruction).  Every operation rounds once.  The assembler contracts a
+// packed multiplication and the addition of its result into one operation (not so the scalar
+// ones), so a product goes into a sum by vfma only, except one by a power of two, which is exact:
+// then all kernel forms give the same bits.
+// ------------------------------------------------------------------------------------
+struct f2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f2 make_f2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float f2_lo(f2 a) { return __uint_as_float((unsigned)a.v); }
+__device__ __forceinline__ float f2_hi(f2 a) { return __uint_as_float((unsigned)(a.v >> 32)); }
+// The same for two cells (paired forms): value a of each cell takes the bits it takes in
+// round_cell.
+template <int Q>
+__device__ __forceinline__ void round_pair(const f2* v, float* h0, float* h1, bool, unsigned, unsigned) {
+#pragma unroll
+    for (int a = 0; a < Q; ++a) {
+        h0[a] = f2_lo(v[a]);
+        h1[a] = f2_hi(v[a]);
+    }
+}
+template <int Q>
+__device__ __forceinline__ void round_pair(const f2* v, __half* h0, __half* h1, bool sr, unsigned seed0,
+                                           unsigned seed1) {
+#pragma unroll
+    for (int j = 0; 2 * j < Q; ++j) {
+        const unsigned w0 = sr ? sr_word(seed0, j) : 0u, w1 = sr ? sr_word(seed1, j) : 0u;
+#pragma unroll
+        for (int a = 2 * j; a < 2 * j + 2 && a < Q; ++a) {
+            if (sr) {
+                const unsigned r0 = (a & 1) ? w0 >> 16 : w0 & 0xFFFFu, r1 = (a & 1) ? w1 >> 16 : w1 & 0xFFFFu;
+                const unsigned d = cvt_rs_f16x2(f2_hi(v[a]), f2_lo(v[a]), (r1 << 16) | r0);
+                h0[a] = lo_half(d);
+                h1[a] = hi_half(d);
+            } else {
+                h0[a] = __float2half_rn(f2_lo(v[a]));
+                h1[a] = __float2half_rn(f2_hi(v[a]));
+            }
+        }
+    }
+}
+
+template <class V> __device__ __forceinline__ V vset(float c);
+template <> __device__ __forceinline__ float vset<float>(float c) { return c; }
+template <> __device__ __forceinline__ f2 vset<f2>(float c) { return make_f2(c, c); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ f2 vfma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f2 vadd(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 vsub(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 vmul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ float vneg(float a) { return -a; }
+__device__ __forceinline__ f2 vneg(f2 a) {
+    f2 r;
+    r.v = a.v ^ 0x8000000080000000ULL;
+    return r;
+}
+template <class V> __device__ __forceinline__ V vfma(float a, V b, V c) { return vfma(vset<V>(a), b, c); }
+template <class V> __device__ __forceinline__ V vmul(float a, V b) { return vmul(vset<V>(a), b); }
+__device__ __forceinline__ float rcp_seed(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float vrcp_seed(float x) { return rcp_seed(x); }
+__device__ __forceinline__ f2 vrcp_seed(f2 x) { return make_f2(rcp_seed(f2_lo(x)), rcp_seed(f2_hi(x))); }
+// 1/x: the hardware seed (1 ulp) and one step of Newton's iteration
+template <class V>
+__device__ __forceinline__ V vrcp(V x) {
+    const V r = vrcp_seed(x);
+    return vfma(r, vfma(vneg(x), r, vset<V>(1.0f)), r);
+}
+
+// Macro step of the flow (fmacro's, 3DRB.F90:1066-1098, 2DRB.F90:878-894) on deviations, from
+// the sums E and differences O of opposite directions: rho - 1, j = sum e d, rho v with half the
+// lag's force (3D: rho gBeta lag with lag = T_lag - Tref; 2D: lag is the stored force), u.
+// Pairs (E and O indices): 3D 0..2 axes, 3 (7, 10), 4 (8, 9), 5 (11, 14), 6 (12, 13), 7 (15, 18),
+// 8 (17, 16); 2D 0 (1, 3), 1 (2, 4), 2 (5, 7), 3 (6, 8).
+template <int D>
+__host__ __device__ constexpr int pair_lo(int b) {
+    return D == 2 ? (b == 0 ? 1 : b == 1 ? 2 : b == 2 ? 5 : 6)
+                  : (b < 3 ? 2 * b + 1 : b == 3 ? 7 : b == 4 ? 8 : b == 5 ? 11 : b == 6 ? 12 : b == 7 ? 15 : 17);
+}
+template <int D>
+__host__ __device__ constexpr int pair_hi(int b) {
+    return D == 2 ? Lat<9>::opp(pair_lo<D>(b)) : Lat<19>::opp(pair_lo<D>(b));
+}
+// gr: rho gBeta.
+template <int D, class V>
+__device__ __forceinline__ void steady_macro(V d0, const V* E, const V* O, V lag, const PhysF& P, V& dr, V& gr, V* j,
+                                             V& py, V* u) {
+    if (D == 2) {
+        dr = vadd(vadd(d0, vadd(E[0], E[1])), vadd(E[2], E[3]));
+        j[0] = vadd(O[0], vsub(O[2], O[3]));
+        j[1] = vadd(O[1], vadd(O[2], O[3]));
+        j[2] = vset<V>(0.0f);
+    } else {
+        dr = vadd(vadd(d0, vadd(vadd(E[0], E[1]), E[2])),
+                  vadd(vadd(vadd(E[3], E[4]), vadd(E[5], E[6])), vadd(E[7], E[8])));
+        j[0] = vadd(O[0], vadd(vsub(O[3], O[4]), vsub(O[5], O[6])));
+        j[1] = vadd(O[1], vadd(vadd(O[3], O[4]), vadd(O[7], O[8])));
+        j[2] = vadd(O[2], vadd(vadd(O[5], O[6]), vsub(O[7], O[8])));
+    }
+    const V rho = vadd(vset<V>(1.0f), dr);
+    gr = vmul(P.gBeta, rho);
+    const V inv = vrcp(rho);
+    py = vfma(0.5f, D == 2 ? lag : vmul(gr, lag), j[1]);
+    u[0] = vmul(j[0], inv);
+    u[1] = vmul(py, inv);
+    u[2] = D == 3 ? vmul(j[2], inv) : vset<V>(0.0f);
+}
+
+// The lag of a cell as steady_macro takes it, from the stored one (3D: T_lag; 2D: F_y).
+template <int D, class V>
+__device__ __forceinline__ V steady_lag(V stored, const PhysF& P) {
+    return D == 3 ? vsub(stored, vset<V>(P.Tref)) : stored;
+}
+
+// Flow collision with Guo forcing of a steady-state step (fcollide_2d / fcollide_3d for a cell's
+// own rho and u), in place on deviations.  lag: as in steady_macro; ts: sum of the thermal
+// deviations (T - Tref); returns the force F_y.  The moments relax at two rates (even s, odd q)
+// towards the quadratic equilibrium, so the relaxation acts on E = d_a + d_-a and O = d_a - d_-a:
+//   E' = (1 - s) E + 2 g,  g = s feq+ + (1 - s/2) S+ (S+ the even Guo source),
+//   O' = (1 - q) O + 2 k,  k = q 3w e.j + 3w e_y F (and the lagged force's share G of the odd
+//                          fourth-order moment);
+// the momentum is conserved because sum e O over the pairs and 2k cancel.  About 150 operations
+// in 3D instead of 340 in moment space.
+template <int D, class V>
+__device__ __forceinline__ V steady_flow(V* d, V lag, V ts, const PhysF& P) {
+    constexpr int NP = D == 3 ? 9 : 4;
+    V E[NP], O[NP], dr, gr, j[3], py, u[3];
+#pragma unroll
+    for (int b = 0; b < NP; ++b) {
+        E[b] = vadd(d[pair_lo<D>(b)], d[pair_hi<D>(b)]);
+        O[b] = vsub(d[pair_lo<D>(b)], d[pair_hi<D>(b)]);
+    }
+    steady_macro<D>(d[0], E, O, lag, P, dr, gr, j, py, u);
+    const V F = vmul(gr, ts);
+    // even parts: g of the axes is Am + kx (xx, zz) and Am + Y, of the diagonals half their sums
+    // (2D: a quarter) with the cross term added and taken off
+    const V vF = vmul(u[1], F), uF = vmul(u[0], F);
+    const V xx = vmul(j[0], u[0]), yy = vmul(u[1], vfma(vneg(gr), ts, py));
+    V t = vfma(j[0], u[0], yy), zz = vset<V>(0.0f);
+    if (D == 3) {
+        zz = vmul(j[2], u[2]);
+        t = vfma(j[2], u[2], t);
+    }
+    const V Am = vfma(P.kv, vF, vfma(-P.kt, t, vmul(P.kd, dr)));
+    const V Y = vfma(P.kx, yy, D == 3 ? vmul(0.5f, vF) : vF);
+    const V cxy = vfma(P.kf, uF, vmul(P.kc, vmul(j[0], u[1])));
+    const V ax = vfma(P.kx, xx, Am), ay = vadd(Am, Y);
+    // odd parts: k of the axes and diagonals from q12 j, with the force and its lag's share G
+    const V M = vfma(1.0f / 12.0f, F, vmul(P.q12, j[1]));
+    const V w = D == 3 ? vmul(gr, vsub(ts, lag)) : vfma(gr, ts, vneg(lag));  // F - F_lag
+    const V jy = vfma(P.sqg, w, M);
+    V g[NP], k[NP];
+    g[0] = ax;
+    g[1] = ay;
+    if (D == 2) {
+        const V xy = vmul(0.25f, vadd(ax, Y));
+        g[2] = vadd(xy, cxy);
+        g[3] = vsub(xy, cxy);
+        k[2] = vfma(P.q12, j[0], jy);
+        k[3] = vfma(-P.q12, j[0], jy);
+    } else {
+        const V xy = vmul(0.5f, vadd(ax, Y)), xz = vmul(0.5f, vfma(P.kx, zz, ax)), yz = vmul(0.5f, vfma(P.kx, zz, ay));
+        const V ruw = vmul(j[0], u[2]), cyz = vfma(P.kf, vmul(u[2], F), vmul(P.kc, vmul(py, u[2])));
+        const V jz = vmul(P.q12, j[2]);
+        g[2] = vfma(P.kx, zz, Am);
+        g[3] = vadd(xy, cxy);
+        g[4] = vsub(xy, cxy);
+        g[5] = vfma(P.kc, ruw, xz);
+        g[6] = vfma(-P.kc, ruw, xz);
+        g[7] = vadd(yz, cyz);
+        g[8] = vsub(yz, cyz);
+        k[3] = vfma(P.q12, j[0], jy);
+        k[4] = vfma(-P.q12, j[0], jy);
+        k[5] = vfma(P.q12, j[0], jz);
+        k[6] = vfma(-P.q12, j[0], jz);
+        k[7] = vfma(P.q12, j[2], jy);
+        k[8] = vfma(-P.q12, j[2], jy);
+    }
+    // The axis pairs' odd parts are what the momentum j + F_y leaves after the diagonals', and the
+    // rest population what the mass leaves: constants that do not sum to one in FP32 would scale
+    // both a little in every step.  The momentum passes through fcollide's own FP32 factor (1/6,
+    // 1/10; 3e-8 and 1.5e-8 from exact), so that long runs stay with those of the moment form.
+#pragma unroll
+    for (int b = 0; b < NP; ++b) E[b] = vfma(P.ce, E[b], g[b]);
+#pragma unroll
+    for (int b = D; b < NP; ++b) O[b] = vfma(P.co, O[b], k[b]);
+    const V jf = vfma(gr, ts, j[1]);
+    if (D == 2) {
+        O[0] = vfma(3.0f, vmul(1.0f / 6.0f, j[0]), vsub(O[3], O[2]));
+        O[1] = vfma(3.0f, vmul(1.0f / 6.0f, jf), vneg(vadd(O[2], O[3])));
+        d[0] = vfma(-2.0f, vadd(vadd(E[0], E[1]), vadd(E[2], E[3])), dr);
+    } else {
+        O[0] = vfma(5.0f, vmul(0.1f, j[0]), vadd(vsub(O[4], O[3]), vsub(O[6], O[5])));
+        O[1] = vfma(5.0f, vmul(0.1f, jf), vneg(vadd(vadd(O[3], O[4]), vadd(O[7], O[8]))));
+        O[2] = vfma(5.0f, vmul(0.1f, j[2]), vsub(vsub(O[8], O[7]), vadd(O[5], O[6])));
+        d[0] = vfma(-2.0f, vadd(vadd(vadd(vadd(E[0], E[1]), E[2]), vadd(E[3], E[4])), vadd(vadd(E[5], E[6]), vadd(E[7], E[8]))), dr);
+    }
+#pragma unroll
+    for (int b = 0; b < NP; ++b) {
+        d[pair_lo<D>(b)] = vadd(E[b], O[b]);
+        d[pair_hi<D>(b)] = vsub(E[b], O[b]);
+    }
+    return F;
+}
+
+// Macro step of the flow and thermal collision with the M1G term of a steady-state step
+// (fmacro and fcollideT_2d / fcollideT_3d on deviations): d the streamed flow populations, e the
+// streamed thermal deviations (in place), lag the 2D stored force, B the previous u T (in and,
+// when use_g, out).  Returns T.  Even parts relax at Qnu, odd parts at Qk.
+template <int D, class V>
+__device__ __forceinline__ V steady_thermal(const V* d, V* e, V lag, V* B, const PhysF& P) {
+    constexpr int NP = D == 3 ? 9 : 4;
+    V E[NP], O[NP], dr, gr, j[3], py, u[3];
+#pragma unroll
+    for (int b = 0; b < NP; ++b) {
+        E[b] = vadd(d[pair_lo<D>(b)], d[pair_hi<D>(b)]);
+        O[b] = vsub(d[pair_lo<D>(b)], d[pair_hi<D>(b)]);
+    }
+    V sE[D], sO[D], tdev = e[0];
+#pragma unroll
+    for (int b = 0; b < D; ++b) {
+        const int lo = D == 3 ? 2 * b + 1 : b + 1, hi = D == 3 ? 2 * b + 2 : b + 3;
+        sE[b] = vadd(e[lo], e[hi]);
+        sO[b] = vsub(e[lo], e[hi]);
+        tdev = vadd(tdev, sE[b]);
+    }
+    const V T = vadd(tdev, vset<V>(P.Tref));
+    steady_macro<D>(d[0], E, O, D == 3 ? steady_lag<D>(T, P) : lag, P, dr, gr, j, py, u);
+    // even parts from the moments, with fcollideT's factors
+    V ev[D], S = vadd(sE[0], sE[1]);
+    if (D == 2) {
+        const V p3 = vfma(P.te, vfma(-4.0f, e[0], S), vmul(P.ta, tdev)), p4 = vmul(P.te, vsub(sE[0], sE[1]));
+        const V a = vmul(0.2f, tdev), c = vfma(0.05f, p3, a);
+        e[0] = vfma(-0.2f, p3, a);
+        ev[0] = vfma(0.25f, p4, c);
+        ev[1] = vfma(-0.25f, p4, c);
+    } else {
+        const V yz = vadd(sE[1], sE[D - 1]);
+        S = vadd(sE[0], yz);
+        const V p4 = vfma(P.te, vfma(-6.0f, e[0], S), vmul(P.ta, tdev));
+        const V p5 = vmul(P.te, vfma(2.0f, sE[0], vneg(yz))), p6 = vmul(P.te, vsub(sE[1], sE[D - 1]));
+        const V a = vmul(1.0f / 7.0f, tdev), b = vfma(1.0f / 42.0f, p4, a), c = vfma(-1.0f / 12.0f, p5, b);
+        e[0] = vfma(-1.0f / 7.0f, p4, a);
+        ev[0] = vfma(1.0f / 6.0f, p5, b);
+        ev[1] = vfma(0.25f, p6, c);
+        ev[D - 1] = vfma(-0.25f, p6, c);
+    }
+#pragma unroll
+    for (int b = 0; b < D; ++b) {
+        const int lo = D == 3 ? 2 * b + 1 : b + 1, hi = D == 3 ? 2 * b + 2 : b + 3;
+        const V b1 = vmul(u[b], T);
+        V k = vmul(P.tb, b1);
+        if (P.use_g) {
+            k = vfma(P.tg, vfma(u[b], T, vneg(B[b])), k);
+            B[b] = b1;
+        }
+        const V od = vfma(P.to, sO[b], k);
+        e[lo] = vadd(ev[b], od);
+        e[hi] = vsub(ev[b], od);
+    }
+    return T;
+}
+
+// ------------------------------------------------------------------------------------
+// per-cell arithmetic in moment space (FP32, deviations): the first step after `initial` or a
+// state load, whose rho, u and T are the loaded ones and need not be those of the populations
 // ------------------------------------------------------------------------------------
 // D2Q9 MRT collision with Guo forcing (2DRB.F90:688-759) on deviations d.
 __device__ __forceinline__ void fcollide_2d(const float* d, float dr, float rho, float u, float v, float Fy,

@@ -10,7 +10,7 @@
 // vectors that hold it.  Cells whose source lies outside the lattice (the x faces for the
 // cell at the face, every direction with an out-of-range y or z source) take the scalar
 // pull with the reference's boundary rule, so the values are those of the one-cell path.
-// The per-cell arithmetic is the same inline functions in the same order.
+// The per-cell arithmetic is the same inline functions, on both cells at once (f2).
 #pragma once
 
 #include "lbm_fast_cells.cuh"
@@ -102,43 +102,41 @@ __device__ __forceinline__ void flow_pair_2k(const Geo& g, const PhysF& P, const
     const long long n = g.ncell;
     auto lf = [&](int a, long long cc) { return ldS(fin, a * n + cc); };
     auto lg = [&](int a, long long cc) { return ldS(gin, a * n + cc); };
-    float d0[Q], d1[Q];
+    f2 d[Q], ts = make_f2(0.0f, 0.0f);
 #pragma unroll
     for (int a = 0; a < Q; ++a) {
         const float2 v = pull_flow_pair<Q, S>(g, fin, a, i0, j, k, c0, n, lf);
-        d0[a] = v.x;
-        d1[a] = v.y;
+        d[a] = make_f2(v.x, v.y);
     }
-    float ts0 = 0.0f, ts1 = 0.0f;
 #pragma unroll
     for (int a = 0; a < QT; ++a) {
         const float2 e = pull_thermal_pair<QT, S>(g, gin, a, i0, j, k, c0, n, lg);
-        ts0 += e.x;
-        ts1 += e.y;
+        ts = vadd(ts, make_f2(e.x, e.y));
     }
     const float2 lag = ldf2(A.lag_in, c0);
-    float dp0[Q], dp1[Q], Fy0, Fy1;
-    {
-        const float T = ts0 + P.Tref;
-        float dr, rho, u, v, w = 0.0f, Fm;
-        fmacro<D>(d0, lag.x, P, dr, rho, u, v, w, Fm);
-        Fy0 = rho * P.gBeta * (T - P.Tref);
-        if (D == 2) fcollide_2d(d0, dr, rho, u, v, Fy0, P, dp0);
-        else fcollide_3d(d0, dr, rho, u, v, w, Fy0, P, dp0);
-    }
-    {
-        const float T = ts1 + P.Tref;
-        float dr, rho, u, v, w = 0.0f, Fm;
-        fmacro<D>(d1, lag.y, P, dr, rho, u, v, w, Fm);
-        Fy1 = rho * P.gBeta * (T - P.Tref);
-        if (D == 2) fcollide_2d(d1, dr, rho, u, v, Fy1, P, dp1);
-        else fcollide_3d(d1, dr, rho, u, v, w, Fy1, P, dp1);
-    }
-    if (D == 2) stf2(A.lag_out, c0, Fy0, Fy1);
+    const f2 Fy = steady_flow<D>(d, steady_lag<D>(make_f2(lag.x, lag.y), P), ts, P);
+    if (D == 2) stf2(A.lag_out, c0, f2_lo(Fy), f2_hi(Fy));
     S h0[Q], h1[Q];
-    round_pair<Q>(dp0, dp1, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 0), sr_seed(*A.tick, c0 + 1, 0));
+    round_pair<Q>(d, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 0), sr_seed(*A.tick, c0 + 1, 0));
 #pragma unroll
     for (int a = 0; a < Q; ++a) Vec2<S>::st_raw(fout, a * n + c0, h0[a], h1[a]);
+}
+
+// thermal_cell_end (not FIRST) for the cells c0 and c0 + 1.
+template <int D, class S>
+__device__ __forceinline__ void thermal_pair_end(const PhysF& P, const FastArgs<S>& A, const f2* d, f2* e,
+                                                 long long c0) {
+    const float2 bx = ldf2(A.Bin0, c0), by = ldf2(A.Bin1, c0);
+    const float2 bz = D == 3 ? ldf2(A.Bin2, c0) : make_float2(0.0f, 0.0f);
+    const float2 lag = D == 2 ? ldf2(A.lag_in, c0) : make_float2(0.0f, 0.0f);
+    f2 B[3] = {make_f2(bx.x, bx.y), make_f2(by.x, by.y), make_f2(bz.x, bz.y)};
+    const f2 T = steady_thermal<D>(d, e, make_f2(lag.x, lag.y), B, P);
+    stf2(A.Bout0, c0, f2_lo(B[0]), f2_hi(B[0]));
+    stf2(A.Bout1, c0, f2_lo(B[1]), f2_hi(B[1]));
+    if (D == 3) {
+        stf2(A.Bout2, c0, f2_lo(B[2]), f2_hi(B[2]));
+        stf2(A.lag_out, c0, f2_lo(T), f2_hi(T));
+    }
 }
 
 // thermal_cell_2k (not FIRST) for the cells c0 and c0 + 1.
@@ -150,53 +148,20 @@ __device__ __forceinline__ void thermal_pair_2k(const Geo& g, const PhysF& P, co
     const long long n = g.ncell;
     auto lf = [&](int a, long long cc) { return ldS(fin, a * n + cc); };
     auto lg = [&](int a, long long cc) { return ldS(gin, a * n + cc); };
-    float d0[Q], d1[Q], G0[QT], G1[QT];
+    f2 d[Q], e[QT];
 #pragma unroll
     for (int a = 0; a < Q; ++a) {
         const float2 v = pull_flow_pair<Q, S>(g, fin, a, i0, j, k, c0, n, lf);
-        d0[a] = v.x;
-        d1[a] = v.y;
+        d[a] = make_f2(v.x, v.y);
     }
-    float ts0 = 0.0f, ts1 = 0.0f;
 #pragma unroll
     for (int a = 0; a < QT; ++a) {
-        const float2 e = pull_thermal_pair<QT, S>(g, gin, a, i0, j, k, c0, n, lg);
-        G0[a] = e.x + wT<QT>(P, a) * P.Tref;
-        G1[a] = e.y + wT<QT>(P, a) * P.Tref;
-        ts0 += G0[a];
-        ts1 += G1[a];
+        const float2 v = pull_thermal_pair<QT, S>(g, gin, a, i0, j, k, c0, n, lg);
+        e[a] = make_f2(v.x, v.y);
     }
-    const float2 bx = ldf2(A.Bin0, c0), by = ldf2(A.Bin1, c0);
-    const float2 bz = D == 3 ? ldf2(A.Bin2, c0) : make_float2(0.0f, 0.0f);
-    const float2 lag = D == 2 ? ldf2(A.lag_in, c0) : make_float2(0.0f, 0.0f);
-    float GP0[QT], GP1[QT];
-    float Bx0 = bx.x, By0 = by.x, Bz0 = bz.x, Bx1 = bx.y, By1 = by.y, Bz1 = bz.y;
-    {
-        float dr, rho, u, v, w, Fy;
-        fmacro<D>(d0, D == 2 ? lag.x : ts0, P, dr, rho, u, v, w, Fy);
-        if (D == 2) fcollideT_2d(G0, u, v, ts0, Bx0, By0, P, GP0);
-        else fcollideT_3d(G0, u, v, w, ts0, Bx0, By0, Bz0, P, GP0);
-    }
-    {
-        float dr, rho, u, v, w, Fy;
-        fmacro<D>(d1, D == 2 ? lag.y : ts1, P, dr, rho, u, v, w, Fy);
-        if (D == 2) fcollideT_2d(G1, u, v, ts1, Bx1, By1, P, GP1);
-        else fcollideT_3d(G1, u, v, w, ts1, Bx1, By1, Bz1, P, GP1);
-    }
-    stf2(A.Bout0, c0, Bx0, Bx1);
-    stf2(A.Bout1, c0, By0, By1);
-    if (D == 3) {
-        stf2(A.Bout2, c0, Bz0, Bz1);
-        stf2(A.lag_out, c0, ts0, ts1);
-    }
-    float e0[QT], e1[QT];
+    thermal_pair_end<D, S>(P, A, d, e, c0);
     S h0[QT], h1[QT];
-#pragma unroll
-    for (int a = 0; a < QT; ++a) {
-        e0[a] = GP0[a] - wT<QT>(P, a) * P.Tref;
-        e1[a] = GP1[a] - wT<QT>(P, a) * P.Tref;
-    }
-    round_pair<QT>(e0, e1, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 1), sr_seed(*A.tick, c0 + 1, 1));
+    round_pair<QT>(e, h0, h1, P.sr != 0, sr_seed(*A.tick, c0, 1), sr_seed(*A.tick, c0 + 1, 1));
 #pragma unroll
     for (int a = 0; a < QT; ++a) Vec2<S>::st_raw(gout, a * n + c0, h0[a], h1[a]);
 }

@@ -350,49 +350,27 @@ __global__ void __launch_bounds__(PP::threads, PP::blocks)
                 float ts = 0.0f;
 #pragma unroll
                 for (int a = 0; a < QT; ++a) ts += s2f(sg[a * rc + (size_t)r * nx + (i - (LG == kRowLocal ? 0 : Lat<QT>::ex(a)))]);
-                const float T = ts + P.Tref;
-                float dr, rho, u, v, w = 0.0f, Fm;
-                fmacro<D>(d, sfl[(size_t)r * nx + i], P, dr, rho, u, v, w, Fm);
-                const float Fy = rho * P.gBeta * (T - P.Tref);
-                float dp[Q];
-                if (D == 2) {
-                    A.lag_out[c] = Fy;
-                    fcollide_2d(d, dr, rho, u, v, Fy, P, dp);
-                } else {
-                    fcollide_3d(d, dr, rho, u, v, w, Fy, P, dp);
-                }
+                const float Fy = steady_flow<D>(d, steady_lag<D>(sfl[(size_t)r * nx + i], P), ts, P);
+                if (D == 2) A.lag_out[c] = Fy;
                 S hs[Q];
-                round_cell<Q>(dp, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
+                round_cell<Q>(d, hs, P.sr != 0, sr_seed(*A.tick, c, 0));
 #pragma unroll
                 for (int a = 0; a < Q; ++a) out[store_index<Q, ST>(g, a, c, n)] = hs[a];
             } else {
-                float G[QT], GP[QT], ts = 0.0f;
+                float ee[QT];
 #pragma unroll
-                for (int a = 0; a < QT; ++a) {
-                    G[a] = s2f(sg[a * rc + (size_t)r * nx + (i - (LG == kRowLocal ? 0 : Lat<QT>::ex(a)))]) + wT<QT>(P, a) * P.Tref;
-                    ts += G[a];
-                }
+                for (int a = 0; a < QT; ++a) ee[a] = s2f(sg[a * rc + (size_t)r * nx + (i - (LG == kRowLocal ? 0 : Lat<QT>::ex(a)))]);
                 const size_t e = (size_t)r * nx + i;
-                float dr, rho, u, v, w, Fy;
-                fmacro<D>(d, D == 2 ? sfl[2 * rc + e] : ts, P, dr, rho, u, v, w, Fy);
-                if (D == 2) {
-                    float Bx = sfl[e], By = sfl[rc + e];
-                    fcollideT_2d(G, u, v, ts, Bx, By, P, GP);
-                    A.Bout0[c] = Bx;
-                    A.Bout1[c] = By;
-                } else {
-                    float Bx = sfl[e], By = sfl[rc + e], Bz = sfl[2 * rc + e];
-                    fcollideT_3d(G, u, v, w, ts, Bx, By, Bz, P, GP);
-                    A.Bout0[c] = Bx;
-                    A.Bout1[c] = By;
-                    A.Bout2[c] = Bz;
-                    A.lag_out[c] = ts;
+                float B[3] = {sfl[e], sfl[rc + e], D == 3 ? sfl[2 * rc + e] : 0.0f};
+                const float T = steady_thermal<D>(d, ee, D == 2 ? sfl[2 * rc + e] : 0.0f, B, P);
+                A.Bout0[c] = B[0];
+                A.Bout1[c] = B[1];
+                if (D == 3) {
+                    A.Bout2[c] = B[2];
+                    A.lag_out[c] = T;
                 }
-                float ev[QT];
                 S hs[QT];
-#pragma unroll
-                for (int a = 0; a < QT; ++a) ev[a] = GP[a] - wT<QT>(P, a) * P.Tref;
-                round_cell<QT>(ev, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
+                round_cell<QT>(ee, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
 #pragma unroll
                 for (int a = 0; a < QT; ++a) out[store_index<QT, ST>(g, a, c, n)] = hs[a];
             }

@@ -49,55 +49,41 @@ __device__ __forceinline__ float stored_value(float h) { return h; }
 __device__ __forceinline__ float stored_value(__half h) { return __half2float(h); }
 
 // Thermal stage at one cell: pulls, macro, thermal collision.  Returns g_post_n as the
-// next pull reads it (the stored deviations, rounded to the storage type and back; halo
-// cells round with the owner's random bits, so they hold the owner's values) and, through
-// the references, the flow state f_n (deviations), rho_n, u_n.
+// next pull reads it (GP: the stored deviations, rounded to the storage type and back; halo
+// cells round with the owner's random bits, so they hold the owner's values) and the lag of
+// the cell's macro step (3D: T_{n-1}; 2D: F_y,n), which the flow stage repeats.
 template <int D, class S>
-__device__ __forceinline__ void thermal_cell(const Geo& g, const PhysF& P, const FusedArgs<S>& A, int x, int y, int z,
-                                             bool owner, float* d, float& dr, float& rho, float& u, float& v, float& w,
-                                             float* GP) {
+__device__ __forceinline__ float thermal_cell(const Geo& g, const PhysF& P, const FusedArgs<S>& A, int x, int y, int z,
+                                              bool owner, float* GP) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     const long long c = cell_index(g, x, y, z);
     auto lf = [&](int a, long long cc) { return ldS(A.fin, a * n + cc); };
     auto lg = [&](int a, long long cc) { return ldS(A.gin, a * n + cc); };
+    float d[Q], e[QT];
 #pragma unroll
     for (int a = 0; a < Q; ++a) d[a] = pull_flow<Q, float>(g, a, x, y, z, c, lf);
-    float G[QT], Tprev = 0.0f;
 #pragma unroll
-    for (int a = 0; a < QT; ++a) {
-        G[a] = pull_thermal<QT, float>(g, a, x, y, z, c, lg) + wT<QT>(P, a) * P.Tref;
-        Tprev += G[a];
-    }
-    float Fy;
-    fmacro<D>(d, D == 2 ? A.lag_in[c] : Tprev, P, dr, rho, u, v, w, Fy);
-    if (D == 2) {
-        float Bx = A.Bin0[c], By = A.Bin1[c];
-        fcollideT_2d(G, u, v, Tprev, Bx, By, P, GP);
-        if (owner) {
-            A.Bout0[c] = Bx;
-            A.Bout1[c] = By;
-        }
-    } else {
-        float Bx = A.Bin0[c], By = A.Bin1[c], Bz = A.Bin2[c];
-        fcollideT_3d(G, u, v, w, Tprev, Bx, By, Bz, P, GP);
-        if (owner) {
-            A.Bout0[c] = Bx;
-            A.Bout1[c] = By;
-            A.Bout2[c] = Bz;
-            A.lag_out[c] = Tprev;
+    for (int a = 0; a < QT; ++a) e[a] = pull_thermal<QT, float>(g, a, x, y, z, c, lg);
+    const float Fy = D == 2 ? A.lag_in[c] : 0.0f;
+    float B[3] = {A.Bin0[c], A.Bin1[c], D == 3 ? A.Bin2[c] : 0.0f};
+    const float T = steady_thermal<D>(d, e, Fy, B, P);
+    if (owner) {
+        A.Bout0[c] = B[0];
+        A.Bout1[c] = B[1];
+        if (D == 3) {
+            A.Bout2[c] = B[2];
+            A.lag_out[c] = T;
         }
     }
-    float ev[QT];
     S hs[QT];
-#pragma unroll
-    for (int a = 0; a < QT; ++a) ev[a] = GP[a] - wT<QT>(P, a) * P.Tref;
-    round_cell<QT>(ev, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
+    round_cell<QT>(e, hs, P.sr != 0, sr_seed(*A.tick, c, 1));
 #pragma unroll
     for (int a = 0; a < QT; ++a) {
         if (owner) A.gout[a * n + c] = hs[a];
         GP[a] = stored_value(hs[a]);
     }
+    return D == 2 ? Fy : T;
 }
 
 // Wrap a coordinate along a periodic axis; return -1 when it is outside a walled axis.
@@ -118,25 +104,23 @@ struct Place {
 };
 
 // Thermal stage of plane kp into the ring slot `sgs` (layout [QT][HY][HX]); the own
-// cell's (dr, rho, u, v, w) go to `keep` when keep_own is set.
+// cell's lag goes to `keep` when keep_own is set.
 template <int D, class S, int HX, int HY>
 __device__ __forceinline__ void thermal_plane(const Geo& g, const PhysF& P, const FusedArgs<S>& A, const Place& pl,
-                                              float* sgs, int kp, bool keep_own, float* keep) {
-    constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
+                                              float* sgs, int kp, bool keep_own, float& keep) {
+    constexpr int QT = (D == 2) ? 5 : 7;
     const int gz = (D == 3) ? wrap_or_skip(kp, g.nz, pl.perz) : 0;
     if (gz < 0) return;
     const bool owned = (D == 2) || (kp >= pl.kb && kp < pl.ke);
-    float d[Q], GP[QT], dr, rho, u, v, w;
+    float GP[QT];
     if (pl.own_xy) {
-        thermal_cell<D, S>(g, P, A, pl.x, pl.y, gz, owned, d, dr, rho, u, v, w, GP);
+        const float lag = thermal_cell<D, S>(g, P, A, pl.x, pl.y, gz, owned, GP);
 #pragma unroll
         for (int a = 0; a < QT; ++a) sgs[(a * HY + pl.ty + 1) * HX + pl.tx + 1] = GP[a];
-        if (keep_own) {
-            keep[0] = dr; keep[1] = rho; keep[2] = u; keep[3] = v; keep[4] = w;
-        }
+        if (keep_own) keep = lag;
     }
     if (pl.halo) {
-        thermal_cell<D, S>(g, P, A, pl.hgx, pl.hgy, gz, false, d, dr, rho, u, v, w, GP);
+        thermal_cell<D, S>(g, P, A, pl.hgx, pl.hgy, gz, false, GP);
 #pragma unroll
         for (int a = 0; a < QT; ++a) sgs[(a * HY + pl.hy) * HX + pl.hx] = GP[a];
     }
@@ -145,12 +129,12 @@ __device__ __forceinline__ void thermal_plane(const Geo& g, const PhysF& P, cons
 // Flow stage of the own cell on plane k: f_n pulled again (the thermal stage loaded the
 // same lines one plane earlier), T_n summed from the ring's stored deviations with the
 // thermal wall rules in pull_thermal's order and form (so T_n equals the two-kernel
-// step's bit for bit), then the MRT collision.  m = (dr, rho, u, v, w) of the cell from the
-// thermal stage, whose macro step takes the same pulled f and the same lagged T.
+// step's bit for bit), then the MRT collision, with the lag that the thermal stage's macro
+// step of the same pulled f took.
 template <int D, class S, int HX, int HY>
 __device__ __forceinline__ void flow_cell(const Geo& g, const PhysF& P, const FusedArgs<S>& A, const Place& pl,
                                           const float* s_prev, const float* s_cur, const float* s_next, int k,
-                                          const float* m) {
+                                          float lag) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     if (!pl.own_xy) return;
     const long long n = g.ncell;
@@ -174,20 +158,14 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysF& P, const Fu
                                                          : eopp;
         }
     }
-    const float Tn = ts + P.Tref;  // sum of deviations + Tref * sum(wT)
-    float d[Q], dp[Q];
+    float d[Q];
     auto lf = [&](int a, long long cc) { return ldS(A.fin, a * n + cc); };
 #pragma unroll
     for (int a = 0; a < Q; ++a) d[a] = pull_flow<Q, float>(g, a, x, y, k, c, lf);
-    const float Fy = m[1] * P.gBeta * (Tn - P.Tref);
-    if (D == 2) {
-        A.lag_out[c] = Fy;
-        fcollide_2d(d, m[0], m[1], m[2], m[3], Fy, P, dp);
-    } else {
-        fcollide_3d(d, m[0], m[1], m[2], m[3], m[4], Fy, P, dp);
-    }
+    const float Fy = steady_flow<D>(d, steady_lag<D>(lag, P), ts, P);
+    if (D == 2) A.lag_out[c] = Fy;
     S hs[Q];
-    round_cell<Q>(dp, hs, P.sr != 0, sr_seed(*A.tick + 1, c, 0));
+    round_cell<Q>(d, hs, P.sr != 0, sr_seed(*A.tick + 1, c, 0));
 #pragma unroll
     for (int a = 0; a < Q; ++a) A.fout[a * n + c] = hs[a];
 }
@@ -225,7 +203,7 @@ __global__ void __launch_bounds__(Tile<D>::TX * Tile<D>::TY, Tile<D>::MINB)
     }
     pl.halo = pl.hgx >= 0 && pl.hgy >= 0;
 
-    float mc[5] = {0.f, 1.f, 0.f, 0.f, 0.f}, mn[5] = {0.f, 1.f, 0.f, 0.f, 0.f};
+    float mc = 0.0f, mn = 0.0f;
     if (D == 2) {
         thermal_plane<D, S, HX, HY>(g, P, A, pl, sg, 0, true, mc);
         __syncthreads();
@@ -242,8 +220,7 @@ __global__ void __launch_bounds__(Tile<D>::TX * Tile<D>::TY, Tile<D>::MINB)
         __syncthreads();
         flow_cell<D, S, HX, HY>(g, P, A, pl, sg + sp * SLOT, sg + sc * SLOT, sg + sn * SLOT, k, mc);
         __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 5; ++q) mc[q] = mn[q];
+        mc = mn;
     }
 }
 
