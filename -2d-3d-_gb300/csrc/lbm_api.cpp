@@ -2315,10 +2315,9 @@ extern "C" int lbm_ensemble_get_launch(const lbm_ensemble* e, int* block, int* t
 extern "C" int lbm_ensemble_autotune(lbm_ensemble* e, int nsteps, int* best_block, int* best_tile, int* best_grid) {
     if (!e || nsteps <= 0) return LBM_ERR_PARAM;
     if (e->members.empty()) return LBM_OK;
-    // pairs: bit 0 pairs the 2D members, bit 1 the 3D members
     const EnsLaunchCfg cands[] = {{128, 1024, 16, 1}, {128, 1024, 32, 1}, {128, 1024, 64, 1}, {128, 512, 64, 1},
-                                  {128, 2048, 32, 1}, {256, 2048, 16, 1}, {256, 4096, 8, 1},  {128, 1024, 32, 3},
-                                  {128, 1024, 16, 0}, {128, 1024, 32, 0}, {128, 512, 64, 0},  {256, 2048, 8, 0}};
+                                  {128, 2048, 32, 1}, {128, 2048, 16, 1}, {128, 2048, 8, 1},  {128, 512, 32, 1},
+                                  {128, 256, 64, 1},  {128, 4096, 8, 1},  {128, 4096, 16, 1}, {128, 1024, 6, 1}};
     ECK(e, cudaSetDevice(e->device));
     int st = lbm_ensemble_step(e, 1);  // first steps and ordering
     if (st != LBM_OK) return st;

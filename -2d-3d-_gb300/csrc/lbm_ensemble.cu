@@ -5,8 +5,7 @@
 // (member m, first cell c0) and covers tile_cells consecutive cells of member m.  Each
 // block reads the member's descriptor (geometry, relaxation rates, buffer pointers and
 // parity), then runs the same per-cell bodies as the single-lattice two-kernel step
-// (lbm_fast_cells.cuh, or the paired bodies of lbm_fast_pairs.cuh for members with even
-// nx) on its cells.  Small lattices therefore fill the GPU together instead of one launch
+// (lbm_fast_duo.cuh, or lbm_fast_cells.cuh for members beyond 32-bit indices) on its cells.  Small lattices therefore fill the GPU together instead of one launch
 // each.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -14,7 +13,7 @@
 #include <vector>
 
 #include "lbm_ensemble.h"
-#include "lbm_fast_pairs.cuh"
+#include "lbm_fast_duo.cuh"
 
 namespace lbm {
 
@@ -30,19 +29,9 @@ struct EnsMember {
     int cur;    // buffer parity when the table was built
 };
 
-// Fixed-offset pulls for the cells off the faces (lbm_fast_cells.cuh).  Resident blocks of
-// 256 threads per SM: three, except two for the paired 3D bodies (about 115 registers);
-// four for the paired 2D bodies spills 48-60 bytes and measured no faster on GB300.
-// With the member descriptor and buffer arguments staged in shared memory the one-cell
-// kernels take 66-80 registers, against 96-128 with register copies of the descriptor
-// (the 3D thermal kernel took 242 without a bound), and none spills.
-#ifndef LBM_ENS_PAIR2D_BLOCKS
-#define LBM_ENS_PAIR2D_BLOCKS 3
-#endif
-template <int D>
-constexpr bool kEnsInner = true;
-template <int D, bool PAIR>
-constexpr int kEnsBlocks = (D == 3 && PAIR) ? 2 : (D == 2 && PAIR) ? LBM_ENS_PAIR2D_BLOCKS : 3;
+// Resident blocks of 128 threads per SM (the launch asks for half of them with 256): six, as the
+// single-lattice duo kernels; the one-cell kernels (64-bit indices) take six as well.
+constexpr int kEnsBlocks = 6;
 
 // Cell coordinates of a thread's cells in a tile, stepped instead of divided: one division
 // at the thread's first cell, then (i, j, k) advance by `stride` cells with carries (i by
@@ -98,13 +87,11 @@ __device__ __forceinline__ const EnsStage<S>& stage_member(const EnsMember<S>* _
     return st;
 }
 
-// PAIR: the thread's cells are c and c + 1 (same row: nx even, tiles start on even cells,
-// c even), walked with a stride of two cells per thread.
-template <int D, class S, bool PAIR>
-__global__ void __launch_bounds__(256, (kEnsBlocks<D, PAIR>)) k_ens_flow(const EnsMember<S>* __restrict__ mem,
-                                                                       const int2* __restrict__ tiles, int ntiles,
-                                                                       int tile_cells, int flip) {
-    constexpr int W = PAIR ? 2 : 1;
+// WIDE: one cell per thread with 64-bit indices (members too large for 32-bit ones); otherwise two
+// cells per thread (lbm_fast_duo.cuh), a block taking 2 * blockDim.x cells of its tile at a time.
+template <int D, class S, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEnsBlocks))
+    k_ens_flow(const EnsMember<S>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int tile_cells, int flip) {
     __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int2 tt = tiles[t];
@@ -113,6 +100,7 @@ __global__ void __launch_bounds__(256, (kEnsBlocks<D, PAIR>)) k_ens_flow(const E
             A.lag_in = gm.L[c];
             A.lag_out = gm.L[c ^ 1];
             A.tick = gm.tick;
+            A.ticks = gm.tick;
         });
         const EnsMember<S>& m = st.m;
         const FastArgs<S>& A = st.A;
@@ -121,20 +109,23 @@ __global__ void __launch_bounds__(256, (kEnsBlocks<D, PAIR>)) k_ens_flow(const E
         const int cur = m.cur ^ flip, nxt = cur ^ 1;
         const long long c0 = (long long)tt.y * tile_cells;
         const long long ce = min(c0 + tile_cells, g.ncell);
-        for (CellWalk w(g, c0 + W * (long long)threadIdx.x, W * (int)blockDim.x); w.c < ce; w.next(g)) {
-            if constexpr (PAIR)
-                flow_pair_2k<D, S>(g, P, A, m.f[cur], m.gp[cur], m.f[nxt], w.c, w.i, w.j, w.k);
-            else
-                flow_cell_2k<D, false, S, kEnsInner<D>>(g, P, A, m.f[cur], m.gp[cur], m.f[nxt], w.c, w.i, w.j, w.k);
+        const bool one = tt.y == 0 && threadIdx.x == 0;
+        const unsigned long long tick = sizeof(S) == 2 || one ? flow_tick(A.ticks, one) : 0ULL;
+        if constexpr (WIDE) {
+            for (CellWalk w(g, c0 + (long long)threadIdx.x, (int)blockDim.x); w.c < ce; w.next(g))
+                flow_cell_2k<D, false, S>(g, P, A, m.f[cur], m.gp[cur], m.f[nxt], w.c, w.i, w.j, w.k);
+        } else {
+            for (int c = (int)c0 + 2 * (int)(threadIdx.x & ~31u); c < (int)ce; c += 2 * (int)blockDim.x)
+                flow_duo_2k<D, S>(g, P, A, m.f[cur], m.gp[cur], m.f[nxt], duo_at(g, c + (int)(threadIdx.x & 31u), (int)ce),
+                                  tick);
         }
     }
 }
 
-template <int D, class S, bool PAIR>
-__global__ void __launch_bounds__(256, (kEnsBlocks<D, PAIR>)) k_ens_thermal(const EnsMember<S>* __restrict__ mem,
-                                                                          const int2* __restrict__ tiles, int ntiles,
-                                                                          int tile_cells, int flip) {
-    constexpr int W = PAIR ? 2 : 1;
+template <int D, class S, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEnsBlocks))
+    k_ens_thermal(const EnsMember<S>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int tile_cells,
+                  int flip) {
     __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int2 tt = tiles[t];
@@ -144,7 +135,8 @@ __global__ void __launch_bounds__(256, (kEnsBlocks<D, PAIR>)) k_ens_thermal(cons
             A.Bout0 = gm.B[n][0]; A.Bout1 = gm.B[n][1]; A.Bout2 = gm.B[n][2];
             A.lag_in = gm.L[n];
             A.lag_out = gm.L[n];
-            A.tick = gm.tick;
+            A.tick = gm.tick + 1;  // the copy the flow kernel left
+            A.ticks = gm.tick;
         });
         const EnsMember<S>& m = st.m;
         const FastArgs<S>& A = st.A;
@@ -153,35 +145,28 @@ __global__ void __launch_bounds__(256, (kEnsBlocks<D, PAIR>)) k_ens_thermal(cons
         const int cur = m.cur ^ flip, nxt = cur ^ 1;
         const long long c0 = (long long)tt.y * tile_cells;
         const long long ce = min(c0 + tile_cells, g.ncell);
-        for (CellWalk w(g, c0 + W * (long long)threadIdx.x, W * (int)blockDim.x); w.c < ce; w.next(g)) {
-            if constexpr (PAIR)
-                thermal_pair_2k<D, S>(g, P, A, m.f[nxt], m.gp[cur], m.gp[nxt], w.c, w.i, w.j, w.k);
-            else
-                thermal_cell_2k<D, false, S, kEnsInner<D>>(g, P, A, m.f[nxt], m.gp[cur], m.gp[nxt], w.c, w.i, w.j,
-                                                           w.k);
+        const bool one = tt.y == 0 && threadIdx.x == 0;
+        const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
+        if constexpr (WIDE) {
+            for (CellWalk w(g, c0 + (long long)threadIdx.x, (int)blockDim.x); w.c < ce; w.next(g))
+                thermal_cell_2k<D, false, S>(g, P, A, m.f[nxt], m.gp[cur], m.gp[nxt], w.c, w.i, w.j, w.k);
+        } else {
+            for (int c = (int)c0 + 2 * (int)(threadIdx.x & ~31u); c < (int)ce; c += 2 * (int)blockDim.x)
+                thermal_duo_2k<D, S>(g, P, A, m.f[nxt], m.gp[cur], m.gp[nxt],
+                                     duo_at(g, c + (int)(threadIdx.x & 31u), (int)ce), tick);
         }
     }
 }
 
-// Every member's step counter advances by one after a batched step.
-template <class S>
-__global__ void k_ens_tick(const EnsMember<S>* __restrict__ mem, int nmem) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < nmem) *mem[m].tick += 1ULL;
-}
-
 template <class S>
 static cudaError_t build_typed(EnsPlan& plan, const std::vector<EnsMemberHost>& members) {
-    // a member pairs when the configuration pairs, its rows hold whole pairs, and every tile
-    // starts on an even cell
     for (int li = 0; li < kEnsLists; ++li) {
         const int dim = (li & 1) ? 3 : 2;
-        const bool paired = (li & 2) != 0;
-        const bool pairing = (plan.cfg.pairs & (dim == 3 ? 2 : 1)) != 0 && plan.cfg.tile_cells % 2 == 0;
+        const bool wide = (li & 2) != 0;
         std::vector<EnsMember<S>> hm;
         std::vector<int2> tiles;
         for (const EnsMemberHost& mh : members) {
-            if (mh.dim != dim || (pairing && mh.geo.nx % 2 == 0) != paired) continue;
+            if (mh.dim != dim || ((dim == 3 ? 19LL : 9LL) * mh.geo.ncell >= (1LL << 31) - 64) != wide) continue;
             EnsMember<S> m{};
             m.g = dev_geo(mh.geo, mh.phys);
             m.P = fast_physf(*mh.F, mh.phys);
@@ -233,16 +218,16 @@ cudaError_t ens_build(EnsPlan& plan, const std::vector<EnsMemberHost>& members, 
     return plan.precision == LBM_FP16 ? build_typed<__half>(plan, members) : build_typed<float>(plan, members);
 }
 
-template <int D, class S, bool PAIR>
+template <int D, class S, bool WIDE>
 static void launch_list(const EnsPlan& plan, int li, int stage, int flip, cudaStream_t s) {
+    // a duo block of 128 threads takes the cells that a one-cell block of 256 takes
+    const int block = WIDE ? plan.cfg.block : 128;
     const int grid = min(plan.ntiles[li], plan.sms * plan.cfg.grid_mul);
     const EnsMember<S>* mem = (const EnsMember<S>*)plan.d_members[li];
     if (stage == 0)
-        k_ens_flow<D, S, PAIR><<<grid, plan.cfg.block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li],
-                                                               plan.cfg.tile_cells, flip);
+        k_ens_flow<D, S, WIDE><<<grid, block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells, flip);
     else
-        k_ens_thermal<D, S, PAIR><<<grid, plan.cfg.block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li],
-                                                                  plan.cfg.tile_cells, flip);
+        k_ens_thermal<D, S, WIDE><<<grid, block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells, flip);
 }
 
 template <class S>
@@ -257,11 +242,6 @@ static void step_typed(const EnsPlan& plan, int flip, cudaStream_t s) {
                 default: launch_list<3, S, true>(plan, li, stage, flip, s); break;
             }
         }
-    }
-    for (int li = 0; li < kEnsLists; ++li) {
-        if (plan.nmembers[li] == 0) continue;
-        k_ens_tick<S><<<(plan.nmembers[li] + 127) / 128, 128, 0, s>>>((const EnsMember<S>*)plan.d_members[li],
-                                                                      plan.nmembers[li]);
     }
 }
 

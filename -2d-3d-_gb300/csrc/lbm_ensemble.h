@@ -4,8 +4,8 @@
 // device table of member descriptors (geometry, constants, buffer pointers, buffer
 // parity) and a packed tile table (member, first cell) per member list, and advances every
 // member with one flow and one thermal launch per list and step.  Lists: 2D and 3D members
-// taken one cell per thread, and 2D and 3D members with even nx taken two x-adjacent cells
-// per thread (2-element vector loads and stores) when the launch configuration pairs.
+// taken two cells per thread with packed arithmetic, and those whose cell indices need 64 bits,
+// taken one cell per thread.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -27,10 +27,10 @@ struct EnsLaunchCfg {
     int block = 128;        // threads per block
     int tile_cells = 1024;  // cells per tile (a multiple of `block`)
     int grid_mul = 32;      // grid = min(tiles, SMs * grid_mul)
-    int pairs = 1;          // members with even nx two cells per thread: bit 0 2D, bit 1 3D
+    int pairs = 1;          // kept for callers: every member takes two cells per thread now
 };
 
-// Member lists of a plan: index (dim == 3) + 2 * paired.
+// Member lists of a plan: index (dim == 3) + 2 * wide (64-bit cell indices).
 constexpr int kEnsLists = 4;
 
 struct EnsPlan {
