@@ -67,33 +67,6 @@ __device__ __forceinline__ unsigned short ld_raw(const __half* p) {
 __device__ __forceinline__ float raw_value(float x) { return x; }
 __device__ __forceinline__ float raw_value(unsigned short x) { return __half2float(__ushort_as_half(x)); }
 
-// The lattice's boundary switches as the index rules take them: whether an x (z) face of the set is
-// a wall, and for the thermal set which axes hold constant-temperature walls.
-struct PullRule {
-    bool wx, wz, cx, cy;
-};
-template <bool TH>
-__device__ __forceinline__ PullRule pull_rule(const Geo& g) {
-    if (TH) return {g.bct[0] != LBM_BCT_PERIODIC, g.bct[2] != LBM_BCT_PERIODIC, g.bct[0] == LBM_BCT_CONST,
-                    g.bct[1] == LBM_BCT_CONST};
-    return {g.bcf[0] == LBM_BC_NOSLIP, g.bcf[2] == LBM_BC_NOSLIP, false, false};
-}
-
-// Index of the value that the pull of direction a into a cell reads (pull_flow's and
-// pull_thermal's rule) as selects on the index, not on loaded values: every load of a warp is
-// issued before the first is used.  FACES: the cell's row may lie on a y or z face (the y faces
-// are walls, include/lbm_gpu.h).
-template <int Q, bool FACES>
-__device__ __forceinline__ int pull_index(const Geo& g, int n, const PullRule& r, int a, int i, int j, int k, int c) {
-    const int ex = Lat<Q>::ex(a), ey = Lat<Q>::ey(a), ez = Lat<Q>::ez(a);
-    const int plane = g.nx * g.ny, back = Lat<Q>::opp(a) * n + c, own = a * n + c;
-    int at = own - (ex + g.nx * ey + plane * ez);
-    if (ex != 0) at = (ex > 0 ? i == 0 : i == g.nx - 1) ? (r.wx ? back : own + ex * (g.nx - 1)) : at;
-    if (FACES && ey != 0) at = (ey > 0 ? j == 0 : j == g.ny - 1) ? back : at;
-    if (FACES && ez != 0) at = (ez > 0 ? k == 0 : k == g.nz - 1) ? (r.wz ? back : own + ez * (g.nz - 1) * plane) : at;
-    return at;
-}
-
 // The wall rule of a constant-temperature face on a pulled thermal value.
 template <int QT, bool FACES>
 __device__ __forceinline__ float wall_value(const Geo& g, const PullRule& r, int a, int i, int j, float v) {

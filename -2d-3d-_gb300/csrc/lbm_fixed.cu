@@ -13,17 +13,10 @@ namespace lbm {
 
 using namespace fxa;
 
-// Resident blocks per SM asked of the flow kernels: 5 (96 registers).  GB300, flow half at 128^3 /
-// 256^3: 4 blocks 157 / 1163 us, 5 blocks 146 / 1071 us, 6 blocks (120 B of spill) 145 / 1077 us.
-#ifndef LBM_XFLOW_MIN_BLOCKS
-#define LBM_XFLOW_MIN_BLOCKS 5
-#endif
-// Resident blocks per SM asked of the interior thermal kernel: 7 (70 registers, no spill)
-// ran it 4% faster on GB300 than 6 (80 registers) or 8 (64) at 256^3 and 384^3, at about
-// the HBM copy rate on its measured traffic.
-#ifndef LBM_XTHERMAL_MIN_BLOCKS
-#define LBM_XTHERMAL_MIN_BLOCKS 7
-#endif
+// Resident blocks per SM asked of the steady-state kernels: flow 6 (80 registers, 56 B of spill),
+// thermal 8 (64).  GB300, us per step at 128^3 / 256^3 with 4 and 6 blocks 227 / 1746, 5 and 7
+// 219 / 1690, 6 and 8 215 / 1659.
+constexpr int kXFlowBlocks = 6, kXThermalBlocks = 8;
 
 __device__ __forceinline__ bool fixed_cell_of_thread(const Geo& g, long long& c, int& i, int& j, int& k) {
     c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -50,17 +43,16 @@ __global__ void __launch_bounds__(128) k_xthermal(Geo g, PhysX X, FixedArrays A,
     thermal_cell<D, FIRST>(g, X, A, fin, gin, gout, c, i, j, k);
 }
 
-// Interior rows and face rows of the steady-state step (larger lattices): row_interior_cell and
+// Interior rows and face rows of the steady-state step (64-bit indices): row_interior_cell and
 // row_face_cell (lbm_device.cuh).  Interior rows pull with selects for the x faces; the face
 // kernels take the y- and z-face rows with the full boundary rule.
-// I: int when q * ncell < 2^31 (every array index fits in 32 bits), else long long.
-template <int D, class I>
-__global__ void __launch_bounds__(128, LBM_XFLOW_MIN_BLOCKS) k_xflow_in(Geo g, PhysX X, FixedArrays A, const long long* __restrict__ fin,
+template <int D>
+__global__ void __launch_bounds__(128, kXFlowBlocks) k_xflow_in(Geo g, PhysX X, FixedArrays A, const long long* __restrict__ fin,
                                                      const long long* __restrict__ gin, long long* __restrict__ fout) {
     long long c;
     int i, j, k;
     if (!row_interior_cell(g, c, i, j, k)) return;
-    flow_cell<D, false, 3, I>(g, X, A, fin, gin, fout, c, i, j, k);
+    flow_cell<D, false, 3>(g, X, A, fin, gin, fout, c, i, j, k);
 }
 
 template <int D>
@@ -72,14 +64,14 @@ __global__ void __launch_bounds__(128) k_xflow_face(Geo g, PhysX X, FixedArrays 
     flow_cell<D, false, 2>(g, X, A, fin, gin, fout, c, i, j, k);
 }
 
-template <int D, class I>
-__global__ void __launch_bounds__(128, LBM_XTHERMAL_MIN_BLOCKS) k_xthermal_in(Geo g, PhysX X, FixedArrays A,
+template <int D>
+__global__ void __launch_bounds__(128, kXThermalBlocks) k_xthermal_in(Geo g, PhysX X, FixedArrays A,
                                                         const long long* __restrict__ fin,
                                                         const long long* __restrict__ gin, long long* __restrict__ gout) {
     long long c;
     int i, j, k;
     if (!row_interior_cell(g, c, i, j, k)) return;
-    thermal_cell<D, false, 3, I>(g, X, A, fin, gin, gout, c, i, j, k);
+    thermal_cell<D, false, 3>(g, X, A, fin, gin, gout, c, i, j, k);
 }
 
 template <int D>
@@ -92,37 +84,41 @@ __global__ void __launch_bounds__(128) k_xthermal_face(Geo g, PhysX X, FixedArra
     thermal_cell<D, false, 2>(g, X, A, fin, gin, gout, c, i, j, k);
 }
 
-// The same step on every row in one launch per half (small lattices, row_step): a block holds
-// blockDim.x cells of blockDim.y rows, blockDim.x a multiple of 32, so that the cells of a warp
-// share their row.
-template <int D>
-__device__ __forceinline__ bool row_cell(const Geo& g, long long& c, int& i, int& j, int& k) {
-    i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    k = D == 3 ? (int)blockIdx.z : 0;
-    if (i >= g.nx || j >= g.ny) return false;
-    c = (long long)i + (long long)g.nx * ((long long)j + (long long)g.ny * (long long)k);
-    return true;
+// Steady-state step, one cell per thread in lattice order, every boundary rule as selects on the
+// load indices (32-bit: q * ncell < 2^31).  The kernels are bound by HBM: with branches between
+// the loads a warp waited for some of them one after the other, and rows at the lattice's faces
+// took a launch of their own.  GB300, us per step against interior and face kernels: 2D 128x64
+// 4.4 / 10.4, 2050x1025 123 / 154; 3D 64^3 27 / 46, 128^3 215 / 259, 161x97x131 214 / 310, 256^3
+// 1659 / 1943 with the collision before (6.7 TB/s on 664 B per cell, 0.99 of the copy rate).
+__device__ __forceinline__ bool index_cell(const Geo& g, int& c, int& i, int& j, int& k, bool& rows) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), n = (int)g.ncell;
+    c = min(t, n - 1);
+    const int r = c / g.nx;
+    i = c - r * g.nx;
+    k = g.nz > 1 ? r / g.ny : 0;
+    j = r - k * g.ny;
+    rows = __all_sync(0xFFFFFFFFu, row_off_faces(g, j, k));
+    return t < n;
 }
 
 template <int D>
-__global__ void __launch_bounds__(128, LBM_XFLOW_MIN_BLOCKS) k_xflow_rows(Geo g, PhysX X, FixedArrays A,
-                                                       const long long* __restrict__ fin,
-                                                       const long long* __restrict__ gin, long long* __restrict__ fout) {
-    long long c;
-    int i, j, k;
-    if (!row_cell<D>(g, c, i, j, k)) return;
-    flow_cell<D, false, 4, int>(g, X, A, fin, gin, fout, c, i, j, k);
+__global__ void __launch_bounds__(128, kXFlowBlocks) k_xflow_ix(Geo g, PhysX X, FixedArrays A,
+                                                     const long long* __restrict__ fin,
+                                                     const long long* __restrict__ gin, long long* __restrict__ fout) {
+    int c, i, j, k;
+    bool rows;
+    if (!index_cell(g, c, i, j, k, rows)) return;
+    flow_cell<D, false, 4, int>(g, X, A, fin, gin, fout, c, i, j, k, rows);
 }
 
 template <int D>
-__global__ void __launch_bounds__(128, LBM_XTHERMAL_MIN_BLOCKS) k_xthermal_rows(Geo g, PhysX X, FixedArrays A,
+__global__ void __launch_bounds__(128, kXThermalBlocks) k_xthermal_ix(Geo g, PhysX X, FixedArrays A,
                                                         const long long* __restrict__ fin,
                                                         const long long* __restrict__ gin, long long* __restrict__ gout) {
-    long long c;
-    int i, j, k;
-    if (!row_cell<D>(g, c, i, j, k)) return;
-    thermal_cell<D, false, 4, int>(g, X, A, fin, gin, gout, c, i, j, k);
+    int c, i, j, k;
+    bool rows;
+    if (!index_cell(g, c, i, j, k, rows)) return;
+    thermal_cell<D, false, 4, int>(g, X, A, fin, gin, gout, c, i, j, k, rows);
 }
 
 template <int D>
@@ -370,56 +366,30 @@ void fixed_fused_pass(const Geo& g, const PhysX& X, const long long* fin, const 
 
 
 
-// Largest lattices whose halves run as one launch.  A launch less per half takes 2-3 us off each
-// step, but the flow kernel with both load paths is 2-6% slower per cell than the interior one.
-// GB300, us per step with one launch / two launches per half: 2D 128x64 5.5 / 10.4, 1024x512
-// 34 / 41, 2050x1024 170 / 155; 3D 64^3 35 / 46, 96^3 124.9 / 125.0, 128^3 266 / 259.  The 3D
-// thermal kernel alone: 128^3 108 / 111, 192^3 339 / 353, 256^3 785 / 782.
-constexpr long long kXRowsMaxCells = 1LL << 20;
-constexpr long long kXRowsMaxThermal3d = 8LL << 20;
-
-// Block of the one-launch kernels: 128 threads over as many x cells of a row as leave the
-// fewest warps without a cell, the rest of them over rows.
-template <int D>
-static void row_step(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fprev, const long long* gprev,
-                     long long* fnext, long long* gnext, cudaStream_t s, bool fl, bool th) {
-    const int w = (g.nx + 31) / 32;
-    int bw = 4;
-    for (int x = 3; x >= 1; --x)
-        if ((w + x - 1) / x * x < (w + bw - 1) / bw * bw) bw = x;
-    const dim3 block(32 * bw, 4 / bw, 1);
-    const dim3 grid((w + bw - 1) / bw, (g.ny + block.y - 1) / block.y, D == 3 ? g.nz : 1);
-    if (fl) k_xflow_rows<D><<<grid, block, 0, s>>>(g, X, A, fprev, gprev, fnext);
-    if (th) k_xthermal_rows<D><<<grid, block, 0, s>>>(g, X, A, fnext, gprev, gnext);
-}
-
-// Steady-state step of one dimension: interior kernel and face kernel for each half.
+// Steady-state step of one dimension.
 template <int D>
 static void steady_step(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fprev,
                         const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, bool fl, bool th,
                         bool wide) {
+    constexpr int Q = D == 3 ? 19 : 9;
+    if (!wide && (long long)Q * g.ncell < (1LL << 31)) {
+        const unsigned nb = (unsigned)((g.ncell + 127) / 128);
+        if (fl) k_xflow_ix<D><<<nb, 128, 0, s>>>(g, X, A, fprev, gprev, fnext);
+        if (th) k_xthermal_ix<D><<<nb, 128, 0, s>>>(g, X, A, fnext, gprev, gnext);
+        return;
+    }
+    // 64-bit indices: interior kernel and face kernel for each half
     const unsigned bx = (unsigned)((g.nx + 127) / 128);
     const dim3 bin(128), gin_grid(bx, (unsigned)(g.ny - 2), D == 3 ? (unsigned)(g.nz - 2) : 1u);
     const dim3 gface(bx, (unsigned)face_row_count(g), 1u);
     // a 3D lattice of two planes has no interior rows: the face rows hold every cell
     const bool interior = D == 2 || g.nz > 2;
-    constexpr int Q = D == 3 ? 19 : 9;
-    const bool idx32 = !wide && (long long)Q * g.ncell < (1LL << 31);
-    // 32-bit indices and a grid that holds every row
-    const bool rows = idx32 && g.ny <= 65535 && g.nz <= 65535;
-    const bool small = rows && g.ncell <= kXRowsMaxCells;
-    if (fl && small) {
-        row_step<D>(g, X, A, fprev, gprev, fnext, gnext, s, true, false);
-    } else if (fl) {
-        if (interior && idx32) k_xflow_in<D, int><<<gin_grid, bin, 0, s>>>(g, X, A, fprev, gprev, fnext);
-        else if (interior) k_xflow_in<D, long long><<<gin_grid, bin, 0, s>>>(g, X, A, fprev, gprev, fnext);
+    if (fl) {
+        if (interior) k_xflow_in<D><<<gin_grid, bin, 0, s>>>(g, X, A, fprev, gprev, fnext);
         k_xflow_face<D><<<gface, bin, 0, s>>>(g, X, A, fprev, gprev, fnext);
     }
-    if (th && rows && (small || (D == 3 && g.ncell <= kXRowsMaxThermal3d))) {
-        row_step<D>(g, X, A, fprev, gprev, fnext, gnext, s, false, true);
-    } else if (th) {
-        if (interior && idx32) k_xthermal_in<D, int><<<gin_grid, bin, 0, s>>>(g, X, A, fnext, gprev, gnext);
-        else if (interior) k_xthermal_in<D, long long><<<gin_grid, bin, 0, s>>>(g, X, A, fnext, gprev, gnext);
+    if (th) {
+        if (interior) k_xthermal_in<D><<<gin_grid, bin, 0, s>>>(g, X, A, fnext, gprev, gnext);
         k_xthermal_face<D><<<gface, bin, 0, s>>>(g, X, A, fnext, gprev, gnext);
     }
 }

@@ -668,20 +668,51 @@ struct FixedArrays {
 
 namespace fxa {
 
+// Both population sets pulled into one cell by index (PATH 4 below).
+template <int Q, bool TH, bool FACES>
+__device__ __forceinline__ void pull_set(const Geo& g, const PhysX& X, const long long* f, int c, int i, int j, int k,
+                                         q60* v) {
+    const PullRule r = pull_rule<TH>(g);
+#pragma unroll
+    for (int a = 0; a < Q; ++a) v[a] = ldq(f, pull_index<Q, FACES>(g, (int)g.ncell, r, a, i, j, k, c));
+    if (!TH) return;
+#pragma unroll
+    for (int a = 0; a < Q; ++a) {  // constant-temperature walls
+        const int ex = Lat<Q>::ex(a), ey = Lat<Q>::ey(a);
+        if (ex != 0 && r.cx && (ex > 0 ? i == 0 : i == g.nx - 1)) v[a] = Qb(ex > 0 ? X.bc_lo[0] : X.bc_hi[0]) - v[a];
+        if (FACES && ey != 0 && r.cy && (ey > 0 ? j == 0 : j == g.ny - 1))
+            v[a] = Qb(ey > 0 ? X.bc_lo[1] : X.bc_hi[1]) - v[a];
+    }
+}
+template <int D>
+__device__ __forceinline__ void pull_cell(const Geo& g, const PhysX& X, const long long* fin, const long long* gin,
+                                          long long c, int i, int j, int k, bool rows, q60* d, q60* e) {
+    constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
+    if (rows) {
+        pull_set<Q, false, false>(g, X, fin, (int)c, i, j, k, d);
+        pull_set<QT, true, false>(g, X, gin, (int)c, i, j, k, e);
+    } else {
+        pull_set<Q, false, true>(g, X, fin, (int)c, i, j, k, d);
+        pull_set<QT, true, true>(g, X, gin, (int)c, i, j, k, e);
+    }
+}
+
 // Flow collision of step n (lbm_exact.cu k_flow): FIRST reads the module arrays (f, rho,
 // u, T); otherwise f_{n-1} = pull(f_post_{n-1}), T_{n-1} = sum pull(g_post_{n-1}), and rho,
 // u of the macro step of f_{n-1} with the lag.  2D stores the force F_y,n in the lag.
 // g: geometry whose thermal wall terms are deviations (wall term - 2 wT Tref).
 // PATH: 0 = any cell (the boundary rule where a pull leaves the lattice), 1 = a cell known to
 // touch no face (fixed-offset pulls only), 2 = a face cell (boundary path only), 3 = a cell of
-// an interior row (only x can leave the lattice: pull_flow_xrow / pull_thermal_xrow), 4 = a cell
-// of any row: PATH 3's loads on an interior row, the boundary path's on the others (a warp holds
-// cells of one row, so the choice does not diverge, and only the loads are inside it).
+// an interior row (only x can leave the lattice: pull_flow_xrow / pull_thermal_xrow), 4 = any cell,
+// with the boundary rule as selects on the load index (pull_index; 32-bit indices): all loads of a
+// warp are in flight before the first is used.  rows (PATH 4): no cell of the warp lies on a row
+// of a y or z face, so only the x faces are selected for.
 // I: index type of the cell's own accesses and of PATH 3's pulls (int when every array
 // index fits in 32 bits: half the address arithmetic; the values do not depend on it).
 template <int D, bool FIRST, int PATH = 0, class I = long long>
 __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fin,
-                                          const long long* gin, long long* fout, long long c, int i, int j, int k) {
+                                          const long long* gin, long long* fout, long long c, int i, int j, int k,
+                                          bool rows = true) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     const I ni = (I)g.ncell, ci = (I)c;
@@ -698,7 +729,12 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const Fi
         tdev = q60(A.T[c]) - Qb(X.tref);
     } else {
         q60 ts = Qb(0);
-        if (PATH == 3 || (PATH == 4 && row_off_faces(g, j, k))) {
+        if (PATH == 4) {
+            q60 e[QT];
+            pull_cell<D>(g, X, fin, gin, c, i, j, k, rows, d, e);
+#pragma unroll
+            for (int a = 0; a < QT; ++a) ts = ts + e[a];
+        } else if (PATH == 3) {
             auto lf = [&](int a, I cc) { return ldq(fin, a * ni + cc); };
             auto lg = [&](int a, I cc) { return ldq(gin, a * ni + cc); };
 #pragma unroll
@@ -739,15 +775,17 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const Fi
 // Streaming, boundary and macro of the flow, and thermal collision of step n (k_thermal).
 template <int D, bool FIRST, int PATH = 0, class I = long long>
 __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fin,
-                                             const long long* gin, long long* gout, long long c, int i, int j, int k) {
+                                             const long long* gin, long long* gout, long long c, int i, int j, int k,
+                                             bool rows = true) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     const I ni = (I)g.ncell, ci = (I)c;
     q60 d[Q], e[QT], ep[QT], rho, P[3], U[3], B[3], F, tdev;
     const bool inner = PATH == 1 || (PATH == 0 && aa_inner(g, i, j, k));
     auto lf = [&](int a, long long cc) { return ldq(fin, a * n + cc); };
-    const bool inrow = PATH == 3 || (PATH == 4 && row_off_faces(g, j, k));
-    if (inrow) {
+    if (PATH == 4) {
+        pull_cell<D>(g, X, fin, gin, c, i, j, k, rows, d, e);
+    } else if (PATH == 3) {
         auto lfi = [&](int a, I cc) { return ldq(fin, a * ni + cc); };
 #pragma unroll
         for (int a = 0; a < Q; ++a) d[a] = pull_flow_xrow<Q, q60>(g, a, i, ci, lfi);
@@ -767,7 +805,10 @@ __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const
         B[2] = D == 3 ? q60(A.Bz[c]) : Qb(0);
     } else {
         q60 ts = Qb(0);
-        if (inrow) {
+        if (PATH == 4) {
+#pragma unroll
+            for (int a = 0; a < QT; ++a) ts = ts + e[a];
+        } else if (PATH == 3) {
             auto lg = [&](int a, I cc) { return ldq(gin, a * ni + cc); };
 #pragma unroll
             for (int a = 0; a < QT; ++a) {

@@ -1,6 +1,6 @@
-"""The one-launch row kernels of the fixed arithmetic against its interior and face kernels (64-bit
-indices force those), bit for bit: row lengths at the edges of a warp and of a block, rows at the
-edges of a block, walls and periodic faces, lattices on both sides of the size rule."""
+"""The fixed arithmetic's kernels with 32-bit indices (boundary rules as selects on the load index)
+against its interior and face kernels (64-bit indices force those), bit for bit: row lengths at
+the edges of a warp and of a block, lattices that end inside a block, walls and periodic faces."""
 import numpy as np
 import pytest
 
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
     (2, 5, 5, 1, True), (2, 31, 6, 1, False), (2, 33, 7, 1, True), (2, 64, 9, 1, True), (2, 97, 5, 1, False),
     (2, 129, 13, 1, True), (2, 1025, 1024, 1, False), (3, 5, 5, 2, False), (3, 32, 5, 3, True), (3, 65, 7, 5, False),
     (3, 96, 8, 4, True), (3, 130, 6, 5, False), (3, 105, 100, 101, True)])
-def test_row_kernels_equal_interior_and_face_kernels(gpu_lib, dim, nx, ny, nz, periodic):
+def test_index_kernels_equal_interior_and_face_kernels(gpu_lib, dim, nx, ny, nz, periodic):
     p = rb_params(dim=dim, nx=nx, ny=ny, nz=nz, Ra=1e5, noise_amp=1e-2, precision="fp64x", periodic_x=periodic)
     if dim == 3 and periodic:
         p.bc_flow[2], p.bc_thermal[2] = 1, 2
