@@ -258,11 +258,14 @@ __host__ __device__ __forceinline__ PullRule pull_rule(const Geo& g) {
 // Index of the value that the pull of direction a into a cell reads (pull_flow's and
 // pull_thermal's rule) as selects on the index, not on loaded values: every load of a warp is
 // issued before the first is used.  FACES: the cell's row may lie on a y or z face (the y faces
-// are walls, include/lbm_gpu.h).
-template <int Q, bool FACES>
-__host__ __device__ __forceinline__ int pull_index(const Geo& g, int n, const PullRule& r, int a, int i, int j, int k, int c) {
+// are walls, include/lbm_gpu.h).  SWAP: the array is in the swapped layout of the in-place
+// pattern, direction a of a cell in plane opp(a).
+template <int Q, bool FACES, bool SWAP = false>
+__host__ __device__ __forceinline__ int pull_index(const Geo& g, int n, const PullRule& r, int a, int i, int j, int k,
+                                                   int c) {
     const int ex = Lat<Q>::ex(a), ey = Lat<Q>::ey(a), ez = Lat<Q>::ez(a);
-    const int plane = g.nx * g.ny, back = Lat<Q>::opp(a) * n + c, own = a * n + c;
+    const int plane = g.nx * g.ny;
+    const int own = (SWAP ? Lat<Q>::opp(a) : a) * n + c, back = (SWAP ? a : Lat<Q>::opp(a)) * n + c;
     int at = own - (ex + g.nx * ey + plane * ez);
     if (ex != 0) at = (ex > 0 ? i == 0 : i == g.nx - 1) ? (r.wx ? back : own + ex * (g.nx - 1)) : at;
     if (FACES && ey != 0) at = (ey > 0 ? j == 0 : j == g.ny - 1) ? back : at;

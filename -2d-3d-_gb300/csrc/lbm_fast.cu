@@ -421,9 +421,9 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
     const int cur = F.cur, nxt = F.cur ^ 1;
     if (F.aa) {
         F.ahead = false;
-        fast_step_aa(F, g, pf, dim, first, s, part);
+        const bool ticked = fast_step_aa(F, g, pf, dim, first, s, part);
         if (part != 0) {
-            fast_tick(F, s);
+            if (!ticked) fast_tick(F, s);
             F.cur = nxt;
             F.fused_valid = true;
         }

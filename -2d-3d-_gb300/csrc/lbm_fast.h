@@ -82,8 +82,9 @@ void fast_wait_selftest(FastState& F, unsigned limit, cudaStream_t s);
 PhysF fast_physf(const FastState& F, const PhysC& P);
 // Advance the step counter by one step (after a step's thermal kernel).
 void fast_tick(FastState& F, cudaStream_t s);
-// In-place pattern step and materialisation (lbm_fast_aa.cu); g is the deviation geometry.
-void fast_step_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, bool first, cudaStream_t s, int part);
+// In-place pattern step and materialisation (lbm_fast_aa.cu); g is the deviation geometry.  The
+// step returns whether its kernels advance the step counter.
+bool fast_step_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, bool first, cudaStream_t s, int part);
 void fast_materialize_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, cudaStream_t s);
 // Rebuild the module arrays (f, g, rho, u, v, w, T) of the current step; leaves the fused
 // buffers valid.  In-place pattern: the module scalars only (the arrays are the populations).

@@ -13,6 +13,7 @@
 #include "lbm_fast_cells.cuh"
 #include "lbm_fast_pairs.cuh"
 #include "lbm_fast_aa.cuh"
+#include "lbm_fast_aa_duo.cuh"
 
 namespace lbm {
 
@@ -399,6 +400,23 @@ __global__ void __launch_bounds__(128) k_aa_thermal_p(Geo g, PhysF P, FastArgs<S
     }
 }
 
+// Two cells per thread, 32 apart (lbm_fast_aa_duo.cuh): resident blocks as for the two-buffer
+// kernels (lbm_fast.cu).
+template <int D, class S, bool ODD>
+__global__ void __launch_bounds__(128, 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs<S> A, S* f, const S* __restrict__ gs,
+                                                     int raw) {
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+    const unsigned long long tick = sizeof(S) == 2 || one ? flow_tick(A.ticks, one) : 0ULL;
+    aa_flow_duo<D, S, ODD>(g, P, A, f, gs, raw != 0, duo_cells<true>(g), tick);
+}
+template <int D, class S, bool ODD>
+__global__ void __launch_bounds__(128, 7) k_aa_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fs, S* gg,
+                                                        int raw) {
+    const bool one = blockIdx.x == 0 && threadIdx.x == 0;
+    const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
+    aa_thermal_duo<D, S, ODD>(g, P, A, fs, gg, raw != 0, duo_cells<true>(g), tick);
+}
+
 // ------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------
@@ -413,6 +431,7 @@ static FastArgs<S> aa_args(const FastState& F) {
     a.lag_in = F.L[0];
     a.lag_out = F.L[0];
     a.tick = F.tick;
+    a.ticks = F.tick;
     return a;
 }
 
@@ -425,19 +444,37 @@ static bool any_face(void* const face[3]) { return face[0] || face[1] || face[2]
 
 bool fast_aa_tma_sweep(FastState& F, const Geo& g, const PhysF& pf, int dim, const void* A, int part, cudaStream_t s);
 
+// Returns whether the sweeps advance the step counter themselves (the duo kernels).
 template <int D, class S, bool FIRST>
-static void aa_step_launch(FastState& F, const Geo& g, const PhysF& pf, cudaStream_t s, int part) {
+static bool aa_step_launch(FastState& F, const Geo& g, const PhysF& pf, cudaStream_t s, int part) {
     AAState& st = F.AA;
     const FastArgs<S> A = aa_args<S>(F);
     S* f = (S*)F.fbuf[0];
     S* gg = (S*)F.gbuf[0];
     const unsigned nb = (unsigned)((g.ncell + 127) / 128);
     const int raw = st.graw ? 1 : 0;
-    // Forms measured on GB300 (3D, 128^3 to 384^3): the even flow sweep, whose loads and
-    // stores are all the cell's own slots, is fastest with two cells per thread; every other
-    // sweep with one cell per thread (LBM_OPT_PAIRS / LBM_OPT_STAGED select the paired or
-    // staged form for them).  The first step (module arrays) and odd nx take one cell per
-    // thread.
+    // Walls on every face, indices that fit 32 bits and the regular parities (both arrays in one
+    // layout before the flow sweep): two cells per thread.  GB300, us per step against the forms
+    // below: 384^3 FP16 2896 / 2206, FP32 2991 / 2766; 96^3 FP16 59 / 33.
+    // Otherwise the even flow sweep, whose loads and stores are all the cell's own slots, takes
+    // two x-adjacent cells per thread (even nx) and every other sweep one (LBM_OPT_PAIRS /
+    // LBM_OPT_STAGED select the paired or staged form for them).
+    if (!FIRST && !F.pairs && !F.tma && !F.wide && !any_face(st.face_f) && !any_face(st.face_g) &&
+        (long long)F.q * g.ncell < (1LL << 31) - 64 && (part == 1 ? st.fpar != st.gpar : st.fpar == st.gpar)) {
+        const unsigned nb2 = (unsigned)((g.ncell + 255) / 256);
+        if (part != 1) {
+            if (st.fpar) k_aa_flow_duo<D, S, true><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
+            else k_aa_flow_duo<D, S, false><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
+            st.fpar ^= 1;
+        }
+        if (part != 0) {
+            if (st.gpar) k_aa_thermal_duo<D, S, true><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
+            else k_aa_thermal_duo<D, S, false><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
+            if (st.gpar) st.graw = true;
+            st.gpar ^= 1;
+        }
+        return true;
+    }
     const bool paired = !FIRST && F.pairs && g.nx % 2 == 0;
     const bool paired_even_flow = !FIRST && g.nx % 2 == 0 && st.fpar == 0;
     const int pairs = g.nx / 2, bx = pairs > 32 ? 64 : 32, by = 128 / bx;
@@ -474,22 +511,20 @@ static void aa_step_launch(FastState& F, const Geo& g, const PhysF& pf, cudaStre
         if (st.gpar) st.graw = true;
         st.gpar ^= 1;
     }
+    return false;
 }
 
 template <int D, class S>
-static void aa_step_first(FastState& F, const Geo& g, const PhysF& pf, bool first, cudaStream_t s, int part) {
-    if (first) aa_step_launch<D, S, true>(F, g, pf, s, part);
-    else aa_step_launch<D, S, false>(F, g, pf, s, part);
+static bool aa_step_first(FastState& F, const Geo& g, const PhysF& pf, bool first, cudaStream_t s, int part) {
+    return first ? aa_step_launch<D, S, true>(F, g, pf, s, part) : aa_step_launch<D, S, false>(F, g, pf, s, part);
 }
 
-void fast_step_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, bool first, cudaStream_t s, int part) {
-    if (F.precision == LBM_FP16) {
-        if (dim == 2) aa_step_first<2, __half>(F, g, pf, first, s, part);
-        else aa_step_first<3, __half>(F, g, pf, first, s, part);
-    } else {
-        if (dim == 2) aa_step_first<2, float>(F, g, pf, first, s, part);
-        else aa_step_first<3, float>(F, g, pf, first, s, part);
-    }
+bool fast_step_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, bool first, cudaStream_t s, int part) {
+    if (F.precision == LBM_FP16)
+        return dim == 2 ? aa_step_first<2, __half>(F, g, pf, first, s, part)
+                        : aa_step_first<3, __half>(F, g, pf, first, s, part);
+    return dim == 2 ? aa_step_first<2, float>(F, g, pf, first, s, part)
+                    : aa_step_first<3, float>(F, g, pf, first, s, part);
 }
 
 void fast_materialize_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, cudaStream_t s) {

@@ -15,13 +15,17 @@
 namespace lbm {
 
 struct Duo {
-    int c[2];     // the cells (clamped into the lattice)
-    bool in[2];   // whether each exists
+    int c[2];     // the cells
+    bool in[2];   // whether the lane has them
     int i[2], j[2], k[2];
     bool rows;    // every cell of the warp lies on a row off the y and z faces
 };
 
-// Cells c0 and c0 + 32 of a lane (called by whole warps), those below `end`.
+// Cells c0 and c0 + 32 of a lane (called by whole warps), those below `end`.  A cell beyond the
+// lattice is read as its last one and not stored.  OWN (in-place sweeps, where that cell's slots
+// are being written): a lane without a second cell repeats its first, and one without a first
+// takes no part.
+template <bool OWN = false>
 __device__ __forceinline__ Duo duo_at(const Geo& g, int c0, int end) {
     Duo t;
     const int last = (int)g.ncell - 1;
@@ -45,18 +49,20 @@ __device__ __forceinline__ Duo duo_at(const Geo& g, int c0, int end) {
         t.k[1] = g.nz > 1 ? r1 / g.ny : 0;
         t.j[1] = r1 - t.k[1] * g.ny;
     }
-    if (c0 + 32 > last) {  // clamped: any cell of the lattice will do
-        t.i[1] = g.nx - 1;
-        t.j[1] = g.ny - 1;
-        t.k[1] = g.nz - 1;
+    if (c0 + 32 > last) {
+        t.c[1] = OWN ? t.c[0] : last;
+        t.i[1] = OWN ? t.i[0] : g.nx - 1;
+        t.j[1] = OWN ? t.j[0] : g.ny - 1;
+        t.k[1] = OWN ? t.k[0] : g.nz - 1;
     }
     const bool off = row_off_faces(g, t.j[0], t.k[0]) && row_off_faces(g, t.j[1], t.k[1]);
     t.rows = __all_sync(0xFFFFFFFFu, off);
     return t;
 }
 // The cells of a single-lattice launch (ncell / 256 blocks of 128 threads, rounded up).
+template <bool OWN = false>
 __device__ __forceinline__ Duo duo_cells(const Geo& g) {
-    return duo_at(g, (int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * 2 + (int)(threadIdx.x & 31u), (int)g.ncell);
+    return duo_at<OWN>(g, (int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * 2 + (int)(threadIdx.x & 31u), (int)g.ncell);
 }
 
 // A stored population as loaded, and its value.
@@ -83,7 +89,7 @@ __device__ __forceinline__ float wall_value(const Geo& g, const PullRule& r, int
 }
 
 // The Q populations of one set pulled into both cells.
-template <int Q, bool TH, bool FACES, class S>
+template <int Q, bool TH, bool FACES, class S, bool SWAP = false>
 __device__ __forceinline__ void duo_pull_set(const Geo& g, const S* __restrict__ f, const Duo& t, f2* d) {
     const int n = (int)g.ncell;
     const PullRule r = pull_rule<TH>(g);
@@ -92,7 +98,7 @@ __device__ __forceinline__ void duo_pull_set(const Geo& g, const S* __restrict__
     for (int a = 0; a < Q; ++a) {
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-            x[h][a] = ld_raw(f + pull_index<Q, FACES>(g, n, r, a, t.i[h], t.j[h], t.k[h], t.c[h]));
+            x[h][a] = ld_raw(f + pull_index<Q, FACES, SWAP>(g, n, r, a, t.i[h], t.j[h], t.k[h], t.c[h]));
     }
 #pragma unroll
     for (int a = 0; a < Q; ++a) {
