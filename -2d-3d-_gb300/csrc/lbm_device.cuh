@@ -273,6 +273,44 @@ __host__ __device__ __forceinline__ int pull_index(const Geo& g, int n, const Pu
     return at;
 }
 
+#if defined(__CUDACC__)
+// Cell of a thread in lattice order with 32-bit indices (called by whole warps; a thread past the
+// lattice gets its last cell and false).  rows: no cell of the warp lies on a row of a y or z
+// face, so its pulls select for the x faces only (FACES of pull_index).
+__device__ __forceinline__ bool index_cell(const Geo& g, int& c, int& i, int& j, int& k, bool& rows) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), n = (int)g.ncell;
+    c = min(t, n - 1);
+    const int r = c / g.nx;
+    i = c - r * g.nx;
+    k = g.nz > 1 ? r / g.ny : 0;
+    j = r - k * g.ny;
+    rows = __all_sync(0xFFFFFFFFu, row_off_faces(g, j, k));
+    return t < n;
+}
+#endif
+
+// The Q values of one set pulled into a cell by index, LOAD(index) in the arithmetic type T: what
+// pull_flow and pull_thermal return.
+template <int Q, bool TH, bool FACES, class T, class LOAD>
+__device__ __forceinline__ void pull_set_index(const Geo& g, int i, int j, int k, int c, LOAD load, T* v) {
+    const PullRule r = pull_rule<TH>(g);
+#pragma unroll
+    for (int a = 0; a < Q; ++a) v[a] = load(pull_index<Q, FACES>(g, (int)g.ncell, r, a, i, j, k, c));
+    if (!TH) return;
+#pragma unroll
+    for (int a = 0; a < Q; ++a) {  // constant-temperature walls
+        const int ex = Lat<Q>::ex(a), ey = Lat<Q>::ey(a);
+        if (ex != 0 && r.cx && (ex > 0 ? i == 0 : i == g.nx - 1)) v[a] = -v[a] + (T)(ex > 0 ? g.bcT_lo[0] : g.bcT_hi[0]);
+        if (FACES && ey != 0 && r.cy && (ey > 0 ? j == 0 : j == g.ny - 1))
+            v[a] = -v[a] + (T)(ey > 0 ? g.bcT_lo[1] : g.bcT_hi[1]);
+    }
+}
+template <int Q, bool TH, class T, class LOAD>
+__device__ __forceinline__ void pull_set_rows(const Geo& g, bool rows, int i, int j, int k, int c, LOAD load, T* v) {
+    if (rows) pull_set_index<Q, TH, false, T>(g, i, j, k, c, load, v);
+    else pull_set_index<Q, TH, true, T>(g, i, j, k, c, load, v);
+}
+
 // ------------------------------------------------------------------------------------
 // In-place (AA) access pattern.  One array per lattice; its layout alternates:
 //   parity 0 ("streamed"): slot (a, x) holds the streamed population f_a(x), i.e. what the

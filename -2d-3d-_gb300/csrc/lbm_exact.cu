@@ -310,12 +310,22 @@ __device__ __forceinline__ void thermal_cell(const PhysC& P, const ExactArrays& 
 // sum pull(g_post_{n-1}) (stored for the thermal kernel), and rho, u_{n-1} and the momentum
 // sums from the previous thermal kernel, which computed them from the same f_{n-1} with the
 // lag (3D: T_{n-2}; 2D: the force F_{n-1} stored by the previous flow collision).
-template <int D, bool FIRST>
+// NARROW: every index fits in 32 bits, and the boundary rules are selects on the load index
+// (pull_set_index); otherwise the branching pulls with 64-bit indices.
+template <int D, bool FIRST, bool NARROW>
 __global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, const double* __restrict__ fin,
                                               const double* __restrict__ gin, double* __restrict__ fout) {
     long long c;
     int i, j, k;
-    if (!thread_cell(g, c, i, j, k)) return;
+    bool rows = false;
+    if (NARROW) {
+        int ci;
+        const bool in = index_cell(g, ci, i, j, k, rows);
+        if (!in) return;
+        c = ci;
+    } else if (!thread_cell(g, c, i, j, k)) {
+        return;
+    }
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     double F[Q], FP[Q], T, jx = 0.0, jy = 0.0, jz = 0.0;
@@ -327,13 +337,18 @@ __global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, con
         for (int a = 0; a < Q; ++a) F[a] = A.f[a * n + c];
         T = A.T[c];
     } else {
-        auto lf = [&](int a, long long cc) { return fin[a * n + cc]; };
-        auto lg = [&](int a, long long cc) { return gin[a * n + cc]; };
-#pragma unroll
-        for (int a = 0; a < Q; ++a) F[a] = pull_flow<Q, double>(g, a, i, j, k, c, lf);
         double G[QT];
+        if (NARROW) {
+            pull_set_rows<Q, false, double>(g, rows, i, j, k, (int)c, [&](int x) { return fin[x]; }, F);
+            pull_set_rows<QT, true, double>(g, rows, i, j, k, (int)c, [&](int x) { return gin[x]; }, G);
+        } else {
+            auto lf = [&](int a, long long cc) { return fin[a * n + cc]; };
+            auto lg = [&](int a, long long cc) { return gin[a * n + cc]; };
 #pragma unroll
-        for (int a = 0; a < QT; ++a) G[a] = pull_thermal<QT, double>(g, a, i, j, k, c, lg);
+            for (int a = 0; a < Q; ++a) F[a] = pull_flow<Q, double>(g, a, i, j, k, c, lf);
+#pragma unroll
+            for (int a = 0; a < QT; ++a) G[a] = pull_thermal<QT, double>(g, a, i, j, k, c, lg);
+        }
         T = sumT<QT>(G);
         A.T[c] = T;  // T_{n-1}, the thermal kernel's n0 of the same pulled populations
         jx = A.jx[c];
@@ -355,23 +370,37 @@ __global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, con
 // Streaming + boundary + macro of the flow and thermal collision of step n
 // (B_n .. D_n).  FIRST: g_{n-1} and T_{n-1} are the module arrays; otherwise T_{n-1} is the
 // flow kernel's sum of the same pulled g_{n-1}.
-template <int D, bool FIRST>
+template <int D, bool FIRST, bool NARROW>
 __global__ void __launch_bounds__(128) k_thermal(Geo g, PhysC P, ExactArrays A, const double* __restrict__ fin,
                                                  const double* __restrict__ gin, double* __restrict__ gout) {
     long long c;
     int i, j, k;
-    if (!thread_cell(g, c, i, j, k)) return;
+    bool rows = false;
+    if (NARROW) {
+        int ci;
+        const bool in = index_cell(g, ci, i, j, k, rows);
+        if (!in) return;
+        c = ci;
+    } else if (!thread_cell(g, c, i, j, k)) {
+        return;
+    }
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
     double F[Q], G[QT], GP[QT];
-    auto lf = [&](int a, long long cc) { return fin[a * n + cc]; };
+    if (NARROW) {
+        pull_set_rows<Q, false, double>(g, rows, i, j, k, (int)c, [&](int x) { return fin[x]; }, F);
+    } else {
+        auto lf = [&](int a, long long cc) { return fin[a * n + cc]; };
 #pragma unroll
-    for (int a = 0; a < Q; ++a) F[a] = pull_flow<Q, double>(g, a, i, j, k, c, lf);
+        for (int a = 0; a < Q; ++a) F[a] = pull_flow<Q, double>(g, a, i, j, k, c, lf);
+    }
     // T_{n-1}: the module T, or the flow kernel's sum of the same pulled g_{n-1}
     const double Tprev = A.T[c];
     if (FIRST) {
 #pragma unroll
         for (int a = 0; a < QT; ++a) G[a] = A.g[a * n + c];
+    } else if (NARROW) {
+        pull_set_rows<QT, true, double>(g, rows, i, j, k, (int)c, [&](int x) { return gin[x]; }, G);
     } else {
         auto lg = [&](int a, long long cc) { return gin[a * n + cc]; };
 #pragma unroll
@@ -702,28 +731,29 @@ void exact_stage(int stage, const Geo& g, const PhysC& P, const ExactArrays& A, 
 // hold one block more than the others (the FP64 kernels are bound by each SM's FP64 pipe).
 static inline int step_block(const Geo& g) { return g.ncell < 65536 ? 32 : 128; }
 
-void exact_fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, bool first, const double* fprev,
-                      const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part) {
+template <int D>
+static void fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, bool first, const double* fprev,
+                       const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part) {
     const int bs = step_block(g);
     const unsigned nb = nblocks(g.ncell, bs);
     const bool fl = part != 1, th = part != 0;
-    if (dim == 2) {
-        if (first) {
-            if (fl) k_flow<2, true><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
-            if (th) k_thermal<2, true><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
-        } else {
-            if (fl) k_flow<2, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
-            if (th) k_thermal<2, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
-        }
+    const bool narrow = (D == 3 ? 19LL : 9LL) * g.ncell < (1LL << 31);
+    if (first) {
+        if (fl) k_flow<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
+        if (th) k_thermal<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
+    } else if (narrow) {
+        if (fl) k_flow<D, false, true><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
+        if (th) k_thermal<D, false, true><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
     } else {
-        if (first) {
-            if (fl) k_flow<3, true><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
-            if (th) k_thermal<3, true><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
-        } else {
-            if (fl) k_flow<3, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
-            if (th) k_thermal<3, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
-        }
+        if (fl) k_flow<D, false, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
+        if (th) k_thermal<D, false, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
     }
+}
+
+void exact_fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, bool first, const double* fprev,
+                      const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part) {
+    if (dim == 2) fused_step<2>(g, P, A, first, fprev, gprev, fnext, gnext, s, part);
+    else fused_step<3>(g, P, A, first, fprev, gprev, fnext, gnext, s, part);
 }
 
 static AAFace<double> aa_faces(void* const face[3]) {

@@ -90,17 +90,6 @@ __global__ void __launch_bounds__(128) k_xthermal_face(Geo g, PhysX X, FixedArra
 // took a launch of their own.  GB300, us per step against interior and face kernels: 2D 128x64
 // 4.4 / 10.4, 2050x1025 123 / 154; 3D 64^3 27 / 46, 128^3 215 / 259, 161x97x131 214 / 310, 256^3
 // 1659 / 1943 with the collision before (6.7 TB/s on 664 B per cell, 0.99 of the copy rate).
-__device__ __forceinline__ bool index_cell(const Geo& g, int& c, int& i, int& j, int& k, bool& rows) {
-    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), n = (int)g.ncell;
-    c = min(t, n - 1);
-    const int r = c / g.nx;
-    i = c - r * g.nx;
-    k = g.nz > 1 ? r / g.ny : 0;
-    j = r - k * g.ny;
-    rows = __all_sync(0xFFFFFFFFu, row_off_faces(g, j, k));
-    return t < n;
-}
-
 template <int D>
 __global__ void __launch_bounds__(128, kXFlowBlocks) k_xflow_ix(Geo g, PhysX X, FixedArrays A,
                                                      const long long* __restrict__ fin,

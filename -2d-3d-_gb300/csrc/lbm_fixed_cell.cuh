@@ -669,32 +669,12 @@ struct FixedArrays {
 namespace fxa {
 
 // Both population sets pulled into one cell by index (PATH 4 below).
-template <int Q, bool TH, bool FACES>
-__device__ __forceinline__ void pull_set(const Geo& g, const PhysX& X, const long long* f, int c, int i, int j, int k,
-                                         q60* v) {
-    const PullRule r = pull_rule<TH>(g);
-#pragma unroll
-    for (int a = 0; a < Q; ++a) v[a] = ldq(f, pull_index<Q, FACES>(g, (int)g.ncell, r, a, i, j, k, c));
-    if (!TH) return;
-#pragma unroll
-    for (int a = 0; a < Q; ++a) {  // constant-temperature walls
-        const int ex = Lat<Q>::ex(a), ey = Lat<Q>::ey(a);
-        if (ex != 0 && r.cx && (ex > 0 ? i == 0 : i == g.nx - 1)) v[a] = Qb(ex > 0 ? X.bc_lo[0] : X.bc_hi[0]) - v[a];
-        if (FACES && ey != 0 && r.cy && (ey > 0 ? j == 0 : j == g.ny - 1))
-            v[a] = Qb(ey > 0 ? X.bc_lo[1] : X.bc_hi[1]) - v[a];
-    }
-}
 template <int D>
-__device__ __forceinline__ void pull_cell(const Geo& g, const PhysX& X, const long long* fin, const long long* gin,
-                                          long long c, int i, int j, int k, bool rows, q60* d, q60* e) {
+__device__ __forceinline__ void pull_cell(const Geo& g, const long long* fin, const long long* gin, long long c, int i,
+                                          int j, int k, bool rows, q60* d, q60* e) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
-    if (rows) {
-        pull_set<Q, false, false>(g, X, fin, (int)c, i, j, k, d);
-        pull_set<QT, true, false>(g, X, gin, (int)c, i, j, k, e);
-    } else {
-        pull_set<Q, false, true>(g, X, fin, (int)c, i, j, k, d);
-        pull_set<QT, true, true>(g, X, gin, (int)c, i, j, k, e);
-    }
+    pull_set_rows<Q, false, q60>(g, rows, i, j, k, (int)c, [&](int x) { return ldq(fin, x); }, d);
+    pull_set_rows<QT, true, q60>(g, rows, i, j, k, (int)c, [&](int x) { return ldq(gin, x); }, e);
 }
 
 // Flow collision of step n (lbm_exact.cu k_flow): FIRST reads the module arrays (f, rho,
@@ -731,7 +711,7 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const Fi
         q60 ts = Qb(0);
         if (PATH == 4) {
             q60 e[QT];
-            pull_cell<D>(g, X, fin, gin, c, i, j, k, rows, d, e);
+            pull_cell<D>(g, fin, gin, c, i, j, k, rows, d, e);
 #pragma unroll
             for (int a = 0; a < QT; ++a) ts = ts + e[a];
         } else if (PATH == 3) {
@@ -784,7 +764,7 @@ __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const
     const bool inner = PATH == 1 || (PATH == 0 && aa_inner(g, i, j, k));
     auto lf = [&](int a, long long cc) { return ldq(fin, a * n + cc); };
     if (PATH == 4) {
-        pull_cell<D>(g, X, fin, gin, c, i, j, k, rows, d, e);
+        pull_cell<D>(g, fin, gin, c, i, j, k, rows, d, e);
     } else if (PATH == 3) {
         auto lfi = [&](int a, I cc) { return ldq(fin, a * ni + cc); };
 #pragma unroll
