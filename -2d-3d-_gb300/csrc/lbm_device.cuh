@@ -274,11 +274,16 @@ __host__ __device__ __forceinline__ int pull_index(const Geo& g, int n, const Pu
 }
 
 #if defined(__CUDACC__)
-// Cell of a thread in lattice order with 32-bit indices (called by whole warps; a thread past the
+// Block of a thermal launch: last block first.  The flow kernel before it ended at the last cells
+// and the flow kernel after it begins at the first, so each finds the populations that the other
+// touched last in L2.
+__device__ __forceinline__ int last_first() { return (int)(gridDim.x - 1 - blockIdx.x); }
+
+// Cell of a thread of block `block` in lattice order with 32-bit indices (called by whole warps; a thread past the
 // lattice gets its last cell and false).  rows: no cell of the warp lies on a row of a y or z
 // face, so its pulls select for the x faces only (FACES of pull_index).
-__device__ __forceinline__ bool index_cell(const Geo& g, int& c, int& i, int& j, int& k, bool& rows) {
-    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), n = (int)g.ncell;
+__device__ __forceinline__ bool index_cell(const Geo& g, int block, int& c, int& i, int& j, int& k, bool& rows) {
+    const int t = block * (int)blockDim.x + (int)threadIdx.x, n = (int)g.ncell;
     c = min(t, n - 1);
     const int r = c / g.nx;
     i = c - r * g.nx;

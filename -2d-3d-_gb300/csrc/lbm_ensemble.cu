@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEn
                   int flip) {
     __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int2 tt = tiles[t];
+        const int2 tt = tiles[ntiles - 1 - t];  // last tile first (last_first)
         const EnsStage<S>& st = stage_member<S>(mem, tt.x, sh, [flip](const EnsMember<S>& gm, FastArgs<S>& A) {
             const int c = gm.cur ^ flip, n = c ^ 1;
             A.Bin0 = gm.B[c][0]; A.Bin1 = gm.B[c][1]; A.Bin2 = gm.B[c][2];

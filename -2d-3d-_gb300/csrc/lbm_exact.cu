@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, con
     bool rows = false;
     if (NARROW) {
         int ci;
-        const bool in = index_cell(g, ci, i, j, k, rows);
+        const bool in = index_cell(g, (int)blockIdx.x, ci, i, j, k, rows);
         if (!in) return;
         c = ci;
     } else if (!thread_cell(g, c, i, j, k)) {
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(128) k_thermal(Geo g, PhysC P, ExactArrays A, 
     bool rows = false;
     if (NARROW) {
         int ci;
-        const bool in = index_cell(g, ci, i, j, k, rows);
+        const bool in = index_cell(g, last_first(), ci, i, j, k, rows);
         if (!in) return;
         c = ci;
     } else if (!thread_cell(g, c, i, j, k)) {

@@ -99,14 +99,14 @@ __global__ void __launch_bounds__(128, 6) k_fast_flow_duo(Geo g, PhysF P, FastAr
                                                        const S* __restrict__ gin, S* __restrict__ fout) {
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? flow_tick(A.ticks, one) : 0ULL;
-    flow_duo_2k<D, S>(g, P, A, fin, gin, fout, duo_cells(g), tick);
+    flow_duo_2k<D, S>(g, P, A, fin, gin, fout, duo_cells(g, (int)blockIdx.x), tick);
 }
 template <int D, class S>
 __global__ void __launch_bounds__(128, 7) k_fast_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
                                                           const S* __restrict__ gin, S* __restrict__ gout) {
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
-    thermal_duo_2k<D, S>(g, P, A, fin, gin, gout, duo_cells(g), tick);
+    thermal_duo_2k<D, S>(g, P, A, fin, gin, gout, duo_cells(g, last_first()), tick);
 }
 
 // Paired form of the two kernels (lbm_fast_pairs.cuh): thread (x, y) of a block holds the

@@ -407,14 +407,14 @@ __global__ void __launch_bounds__(128, 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs
                                                      int raw) {
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? flow_tick(A.ticks, one) : 0ULL;
-    aa_flow_duo<D, S, ODD>(g, P, A, f, gs, raw != 0, duo_cells<true>(g), tick);
+    aa_flow_duo<D, S, ODD>(g, P, A, f, gs, raw != 0, duo_cells<true>(g, (int)blockIdx.x), tick);
 }
 template <int D, class S, bool ODD>
 __global__ void __launch_bounds__(128, 7) k_aa_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fs, S* gg,
                                                         int raw) {
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
-    aa_thermal_duo<D, S, ODD>(g, P, A, fs, gg, raw != 0, duo_cells<true>(g), tick);
+    aa_thermal_duo<D, S, ODD>(g, P, A, fs, gg, raw != 0, duo_cells<true>(g, last_first()), tick);
 }
 
 // ------------------------------------------------------------------------------------

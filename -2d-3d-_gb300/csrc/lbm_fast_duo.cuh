@@ -59,10 +59,11 @@ __device__ __forceinline__ Duo duo_at(const Geo& g, int c0, int end) {
     t.rows = __all_sync(0xFFFFFFFFu, off);
     return t;
 }
-// The cells of a single-lattice launch (ncell / 256 blocks of 128 threads, rounded up).
+// The cells of block `block` of a single-lattice launch (ncell / 256 blocks of 128 threads, rounded up).
 template <bool OWN = false>
-__device__ __forceinline__ Duo duo_cells(const Geo& g) {
-    return duo_at<OWN>(g, (int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * 2 + (int)(threadIdx.x & 31u), (int)g.ncell);
+__device__ __forceinline__ Duo duo_cells(const Geo& g, int block) {
+    return duo_at<OWN>(g, (block * (int)blockDim.x + (int)(threadIdx.x & ~31u)) * 2 + (int)(threadIdx.x & 31u),
+                       (int)g.ncell);
 }
 
 // A stored population as loaded, and its value.

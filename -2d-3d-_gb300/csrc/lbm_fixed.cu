@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128, kXFlowBlocks) k_xflow_ix(Geo g, PhysX X, 
                                                      const long long* __restrict__ gin, long long* __restrict__ fout) {
     int c, i, j, k;
     bool rows;
-    if (!index_cell(g, c, i, j, k, rows)) return;
+    if (!index_cell(g, (int)blockIdx.x, c, i, j, k, rows)) return;
     flow_cell<D, false, 4, int>(g, X, A, fin, gin, fout, c, i, j, k, rows);
 }
 
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128, kXThermalBlocks) k_xthermal_ix(Geo g, Phy
                                                         const long long* __restrict__ gin, long long* __restrict__ gout) {
     int c, i, j, k;
     bool rows;
-    if (!index_cell(g, c, i, j, k, rows)) return;
+    if (!index_cell(g, last_first(), c, i, j, k, rows)) return;
     thermal_cell<D, false, 4, int>(g, X, A, fin, gin, gout, c, i, j, k, rows);
 }
 
