@@ -14,6 +14,7 @@
 
 #include "lbm_ensemble.h"
 #include "lbm_fast_duo.cuh"
+#include "lbm_launch.cuh"
 
 namespace lbm {
 
@@ -93,6 +94,7 @@ template <int D, class S, bool WIDE>
 __global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEnsBlocks))
     k_ens_flow(const EnsMember<S>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int tile_cells, int flip) {
     __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];
+    wait_for_previous();
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int2 tt = tiles[t];
         const EnsStage<S>& st = stage_member<S>(mem, tt.x, sh, [flip](const EnsMember<S>& gm, FastArgs<S>& A) {
@@ -120,6 +122,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEn
                                   tick);
         }
     }
+    start_next();
 }
 
 template <int D, class S, bool WIDE>
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEn
     k_ens_thermal(const EnsMember<S>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int tile_cells,
                   int flip) {
     __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];
+    wait_for_previous();
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int2 tt = tiles[ntiles - 1 - t];  // last tile first (last_first)
         const EnsStage<S>& st = stage_member<S>(mem, tt.x, sh, [flip](const EnsMember<S>& gm, FastArgs<S>& A) {
@@ -156,6 +160,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEn
                                      duo_at(g, c + (int)(threadIdx.x & 31u), (int)ce), tick);
         }
     }
+    start_next();
 }
 
 template <class S>
@@ -221,13 +226,15 @@ cudaError_t ens_build(EnsPlan& plan, const std::vector<EnsMemberHost>& members, 
 template <int D, class S, bool WIDE>
 static void launch_list(const EnsPlan& plan, int li, int stage, int flip, cudaStream_t s) {
     // a duo block of 128 threads takes the cells that a one-cell block of 256 takes
-    const int block = WIDE ? plan.cfg.block : 128;
-    const int grid = min(plan.ntiles[li], plan.sms * plan.cfg.grid_mul);
+    const unsigned block = WIDE ? (unsigned)plan.cfg.block : 128u;
+    const unsigned grid = (unsigned)min(plan.ntiles[li], plan.sms * plan.cfg.grid_mul);
     const EnsMember<S>* mem = (const EnsMember<S>*)plan.d_members[li];
     if (stage == 0)
-        k_ens_flow<D, S, WIDE><<<grid, block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells, flip);
+        launch_after(k_ens_flow<D, S, WIDE>, grid, block, s, mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells,
+                     flip);
     else
-        k_ens_thermal<D, S, WIDE><<<grid, block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells, flip);
+        launch_after(k_ens_thermal<D, S, WIDE>, grid, block, s, mem, plan.d_tiles[li], plan.ntiles[li],
+                     plan.cfg.tile_cells, flip);
 }
 
 template <class S>

@@ -23,6 +23,7 @@
 #include "lbm_device.cuh"
 #include "lbm_exact_cell.cuh"
 #include "lbm_internal.h"
+#include "lbm_launch.cuh"
 
 namespace lbm {
 
@@ -320,7 +321,8 @@ __global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, con
     bool rows = false;
     if (NARROW) {
         int ci;
-        const bool in = index_cell(g, (int)blockIdx.x, ci, i, j, k, rows);
+            const bool in = index_cell(g, (int)blockIdx.x, ci, i, j, k, rows);
+        wait_for_previous();
         if (!in) return;
         c = ci;
     } else if (!thread_cell(g, c, i, j, k)) {
@@ -365,6 +367,7 @@ __global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, con
     }
 #pragma unroll
     for (int a = 0; a < Q; ++a) fout[a * n + c] = FP[a];
+    if (NARROW) start_next();
 }
 
 // Streaming + boundary + macro of the flow and thermal collision of step n
@@ -378,7 +381,8 @@ __global__ void __launch_bounds__(128) k_thermal(Geo g, PhysC P, ExactArrays A, 
     bool rows = false;
     if (NARROW) {
         int ci;
-        const bool in = index_cell(g, last_first(), ci, i, j, k, rows);
+            const bool in = index_cell(g, last_first(), ci, i, j, k, rows);
+        wait_for_previous();
         if (!in) return;
         c = ci;
     } else if (!thread_cell(g, c, i, j, k)) {
@@ -409,6 +413,7 @@ __global__ void __launch_bounds__(128) k_thermal(Geo g, PhysC P, ExactArrays A, 
     thermal_cell<D, !FIRST>(P, A, c, F, G, Tprev, GP);
 #pragma unroll
     for (int a = 0; a < QT; ++a) gout[a * n + c] = GP[a];
+    if (NARROW) start_next();
 }
 
 // Rebuild the reference's module arrays after fused step N: f_N, g_N (streamed, with
@@ -742,8 +747,8 @@ static void fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, bool 
         if (fl) k_flow<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
         if (th) k_thermal<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
     } else if (narrow) {
-        if (fl) k_flow<D, false, true><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
-        if (th) k_thermal<D, false, true><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
+        if (fl) launch_after(k_flow<D, false, true>, nb, bs, s, g, P, A, fprev, gprev, fnext);
+        if (th) launch_after(k_thermal<D, false, true>, nb, bs, s, g, P, A, fnext, gprev, gnext);
     } else {
         if (fl) k_flow<D, false, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
         if (th) k_thermal<D, false, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);

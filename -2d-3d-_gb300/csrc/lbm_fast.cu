@@ -15,6 +15,7 @@
 #include "lbm_fast_cells.cuh"
 #include "lbm_fast_duo.cuh"
 #include "lbm_fast_pairs.cuh"
+#include "lbm_launch.cuh"
 
 namespace lbm {
 
@@ -97,16 +98,22 @@ __global__ void __launch_bounds__(128, (OneCellBlocks<S, true>::value)) k_fast_t
 template <int D, class S>
 __global__ void __launch_bounds__(128, 6) k_fast_flow_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
                                                        const S* __restrict__ gin, S* __restrict__ fout) {
+    const Duo t = duo_cells(g, (int)blockIdx.x);
+    wait_for_previous();
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? flow_tick(A.ticks, one) : 0ULL;
-    flow_duo_2k<D, S>(g, P, A, fin, gin, fout, duo_cells(g, (int)blockIdx.x), tick);
+    flow_duo_2k<D, S>(g, P, A, fin, gin, fout, t, tick);
+    start_next();
 }
 template <int D, class S>
 __global__ void __launch_bounds__(128, 7) k_fast_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
                                                           const S* __restrict__ gin, S* __restrict__ gout) {
+    const Duo t = duo_cells(g, last_first());
+    wait_for_previous();
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
-    thermal_duo_2k<D, S>(g, P, A, fin, gin, gout, duo_cells(g, last_first()), tick);
+    thermal_duo_2k<D, S>(g, P, A, fin, gin, gout, t, tick);
+    start_next();
 }
 
 // Paired form of the two kernels (lbm_fast_pairs.cuh): thread (x, y) of a block holds the
@@ -210,8 +217,8 @@ template <int D, class S>
 static void duo_step(const Geo& g, const PhysF& pf, const FastArgs<S>& Af, const FastArgs<S>& At, const S* fin,
                      const S* gin, S* fout, S* gout, cudaStream_t s, bool fl, bool th) {
     const unsigned nb2 = (unsigned)((g.ncell + 255) / 256);
-    if (fl) k_fast_flow_duo<D, S><<<nb2, 128, 0, s>>>(g, pf, Af, fin, gin, fout);
-    if (th) k_fast_thermal_duo<D, S><<<nb2, 128, 0, s>>>(g, pf, At, fout, gin, gout);
+    if (fl) launch_after(k_fast_flow_duo<D, S>, nb2, 128, s, g, pf, Af, fin, gin, fout);
+    if (th) launch_after(k_fast_thermal_duo<D, S>, nb2, 128, s, g, pf, At, fout, gin, gout);
 }
 
 template <int D, class S>

@@ -14,6 +14,7 @@
 #include "lbm_fast_pairs.cuh"
 #include "lbm_fast_aa.cuh"
 #include "lbm_fast_aa_duo.cuh"
+#include "lbm_launch.cuh"
 
 namespace lbm {
 
@@ -405,16 +406,22 @@ __global__ void __launch_bounds__(128) k_aa_thermal_p(Geo g, PhysF P, FastArgs<S
 template <int D, class S, bool ODD>
 __global__ void __launch_bounds__(128, 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs<S> A, S* f, const S* __restrict__ gs,
                                                      int raw) {
+    const Duo t = duo_cells<true>(g, (int)blockIdx.x);
+    wait_for_previous();
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? flow_tick(A.ticks, one) : 0ULL;
-    aa_flow_duo<D, S, ODD>(g, P, A, f, gs, raw != 0, duo_cells<true>(g, (int)blockIdx.x), tick);
+    aa_flow_duo<D, S, ODD>(g, P, A, f, gs, raw != 0, t, tick);
+    start_next();
 }
 template <int D, class S, bool ODD>
 __global__ void __launch_bounds__(128, 7) k_aa_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fs, S* gg,
                                                         int raw) {
+    const Duo t = duo_cells<true>(g, last_first());
+    wait_for_previous();
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
-    aa_thermal_duo<D, S, ODD>(g, P, A, fs, gg, raw != 0, duo_cells<true>(g, last_first()), tick);
+    aa_thermal_duo<D, S, ODD>(g, P, A, fs, gg, raw != 0, t, tick);
+    start_next();
 }
 
 // ------------------------------------------------------------------------------------
@@ -463,13 +470,13 @@ static bool aa_step_launch(FastState& F, const Geo& g, const PhysF& pf, cudaStre
         (long long)F.q * g.ncell < (1LL << 31) - 64 && (part == 1 ? st.fpar != st.gpar : st.fpar == st.gpar)) {
         const unsigned nb2 = (unsigned)((g.ncell + 255) / 256);
         if (part != 1) {
-            if (st.fpar) k_aa_flow_duo<D, S, true><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
-            else k_aa_flow_duo<D, S, false><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
+            if (st.fpar) launch_after(k_aa_flow_duo<D, S, true>, nb2, 128, s, g, pf, A, f, gg, raw);
+            else launch_after(k_aa_flow_duo<D, S, false>, nb2, 128, s, g, pf, A, f, gg, raw);
             st.fpar ^= 1;
         }
         if (part != 0) {
-            if (st.gpar) k_aa_thermal_duo<D, S, true><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
-            else k_aa_thermal_duo<D, S, false><<<nb2, 128, 0, s>>>(g, pf, A, f, gg, raw);
+            if (st.gpar) launch_after(k_aa_thermal_duo<D, S, true>, nb2, 128, s, g, pf, A, f, gg, raw);
+            else launch_after(k_aa_thermal_duo<D, S, false>, nb2, 128, s, g, pf, A, f, gg, raw);
             if (st.gpar) st.graw = true;
             st.gpar ^= 1;
         }

@@ -8,6 +8,7 @@
 
 #include "lbm_fixed.h"
 #include "lbm_fixed_cell.cuh"
+#include "lbm_launch.cuh"
 
 namespace lbm {
 
@@ -96,8 +97,11 @@ __global__ void __launch_bounds__(128, kXFlowBlocks) k_xflow_ix(Geo g, PhysX X, 
                                                      const long long* __restrict__ gin, long long* __restrict__ fout) {
     int c, i, j, k;
     bool rows;
-    if (!index_cell(g, (int)blockIdx.x, c, i, j, k, rows)) return;
+    const bool in = index_cell(g, (int)blockIdx.x, c, i, j, k, rows);
+    wait_for_previous();
+    if (!in) return;
     flow_cell<D, false, 4, int>(g, X, A, fin, gin, fout, c, i, j, k, rows);
+    start_next();
 }
 
 template <int D>
@@ -106,8 +110,11 @@ __global__ void __launch_bounds__(128, kXThermalBlocks) k_xthermal_ix(Geo g, Phy
                                                         const long long* __restrict__ gin, long long* __restrict__ gout) {
     int c, i, j, k;
     bool rows;
-    if (!index_cell(g, last_first(), c, i, j, k, rows)) return;
+    const bool in = index_cell(g, last_first(), c, i, j, k, rows);
+    wait_for_previous();
+    if (!in) return;
     thermal_cell<D, false, 4, int>(g, X, A, fin, gin, gout, c, i, j, k, rows);
+    start_next();
 }
 
 template <int D>
@@ -363,8 +370,8 @@ static void steady_step(const Geo& g, const PhysX& X, const FixedArrays& A, cons
     constexpr int Q = D == 3 ? 19 : 9;
     if (!wide && (long long)Q * g.ncell < (1LL << 31)) {
         const unsigned nb = (unsigned)((g.ncell + 127) / 128);
-        if (fl) k_xflow_ix<D><<<nb, 128, 0, s>>>(g, X, A, fprev, gprev, fnext);
-        if (th) k_xthermal_ix<D><<<nb, 128, 0, s>>>(g, X, A, fnext, gprev, gnext);
+        if (fl) launch_after(k_xflow_ix<D>, nb, 128, s, g, X, A, fprev, gprev, fnext);
+        if (th) launch_after(k_xthermal_ix<D>, nb, 128, s, g, X, A, fnext, gprev, gnext);
         return;
     }
     // 64-bit indices: interior kernel and face kernel for each half
