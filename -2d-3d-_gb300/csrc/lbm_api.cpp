@@ -628,16 +628,18 @@ static FixedArrays fixed_arrays(const lbm_handle* h) {
 // Rebuild the module arrays from the fused buffers (no-op when already there).  The fixed
 // arithmetic keeps its q60 buffers as the state: the module arrays are a rounded FP64 copy,
 // so how often a caller reads diagnostics does not change the run.
-static int materialize(lbm_handle* h) {
+// pops false: the caller reads scalar fields only, so the forms that keep their state elsewhere
+// leave the module populations alone.
+static int materialize(lbm_handle* h, bool pops) {
     if (h->p.precision != LBM_FP64) {
-        fast_materialize(h->F, h->geo, h->phys, h->dim, h->stream);
+        fast_materialize(h->F, h->geo, h->phys, h->dim, pops, h->stream);
         CK_LAUNCH(h, "materialize");
         return LBM_OK;
     }
     if (!h->fused_valid) return LBM_OK;
     if (h->fixed) {
         fixed_materialize(h->xgeo, h->px, fixed_arrays(h), h->dim, (const long long*)h->fbuf[h->cur],
-                          (const long long*)h->gbuf[h->cur], h->stream);
+                          (const long long*)h->gbuf[h->cur], pops, h->stream);
         CK_LAUNCH(h, "materialize");
         return LBM_OK;
     }
@@ -660,7 +662,7 @@ static int materialize(lbm_handle* h) {
 // the stage kernels read, and start the next fused step from the module arrays.
 static int release_fixed(lbm_handle* h) {
     if (!h->fixed || !h->fused_valid) return LBM_OK;
-    int st = materialize(h);
+    int st = materialize(h, true);
     if (st != LBM_OK) return st;
     fixed_post_to_double(h->px, (long long*)h->fbuf[h->cur], (long long*)h->gbuf[h->cur], h->geo.ncell, h->q, h->qt,
                          h->stream);
@@ -682,7 +684,7 @@ static int stage(lbm_handle* h, int which) {
     if (h->p.pattern == LBM_PATTERN_AA)
         return fail(h, LBM_ERR_STATE, "stage entry points need the two-buffer pattern (separate f and f_post)");
     CK(h, cudaSetDevice(h->device));
-    int st = h->fixed ? release_fixed(h) : materialize(h);
+    int st = h->fixed ? release_fixed(h) : materialize(h, true);
     if (st != LBM_OK) return st;
     if (which == STAGE_COLLISION) h->itc += 1;
     exact_stage(which, h->geo, h->phys, h->A, h->dim, h->stream);
@@ -910,7 +912,7 @@ static int diag_prologue(lbm_handle* h) {
     CK(h, cudaSetDevice(h->device));
     int st = take_device_error(h);
     if (st != LBM_OK) return st;
-    return materialize(h);
+    return materialize(h, false);
 }
 
 extern "C" int lbm_check(lbm_handle* h, double* errU, double* errT) {
@@ -1430,7 +1432,9 @@ static int state_io(lbm_handle* h, int field, double* dst, const double* src, si
     // fixed arithmetic: a load makes the module arrays the state; the post-collision arrays
     // exist only in FP64 form
     const bool post = field == LBM_FIELD_F_POST || field == LBM_FIELD_G_POST;
-    int st = (h->fixed && (src || post)) ? release_fixed(h) : materialize(h);
+    // a load continues from the module arrays, so all of them are brought up to date first
+    const bool pops = src || field == LBM_FIELD_F || field == LBM_FIELD_G;
+    int st = (h->fixed && (src || post)) ? release_fixed(h) : materialize(h, pops);
     if (st != LBM_OK) return st;
     const long long n = h->geo.ncell;
     const bool pop = field == LBM_FIELD_F || field == LBM_FIELD_G || field == LBM_FIELD_F_POST || field == LBM_FIELD_G_POST;
@@ -1671,7 +1675,7 @@ extern "C" int lbm_backupData(lbm_handle* h, const char* path, int flags) {
     if (flags != LBM_BACKUP_REFERENCE && flags != LBM_BACKUP_CONTINUE) return fail(h, LBM_ERR_PARAM, "unknown flags");
     if (!h->initialised) return fail(h, LBM_ERR_STATE, "lbm_initial has not been called");
     CK(h, cudaSetDevice(h->device));
-    int st = materialize(h);
+    int st = materialize(h, true);
     if (st != LBM_OK) return st;
     const size_t n = (size_t)h->geo.ncell;
     const bool fp64 = h->p.precision == LBM_FP64;

@@ -296,11 +296,11 @@ __device__ __forceinline__ bool index_cell(const Geo& g, int block, int& c, int&
 
 // The Q values of one set pulled into a cell by index, LOAD(index) in the arithmetic type T: what
 // pull_flow and pull_thermal return.
-template <int Q, bool TH, bool FACES, class T, class LOAD>
+template <int Q, bool TH, bool FACES, bool SWAP, class T, class LOAD>
 __device__ __forceinline__ void pull_set_index(const Geo& g, int i, int j, int k, int c, LOAD load, T* v) {
     const PullRule r = pull_rule<TH>(g);
 #pragma unroll
-    for (int a = 0; a < Q; ++a) v[a] = load(pull_index<Q, FACES>(g, (int)g.ncell, r, a, i, j, k, c));
+    for (int a = 0; a < Q; ++a) v[a] = load(pull_index<Q, FACES, SWAP>(g, (int)g.ncell, r, a, i, j, k, c));
     if (!TH) return;
 #pragma unroll
     for (int a = 0; a < Q; ++a) {  // constant-temperature walls
@@ -310,10 +310,11 @@ __device__ __forceinline__ void pull_set_index(const Geo& g, int i, int j, int k
             v[a] = -v[a] + (T)(ey > 0 ? g.bcT_lo[1] : g.bcT_hi[1]);
     }
 }
-template <int Q, bool TH, class T, class LOAD>
+// rows: as index_cell gives it.  SWAP: the swapped layout of the in-place pattern.
+template <int Q, bool TH, class T, bool SWAP = false, class LOAD>
 __device__ __forceinline__ void pull_set_rows(const Geo& g, bool rows, int i, int j, int k, int c, LOAD load, T* v) {
-    if (rows) pull_set_index<Q, TH, false, T>(g, i, j, k, c, load, v);
-    else pull_set_index<Q, TH, true, T>(g, i, j, k, c, load, v);
+    if (rows) pull_set_index<Q, TH, false, SWAP, T>(g, i, j, k, c, load, v);
+    else pull_set_index<Q, TH, true, SWAP, T>(g, i, j, k, c, load, v);
 }
 
 // ------------------------------------------------------------------------------------

@@ -418,21 +418,30 @@ __global__ void __launch_bounds__(128) k_thermal(Geo g, PhysC P, ExactArrays A, 
 
 // Rebuild the reference's module arrays after fused step N: f_N, g_N (streamed, with
 // boundaries), rho_N, u_N (with the lag), T_N.
-template <int D>
-__global__ void k_materialize(Geo g, PhysC P, ExactArrays A, const double* __restrict__ fin,
-                              const double* __restrict__ gin) {
-    long long c;
-    int i, j, k;
-    if (!thread_cell(g, c, i, j, k)) return;
+template <int D, bool NARROW>
+__global__ void __launch_bounds__(128) k_materialize(Geo g, PhysC P, ExactArrays A, const double* __restrict__ fin,
+                                                  const double* __restrict__ gin) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
+    long long c;
+    int i, j, k;
     double F[Q], G[QT];
-    auto lf = [&](int a, long long cc) { return fin[a * n + cc]; };
-    auto lg = [&](int a, long long cc) { return gin[a * n + cc]; };
+    if (NARROW) {
+        int ci;
+        bool rows;
+        if (!index_cell(g, (int)blockIdx.x, ci, i, j, k, rows)) return;
+        c = ci;
+        pull_set_rows<Q, false, double>(g, rows, i, j, k, ci, [&](int x) { return fin[x]; }, F);
+        pull_set_rows<QT, true, double>(g, rows, i, j, k, ci, [&](int x) { return gin[x]; }, G);
+    } else {
+        if (!thread_cell(g, c, i, j, k)) return;
+        auto lf = [&](int a, long long cc) { return fin[a * n + cc]; };
+        auto lg = [&](int a, long long cc) { return gin[a * n + cc]; };
 #pragma unroll
-    for (int a = 0; a < Q; ++a) F[a] = pull_flow<Q, double>(g, a, i, j, k, c, lf);
+        for (int a = 0; a < Q; ++a) F[a] = pull_flow<Q, double>(g, a, i, j, k, c, lf);
 #pragma unroll
-    for (int a = 0; a < QT; ++a) G[a] = pull_thermal<QT, double>(g, a, i, j, k, c, lg);
+        for (int a = 0; a < QT; ++a) G[a] = pull_thermal<QT, double>(g, a, i, j, k, c, lg);
+    }
     double rho, u, v, w;
     if (D == 2) {
         macro_2d(F, A.Fx[c], A.Fy[c], rho, u, v);
@@ -818,8 +827,11 @@ void exact_reconstruct(const Geo& g, const PhysC& P, const ExactArrays& A, int d
 void exact_materialize(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, const double* fcur,
                        const double* gcur, cudaStream_t s) {
     const unsigned nb = nblocks(g.ncell, 128);
-    if (dim == 2) k_materialize<2><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
-    else k_materialize<3><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
+    const bool narrow = (dim == 3 ? 19LL : 9LL) * g.ncell < (1LL << 31);
+    if (dim == 2 && narrow) k_materialize<2, true><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
+    else if (dim == 2) k_materialize<2, false><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
+    else if (narrow) k_materialize<3, true><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
+    else k_materialize<3, false><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
 }
 
 }  // namespace lbm

@@ -237,37 +237,39 @@ static void rows_step(const Geo& g, const PhysF& pf, const FastArgs<S>& Af, cons
     }
 }
 
-// Module arrays of step N from F[cur] = f_post_N, G[cur] = g_post_N, L[cur] (lag_in).
-template <int D, class S>
-__global__ void k_fast_materialize(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
-                                   const S* __restrict__ gin) {
-    long long c;
-    int i, j, k;
-    if (!fcell(g, c, i, j, k)) return;
+// Module arrays of step N from F[cur] = f_post_N, G[cur] = g_post_N, L[cur] (lag_in).  POPS: the
+// populations as well as the scalar fields.  NARROW: pulls by 32-bit index (pull_set_rows).
+template <int D, class S, bool POPS, bool NARROW>
+__global__ void __launch_bounds__(128) k_fast_materialize(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
+                                                       const S* __restrict__ gin) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    float d[Q];
-    auto lf = [&](int a, long long cc) { return ldS(fin, a * n + cc); };
-    auto lg = [&](int a, long long cc) { return ldS(gin, a * n + cc); };
+    long long c;
+    int i, j, k;
+    float d[Q], e[QT];
+    if (NARROW) {
+        int ci;
+        bool rows;
+        if (!index_cell(g, (int)blockIdx.x, ci, i, j, k, rows)) return;
+        c = ci;
+        pull_set_rows<Q, false, float>(g, rows, i, j, k, ci, [&](int x) { return ldS(fin, x); }, d);
+        pull_set_rows<QT, true, float>(g, rows, i, j, k, ci, [&](int x) { return ldS(gin, x); }, e);
+    } else {
+        if (!fcell(g, c, i, j, k)) return;
+        auto lf = [&](int a, long long cc) { return ldS(fin, a * n + cc); };
+        auto lg = [&](int a, long long cc) { return ldS(gin, a * n + cc); };
 #pragma unroll
-    for (int a = 0; a < Q; ++a) {
-        d[a] = pull_flow<Q, float>(g, a, i, j, k, c, lf);
-        A.fref[a * n + c] = toS<S>(d[a]);
-    }
-    float ts = 0.0f;
+        for (int a = 0; a < Q; ++a) d[a] = pull_flow<Q, float>(g, a, i, j, k, c, lf);
 #pragma unroll
-    for (int a = 0; a < QT; ++a) {
-        const float e = pull_thermal<QT, float>(g, a, i, j, k, c, lg);
-        A.gref[a * n + c] = toS<S>(e);
-        ts += e + wT<QT>(P, a) * P.Tref;
+        for (int a = 0; a < QT; ++a) e[a] = pull_thermal<QT, float>(g, a, i, j, k, c, lg);
     }
-    float dr, rho, u, v, w, Fy;
-    fmacro<D>(d, A.lag_in[c], P, dr, rho, u, v, w, Fy);
-    A.rho[c] = rho;
-    A.u[c] = u;
-    A.v[c] = v;
-    if (D == 3) A.w[c] = w;
-    A.T[c] = ts;
+    if (POPS) {
+#pragma unroll
+        for (int a = 0; a < Q; ++a) A.fref[a * n + c] = toS<S>(d[a]);
+#pragma unroll
+        for (int a = 0; a < QT; ++a) A.gref[a * n + c] = toS<S>(e[a]);
+    }
+    module_scalars<D, S>(P, A, d, e, c);
 }
 
 // export / import (FP64 Fortran layout)
@@ -497,7 +499,18 @@ void fast_enter(FastState& F, const Geo& g0, const PhysC& P, int dim, cudaStream
     F.ahead = true;
 }
 
-void fast_materialize(FastState& F, const Geo& g0, const PhysC& P, int dim, cudaStream_t s) {
+template <int D, class S>
+static void materialize(const FastState& F, const Geo& g, const PhysF& pf, bool pops, cudaStream_t s) {
+    const S* fin = (const S*)F.fbuf[F.cur];
+    const S* gin = (const S*)F.gbuf[F.cur];
+    const FastArgs<S> A = args_for<S>(F, F.cur, F.cur, F.cur, F.cur);
+    const unsigned n = nb(g.ncell, 128);
+    if ((long long)F.q * g.ncell >= (1LL << 31)) k_fast_materialize<D, S, true, false><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
+    else if (pops) k_fast_materialize<D, S, true, true><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
+    else k_fast_materialize<D, S, false, true><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
+}
+
+void fast_materialize(FastState& F, const Geo& g0, const PhysC& P, int dim, bool pops, cudaStream_t s) {
     if (!F.fused_valid) return;
     const PhysF pf = to_physf(P);
     const Geo g = dev_geo(g0, P);
@@ -506,11 +519,8 @@ void fast_materialize(FastState& F, const Geo& g0, const PhysC& P, int dim, cuda
         return;
     }
     DISPATCH_S(F, {
-        const S* fin = (const S*)F.fbuf[F.cur];
-        const S* gin = (const S*)F.gbuf[F.cur];
-        FastArgs<S> A = args_for<S>(F, F.cur, F.cur, F.cur, F.cur);
-        if (dim == 2) k_fast_materialize<2, S><<<nb(g.ncell, 128), 128, 0, s>>>(g, pf, A, fin, gin);
-        else k_fast_materialize<3, S><<<nb(g.ncell, 128), 128, 0, s>>>(g, pf, A, fin, gin);
+        if (dim == 2) materialize<2, S>(F, g, pf, pops, s);
+        else materialize<3, S>(F, g, pf, pops, s);
     });
 }
 

@@ -87,8 +87,9 @@ void fast_tick(FastState& F, cudaStream_t s);
 bool fast_step_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, bool first, cudaStream_t s, int part);
 void fast_materialize_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, cudaStream_t s);
 // Rebuild the module arrays (f, g, rho, u, v, w, T) of the current step; leaves the fused
-// buffers valid.  In-place pattern: the module scalars only (the arrays are the populations).
-void fast_materialize(FastState& F, const Geo& g, const PhysC& P, int dim, cudaStream_t s);
+// buffers valid.  pops false, and in-place pattern (whose arrays are the populations): the module
+// scalars only.
+void fast_materialize(FastState& F, const Geo& g, const PhysC& P, int dim, bool pops, cudaStream_t s);
 inline bool fast_fused_valid(const FastState& F) { return F.fused_valid; }
 inline bool fast_at_origin(const FastState& F) { return F.cur == 0; }
 DiagFields<float> fast_diag_fields(const FastState& F);

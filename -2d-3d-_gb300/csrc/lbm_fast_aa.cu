@@ -146,17 +146,28 @@ __global__ void __launch_bounds__(128, (OneCellBlocks<S, true>::value)) k_aa_the
     aa_thermal_cell<D, S, ODD, FIRST>(g, P, A, fs, gg, wg, fpar, graw, c, i, j, k);
 }
 
-// Module scalars (rho, u, v, w, T) of the current step, populations left in place.
-template <int D, class S>
-__global__ void k_aa_materialize_f(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fs,
-                                   const S* __restrict__ gs, int fpar, int gpar, int graw) {
+// Module scalars (rho, u, v, w, T) of the current step, populations left in place.  NARROW: reads by
+// 32-bit index (pull_set_rows; own slots in the streamed layout).
+template <int D, class S, bool NARROW>
+__global__ void __launch_bounds__(128) k_aa_materialize_f(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fs,
+                                                       const S* __restrict__ gs, int fpar, int gpar, int graw) {
     long long c;
-    int i, j, k;
-    if (!fcell(g, c, i, j, k)) return;
+    int i, j, k, ci = 0;
+    bool rows = false;
+    if (NARROW) {
+        if (!index_cell(g, (int)blockIdx.x, ci, i, j, k, rows)) return;
+        c = ci;
+    } else if (!fcell(g, c, i, j, k)) {
+        return;
+    }
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    float d[Q];
-    if (fpar) {
+    float d[Q], e[QT];
+    auto lfi = [&](int x) { return ldS(fs, x); };
+    auto lgi = [&](int x) { return ldS(gs, x); };
+    if (fpar && NARROW) {
+        pull_set_rows<Q, false, float, true>(g, rows, i, j, k, ci, lfi, d);
+    } else if (fpar) {
         auto lf = [&](int b, long long cc) { return ldS(fs, Lat<Q>::opp(b) * n + cc); };
 #pragma unroll
         for (int a = 0; a < Q; ++a) d[a] = pull_flow<Q, float>(g, a, i, j, k, c, lf);
@@ -164,24 +175,18 @@ __global__ void k_aa_materialize_f(Geo g, PhysF P, FastArgs<S> A, const S* __res
 #pragma unroll
         for (int a = 0; a < Q; ++a) d[a] = ldS(fs, a * n + c);
     }
-    float ts = 0.0f;
-    if (gpar) {
+    if (gpar && NARROW) {
+        pull_set_rows<QT, true, float, true>(g, rows, i, j, k, ci, lgi, e);
+    } else if (gpar) {
         auto lg = [&](int b, long long cc) { return ldS(gs, Lat<QT>::opp(b) * n + cc); };
 #pragma unroll
-        for (int a = 0; a < QT; ++a) ts += pull_thermal<QT, float>(g, a, i, j, k, c, lg) + wT<QT>(P, a) * P.Tref;
+        for (int a = 0; a < QT; ++a) e[a] = pull_thermal<QT, float>(g, a, i, j, k, c, lg);
     } else {
         auto lg = [&](int b, long long cc) { return ldS(gs, b * n + cc); };
 #pragma unroll
-        for (int a = 0; a < QT; ++a)
-            ts += aa_local_thermal<QT, float>(g, a, i, j, k, c, graw != 0, lg) + wT<QT>(P, a) * P.Tref;
+        for (int a = 0; a < QT; ++a) e[a] = aa_local_thermal<QT, float>(g, a, i, j, k, c, graw != 0, lg);
     }
-    float dr, rho, u, v, w, Fy;
-    fmacro<D>(d, A.lag_in[c], P, dr, rho, u, v, w, Fy);
-    A.rho[c] = rho;
-    A.u[c] = u;
-    A.v[c] = v;
-    if (D == 3) A.w[c] = w;
-    A.T[c] = ts;
+    module_scalars<D, S>(P, A, d, e, c);
 }
 
 // ------------------------------------------------------------------------------------
@@ -534,20 +539,26 @@ bool fast_step_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, bool fir
                     : aa_step_first<3, float>(F, g, pf, first, s, part);
 }
 
-void fast_materialize_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, cudaStream_t s) {
+template <int D, class S>
+static void aa_materialize(const FastState& F, const Geo& g, const PhysF& pf, cudaStream_t s) {
     const unsigned nb = (unsigned)((g.ncell + 127) / 128);
     const AAState& st = F.AA;
     const int raw = st.graw ? 1 : 0;
+    const FastArgs<S> A = aa_args<S>(F);
+    const S *f = (const S*)F.fbuf[0], *gg = (const S*)F.gbuf[0];
+    if ((long long)F.q * g.ncell < (1LL << 31))
+        k_aa_materialize_f<D, S, true><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
+    else
+        k_aa_materialize_f<D, S, false><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
+}
+
+void fast_materialize_aa(FastState& F, const Geo& g, const PhysF& pf, int dim, cudaStream_t s) {
     if (F.precision == LBM_FP16) {
-        const FastArgs<__half> A = aa_args<__half>(F);
-        const __half *f = (const __half*)F.fbuf[0], *gg = (const __half*)F.gbuf[0];
-        if (dim == 2) k_aa_materialize_f<2, __half><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
-        else k_aa_materialize_f<3, __half><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
+        if (dim == 2) aa_materialize<2, __half>(F, g, pf, s);
+        else aa_materialize<3, __half>(F, g, pf, s);
     } else {
-        const FastArgs<float> A = aa_args<float>(F);
-        const float *f = (const float*)F.fbuf[0], *gg = (const float*)F.gbuf[0];
-        if (dim == 2) k_aa_materialize_f<2, float><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
-        else k_aa_materialize_f<3, float><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
+        if (dim == 2) aa_materialize<2, float>(F, g, pf, s);
+        else aa_materialize<3, float>(F, g, pf, s);
     }
 }
 

@@ -81,6 +81,22 @@ __device__ __forceinline__ void flow_cell_2k(const Geo& g, const PhysF& P, const
     for (int a = 0; a < Q; ++a) fout[a * ni + ci] = hs[a];
 }
 
+// Module scalars of a cell (rho, u, v, w, T) from its streamed deviations and the lag.
+template <int D, class S>
+__device__ __forceinline__ void module_scalars(const PhysF& P, const FastArgs<S>& A, const float* d, const float* e,
+                                               long long c) {
+    constexpr int QT = D == 2 ? 5 : 7;
+    float ts = 0.0f, dr, rho, u, v, w, Fy;
+#pragma unroll
+    for (int a = 0; a < QT; ++a) ts += e[a] + wT<QT>(P, a) * P.Tref;
+    fmacro<D>(d, A.lag_in[c], P, dr, rho, u, v, w, Fy);
+    A.rho[c] = rho;
+    A.u[c] = u;
+    A.v[c] = v;
+    if (D == 3) A.w[c] = w;
+    A.T[c] = ts;
+}
+
 // Thermal collision of one cell from its streamed flow and thermal deviations (e, in place), with
 // B_prev and the 3D T lag (T_{n-1}).  FIRST: T is the module's, which a state load may have set
 // apart from the populations.

@@ -126,6 +126,17 @@ __global__ void k_xmaterialize(Geo g, PhysX X, FixedArrays A, const long long* _
     materialize_cell<D>(g, X, A, fin, gin, c, i, j, k);
 }
 
+// The module arrays by index, POPS: the populations as well.  GB300, calNuRe at 256^3 (this kernel
+// and the reduction): 3.9 ms with branching pulls and the populations, 1.2 ms without both.
+template <int D, bool POPS>
+__global__ void __launch_bounds__(128) k_xmaterialize_ix(Geo g, PhysX X, FixedArrays A, const long long* __restrict__ fin,
+                                                      const long long* __restrict__ gin) {
+    int c, i, j, k;
+    bool rows;
+    if (!index_cell(g, (int)blockIdx.x, c, i, j, k, rows)) return;
+    materialize_cell<D, true, POPS>(g, X, A, fin, gin, c, i, j, k, rows);
+}
+
 // q60 deviations of a fused buffer -> the FP64 populations they stand for, in place.
 __global__ void k_xpost_to_double(long long* buf, long long n, int q, PhysX X, int thermal) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -412,11 +423,19 @@ void fixed_fused_step(const Geo& g, const PhysX& X, const FixedArrays& A, int di
     }
 }
 
-void fixed_materialize(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, const long long* fcur,
-                       const long long* gcur, cudaStream_t s) {
+template <int D>
+static void materialize(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fcur, const long long* gcur,
+                        bool pops, cudaStream_t s) {
     const unsigned nb = xblocks(g.ncell, 128);
-    if (dim == 2) k_xmaterialize<2><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
-    else k_xmaterialize<3><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
+    if ((D == 3 ? 19LL : 9LL) * g.ncell >= (1LL << 31)) k_xmaterialize<D><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
+    else if (pops) k_xmaterialize_ix<D, true><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
+    else k_xmaterialize_ix<D, false><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
+}
+
+void fixed_materialize(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, const long long* fcur,
+                       const long long* gcur, bool pops, cudaStream_t s) {
+    if (dim == 2) materialize<2>(g, X, A, fcur, gcur, pops, s);
+    else materialize<3>(g, X, A, fcur, gcur, pops, s);
 }
 
 void fixed_post_to_double(const PhysX& X, long long* fbuf, long long* gbuf, long long n, int q, int qt,

@@ -834,26 +834,33 @@ __device__ __forceinline__ void thermal_cell(const Geo& g, const PhysX& X, const
 // f_N, g_N (streamed, with boundaries), rho_N and u_N of the macro step with the lag, T_N,
 // B_prev, and the 3D T lag or 2D force.  A cell whose density or velocity left the range of
 // a physical state gets a NaN density, which the diagnostics report as diverged.
-template <int D>
+// INDEX: pulls by index (PATH 4 of flow_cell).  POPS: f and g as well; the diagnostics and the scalar
+// fields need none.
+template <int D, bool INDEX = false, bool POPS = true>
 __device__ __forceinline__ void materialize_cell(const Geo& g, const PhysX& X, const FixedArrays& A,
                                                  const long long* fin, const long long* gin, long long c, int i, int j,
-                                                 int k) {
+                                                 int k, bool rows = true) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
-    q60 d[Q], rho, P[3], U[3], F;
-    auto lf = [&](int a, long long cc) { return ldq(fin, a * n + cc); };
-    auto lg = [&](int a, long long cc) { return ldq(gin, a * n + cc); };
+    q60 d[Q], e[QT], rho, P[3], U[3], F;
+    if (INDEX) {
+        pull_cell<D>(g, fin, gin, c, i, j, k, rows, d, e);
+    } else {
+        auto lf = [&](int a, long long cc) { return ldq(fin, a * n + cc); };
+        auto lg = [&](int a, long long cc) { return ldq(gin, a * n + cc); };
+#pragma unroll
+        for (int a = 0; a < Q; ++a) d[a] = pull_flow<Q, q60>(g, a, i, j, k, c, lf);
+#pragma unroll
+        for (int a = 0; a < QT; ++a) e[a] = pull_thermal<QT, q60>(g, a, i, j, k, c, lg);
+    }
     q60 ts = Qb(0);
 #pragma unroll
-    for (int a = 0; a < Q; ++a) {
-        d[a] = pull_flow<Q, q60>(g, a, i, j, k, c, lf);
-        A.f[a * n + c] = to_double(d[a] + Qb(X.w[a]));
-    }
+    for (int a = 0; a < QT; ++a) ts = ts + e[a];
+    if (POPS) {
 #pragma unroll
-    for (int a = 0; a < QT; ++a) {
-        const q60 e = pull_thermal<QT, q60>(g, a, i, j, k, c, lg);
-        ts = ts + e;
-        A.g[a * n + c] = to_double(e + Qb(X.wt[a]));
+        for (int a = 0; a < Q; ++a) A.f[a * n + c] = to_double(d[a] + Qb(X.w[a]));
+#pragma unroll
+        for (int a = 0; a < QT; ++a) A.g[a * n + c] = to_double(e[a] + Qb(X.wt[a]));
     }
     const q60 lag = Qb(A.xlag[c]);
     macro<D>(d, lag, X, rho, P, U, F);
