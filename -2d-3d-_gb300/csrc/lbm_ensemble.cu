@@ -229,6 +229,13 @@ static void launch_list(const EnsPlan& plan, int li, int stage, int flip, cudaSt
     const unsigned block = WIDE ? (unsigned)plan.cfg.block : 128u;
     const unsigned grid = (unsigned)min(plan.ntiles[li], plan.sms * plan.cfg.grid_mul);
     const EnsMember<S>* mem = (const EnsMember<S>*)plan.d_members[li];
+    if (WIDE) {  // its cell bodies take read-only loads: no start before the last kernel's end
+        if (stage == 0)
+            k_ens_flow<D, S, WIDE><<<grid, block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells, flip);
+        else
+            k_ens_thermal<D, S, WIDE><<<grid, block, 0, s>>>(mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells, flip);
+        return;
+    }
     if (stage == 0)
         launch_after(k_ens_flow<D, S, WIDE>, grid, block, s, mem, plan.d_tiles[li], plan.ntiles[li], plan.cfg.tile_cells,
                      flip);

@@ -314,8 +314,8 @@ __device__ __forceinline__ void thermal_cell(const PhysC& P, const ExactArrays& 
 // NARROW: every index fits in 32 bits, and the boundary rules are selects on the load index
 // (pull_set_index); otherwise the branching pulls with 64-bit indices.
 template <int D, bool FIRST, bool NARROW>
-__global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, const double* __restrict__ fin,
-                                              const double* __restrict__ gin, double* __restrict__ fout) {
+__global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, const double* fin,
+                                              const double* gin, double* fout) {
     long long c;
     int i, j, k;
     bool rows = false;
@@ -374,8 +374,8 @@ __global__ void __launch_bounds__(128) k_flow(Geo g, PhysC P, ExactArrays A, con
 // (B_n .. D_n).  FIRST: g_{n-1} and T_{n-1} are the module arrays; otherwise T_{n-1} is the
 // flow kernel's sum of the same pulled g_{n-1}.
 template <int D, bool FIRST, bool NARROW>
-__global__ void __launch_bounds__(128) k_thermal(Geo g, PhysC P, ExactArrays A, const double* __restrict__ fin,
-                                                 const double* __restrict__ gin, double* __restrict__ gout) {
+__global__ void __launch_bounds__(128) k_thermal(Geo g, PhysC P, ExactArrays A, const double* fin,
+                                                 const double* gin, double* gout) {
     long long c;
     int i, j, k;
     bool rows = false;

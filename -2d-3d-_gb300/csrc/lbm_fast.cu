@@ -96,8 +96,8 @@ __global__ void __launch_bounds__(128, (OneCellBlocks<S, true>::value)) k_fast_t
 // Against one cell per thread with branches in its pulls: 256^3 FP32 979 / 810 (6.5 TB/s on 313 B
 // per cell: bound by HBM), FP16 955 / 607; 96^3 FP16 89 / 34; 2D 2050x1025 FP32 75 / 63.
 template <int D, class S>
-__global__ void __launch_bounds__(128, 6) k_fast_flow_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
-                                                       const S* __restrict__ gin, S* __restrict__ fout) {
+__global__ void __launch_bounds__(128, 6) k_fast_flow_duo(Geo g, PhysF P, FastArgs<S> A, const S* fin,
+                                                       const S* gin, S* fout) {
     const Duo t = duo_cells(g, (int)blockIdx.x);
     wait_for_previous();
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(128, 6) k_fast_flow_duo(Geo g, PhysF P, FastAr
     start_next();
 }
 template <int D, class S>
-__global__ void __launch_bounds__(128, 7) k_fast_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fin,
-                                                          const S* __restrict__ gin, S* __restrict__ gout) {
+__global__ void __launch_bounds__(128, 7) k_fast_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* fin,
+                                                          const S* gin, S* gout) {
     const Duo t = duo_cells(g, last_first());
     wait_for_previous();
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;

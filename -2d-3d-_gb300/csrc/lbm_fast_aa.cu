@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(128) k_aa_thermal_p(Geo g, PhysF P, FastArgs<S
 // Two cells per thread, 32 apart (lbm_fast_aa_duo.cuh): resident blocks as for the two-buffer
 // kernels (lbm_fast.cu).
 template <int D, class S, bool ODD>
-__global__ void __launch_bounds__(128, 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs<S> A, S* f, const S* __restrict__ gs,
+__global__ void __launch_bounds__(128, 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs<S> A, S* f, const S* gs,
                                                      int raw) {
     const Duo t = duo_cells<true>(g, (int)blockIdx.x);
     wait_for_previous();
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(128, 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs
     start_next();
 }
 template <int D, class S, bool ODD>
-__global__ void __launch_bounds__(128, 7) k_aa_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* __restrict__ fs, S* gg,
+__global__ void __launch_bounds__(128, 7) k_aa_thermal_duo(Geo g, PhysF P, FastArgs<S> A, const S* fs, S* gg,
                                                         int raw) {
     const Duo t = duo_cells<true>(g, last_first());
     wait_for_previous();

@@ -27,7 +27,7 @@ __device__ __forceinline__ int push_index(const Geo& g, int n, int a, int i, int
 // One set read from the cells' own slots of the streamed layout; thermal values that were pushed
 // (raw) take the constant-temperature wall rule.
 template <int Q, bool TH, class S>
-__device__ __forceinline__ void duo_own_set(const Geo& g, const S* __restrict__ f, const Duo& t, bool raw, f2* d) {
+__device__ __forceinline__ void duo_own_set(const Geo& g, const S* f, const Duo& t, bool raw, f2* d) {
     const int n = (int)g.ncell;
     decltype(ld_raw(f)) x[2][Q];
 #pragma unroll
@@ -49,7 +49,7 @@ __device__ __forceinline__ void duo_own_set(const Geo& g, const S* __restrict__ 
 }
 
 template <int Q, bool TH, bool SWAPPED, class S>
-__device__ __forceinline__ void duo_layout_set(const Geo& g, const S* __restrict__ f, const Duo& t, bool raw, f2* d) {
+__device__ __forceinline__ void duo_layout_set(const Geo& g, const S* f, const Duo& t, bool raw, f2* d) {
     if (!SWAPPED) duo_own_set<Q, TH, S>(g, f, t, raw, d);
     else if (t.rows) duo_pull_set<Q, TH, false, S, true>(g, f, t, d);
     else duo_pull_set<Q, TH, true, S, true>(g, f, t, d);
@@ -102,7 +102,7 @@ __device__ __forceinline__ void duo_aa_store(const Geo& g, S* f, const Duo& t, c
 // aa_flow_cell and aa_thermal_cell (not FIRST) for both cells.
 template <int D, class S, bool ODD>
 __device__ __forceinline__ void aa_flow_duo(const Geo& g, const PhysF& P, const FastArgs<S>& A, S* f,
-                                            const S* __restrict__ gs, bool raw, const Duo& t, unsigned long long tick) {
+                                            const S* gs, bool raw, const Duo& t, unsigned long long tick) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     if (!t.in[0]) return;
     f2 d[Q], e[QT], ts = make_f2(0.0f, 0.0f);
@@ -118,7 +118,7 @@ __device__ __forceinline__ void aa_flow_duo(const Geo& g, const PhysF& P, const 
 
 template <int D, class S, bool ODD>
 __device__ __forceinline__ void aa_thermal_duo(const Geo& g, const PhysF& P, const FastArgs<S>& A,
-                                               const S* __restrict__ fs, S* gg, bool raw, const Duo& t,
+                                               const S* fs, S* gg, bool raw, const Duo& t,
                                                unsigned long long tick) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     if (!t.in[0]) return;

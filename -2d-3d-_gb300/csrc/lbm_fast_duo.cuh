@@ -66,11 +66,10 @@ __device__ __forceinline__ Duo duo_cells(const Geo& g, int block) {
                        (int)g.ncell);
 }
 
-// A stored population as loaded, and its value.
-__device__ __forceinline__ float ld_raw(const float* p) { return __ldg(p); }
-__device__ __forceinline__ unsigned short ld_raw(const __half* p) {
-    return __ldg(reinterpret_cast<const unsigned short*>(p));
-}
+// A stored population as loaded, and its value.  Not read-only loads: the kernel before may still
+// be writing when this one starts (lbm_launch.cuh).
+__device__ __forceinline__ float ld_raw(const float* p) { return *p; }
+__device__ __forceinline__ unsigned short ld_raw(const __half* p) { return *reinterpret_cast<const unsigned short*>(p); }
 __device__ __forceinline__ float raw_value(float x) { return x; }
 __device__ __forceinline__ float raw_value(unsigned short x) { return __half2float(__ushort_as_half(x)); }
 
@@ -91,7 +90,7 @@ __device__ __forceinline__ float wall_value(const Geo& g, const PullRule& r, int
 
 // The Q populations of one set pulled into both cells.
 template <int Q, bool TH, bool FACES, class S, bool SWAP = false>
-__device__ __forceinline__ void duo_pull_set(const Geo& g, const S* __restrict__ f, const Duo& t, f2* d) {
+__device__ __forceinline__ void duo_pull_set(const Geo& g, const S* f, const Duo& t, f2* d) {
     const int n = (int)g.ncell;
     const PullRule r = pull_rule<TH>(g);
     decltype(ld_raw(f)) x[2][Q];
@@ -113,7 +112,7 @@ __device__ __forceinline__ void duo_pull_set(const Geo& g, const S* __restrict__
     }
 }
 template <int Q, int QT, class S>
-__device__ __forceinline__ void duo_pull(const Geo& g, const S* __restrict__ f, const S* __restrict__ gs, const Duo& t,
+__device__ __forceinline__ void duo_pull(const Geo& g, const S* f, const S* gs, const Duo& t,
                                          f2* d, f2* e) {
     if (t.rows) {
         duo_pull_set<Q, false, false, S>(g, f, t, d);
@@ -124,7 +123,7 @@ __device__ __forceinline__ void duo_pull(const Geo& g, const S* __restrict__ f, 
     }
 }
 
-__device__ __forceinline__ f2 duo_load(const float* p, const Duo& t) { return make_f2(__ldg(p + t.c[0]), __ldg(p + t.c[1])); }
+__device__ __forceinline__ f2 duo_load(const float* p, const Duo& t) { return make_f2(p[t.c[0]], p[t.c[1]]); }
 __device__ __forceinline__ void duo_store(float* p, const Duo& t, f2 v) {
     if (t.in[0]) p[t.c[0]] = f2_lo(v);
     if (t.in[1]) p[t.c[1]] = f2_hi(v);
@@ -178,8 +177,8 @@ __device__ __forceinline__ unsigned long long thermal_tick(unsigned long long* t
 
 // flow_cell_2k and thermal_cell_2k (not FIRST) for both cells.
 template <int D, class S>
-__device__ __forceinline__ void flow_duo_2k(const Geo& g, const PhysF& P, const FastArgs<S>& A, const S* __restrict__ fin,
-                                            const S* __restrict__ gin, S* __restrict__ fout, const Duo& t,
+__device__ __forceinline__ void flow_duo_2k(const Geo& g, const PhysF& P, const FastArgs<S>& A, const S* fin,
+                                            const S* gin, S* fout, const Duo& t,
                                             unsigned long long tick) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     f2 d[Q], e[QT], ts = make_f2(0.0f, 0.0f);
@@ -194,8 +193,8 @@ __device__ __forceinline__ void flow_duo_2k(const Geo& g, const PhysF& P, const 
 
 template <int D, class S>
 __device__ __forceinline__ void thermal_duo_2k(const Geo& g, const PhysF& P, const FastArgs<S>& A,
-                                               const S* __restrict__ fin, const S* __restrict__ gin,
-                                               S* __restrict__ gout, const Duo& t, unsigned long long tick) {
+                                               const S* fin, const S* gin,
+                                               S* gout, const Duo& t, unsigned long long tick) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     f2 d[Q], e[QT];
     duo_pull<Q, QT, S>(g, fin, gin, t, d, e);

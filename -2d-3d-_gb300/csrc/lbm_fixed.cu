@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(128) k_xthermal_face(Geo g, PhysX X, FixedArra
 // 1659 / 1943 with the collision before (6.7 TB/s on 664 B per cell, 0.99 of the copy rate).
 template <int D>
 __global__ void __launch_bounds__(128, kXFlowBlocks) k_xflow_ix(Geo g, PhysX X, FixedArrays A,
-                                                     const long long* __restrict__ fin,
-                                                     const long long* __restrict__ gin, long long* __restrict__ fout) {
+                                                     const long long* fin,
+                                                     const long long* gin, long long* fout) {
     int c, i, j, k;
     bool rows;
     const bool in = index_cell(g, (int)blockIdx.x, c, i, j, k, rows);
@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(128, kXFlowBlocks) k_xflow_ix(Geo g, PhysX X, 
 
 template <int D>
 __global__ void __launch_bounds__(128, kXThermalBlocks) k_xthermal_ix(Geo g, PhysX X, FixedArrays A,
-                                                        const long long* __restrict__ fin,
-                                                        const long long* __restrict__ gin, long long* __restrict__ gout) {
+                                                        const long long* fin,
+                                                        const long long* gin, long long* gout) {
     int c, i, j, k;
     bool rows;
     const bool in = index_cell(g, last_first(), c, i, j, k, rows);

@@ -668,13 +668,14 @@ struct FixedArrays {
 
 namespace fxa {
 
-// Both population sets pulled into one cell by index (PATH 4 below).
+// Both population sets pulled into one cell by index (PATH 4 below).  Not read-only loads: the
+// kernel before may still be writing when this one starts (lbm_launch.cuh).
 template <int D>
 __device__ __forceinline__ void pull_cell(const Geo& g, const long long* fin, const long long* gin, long long c, int i,
                                           int j, int k, bool rows, q60* d, q60* e) {
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
-    pull_set_rows<Q, false, q60>(g, rows, i, j, k, (int)c, [&](int x) { return ldq(fin, x); }, d);
-    pull_set_rows<QT, true, q60>(g, rows, i, j, k, (int)c, [&](int x) { return ldq(gin, x); }, e);
+    pull_set_rows<Q, false, q60>(g, rows, i, j, k, (int)c, [&](int x) { return Qb(fin[x]); }, d);
+    pull_set_rows<QT, true, q60>(g, rows, i, j, k, (int)c, [&](int x) { return Qb(gin[x]); }, e);
 }
 
 // Flow collision of step n (lbm_exact.cu k_flow): FIRST reads the module arrays (f, rho,

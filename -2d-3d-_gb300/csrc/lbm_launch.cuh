@@ -11,6 +11,9 @@
 // accuracy 256x128 5.3 / 6.5 / 4.0 and 128x64 4.4 / 4.2 / 3.6).
 // Every kernel launched this way waits, so each one also finds everything before its predecessor
 // finished.
+// What such a kernel reads was written during its own lifetime, so it takes no read-only loads
+// (__ldg, or what the compiler makes of a const __restrict__ kernel parameter): those may be moved
+// above the wait or served from a cache that does not see the writes.
 #pragma once
 
 #include <cuda_runtime.h>
