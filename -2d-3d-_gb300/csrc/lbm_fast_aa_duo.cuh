@@ -13,14 +13,14 @@
 namespace lbm {
 
 // Slot that the push of direction a from a cell fills (aa_push on walls).
-template <int Q, bool FACES>
+template <int Q, int AT>
 __device__ __forceinline__ int push_index(const Geo& g, int n, int a, int i, int j, int k, int c) {
     const int ex = Lat<Q>::ex(a), ey = Lat<Q>::ey(a), ez = Lat<Q>::ez(a);
     const int back = Lat<Q>::opp(a) * n + c;
     int at = a * n + c + ex + g.nx * (ey + g.ny * ez);
-    if (ex != 0) at = (ex > 0 ? i == g.nx - 1 : i == 0) ? back : at;
-    if (FACES && ey != 0) at = (ey > 0 ? j == g.ny - 1 : j == 0) ? back : at;
-    if (FACES && ez != 0) at = (ez > 0 ? k == g.nz - 1 : k == 0) ? back : at;
+    if (AT != kInner && ex != 0) at = (ex > 0 ? i == g.nx - 1 : i == 0) ? back : at;
+    if (AT == kFaces && ey != 0) at = (ey > 0 ? j == g.ny - 1 : j == 0) ? back : at;
+    if (AT == kFaces && ez != 0) at = (ez > 0 ? k == g.nz - 1 : k == 0) ? back : at;
     return at;
 }
 
@@ -51,8 +51,9 @@ __device__ __forceinline__ void duo_own_set(const Geo& g, const S* f, const Duo&
 template <int Q, bool TH, bool SWAPPED, class S>
 __device__ __forceinline__ void duo_layout_set(const Geo& g, const S* f, const Duo& t, bool raw, f2* d) {
     if (!SWAPPED) duo_own_set<Q, TH, S>(g, f, t, raw, d);
-    else if (t.rows) duo_pull_set<Q, TH, false, S, true>(g, f, t, d);
-    else duo_pull_set<Q, TH, true, S, true>(g, f, t, d);
+    else if (t.inner) duo_pull_set<Q, TH, kInner, S, true>(g, f, t, d);
+    else if (t.rows) duo_pull_set<Q, TH, kRows, S, true>(g, f, t, d);
+    else duo_pull_set<Q, TH, kFaces, S, true>(g, f, t, d);
 }
 
 template <int Q>
@@ -83,18 +84,33 @@ __device__ __forceinline__ void duo_aa_store(const Geo& g, S* f, const Duo& t, c
     const int n = (int)g.ncell;
     S h[2][Q];
     duo_round<Q>(v, h[0], h[1], P, tick, t, kind);
+    if (!ODD) {
 #pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        if (!t.in[w]) continue;
-        if (!ODD) {
+        for (int w = 0; w < 2; ++w) {
+            if (!t.in[w]) continue;
 #pragma unroll
             for (int a = 0; a < Q; ++a) f[Lat<Q>::opp(a) * n + t.c[w]] = h[w][a];
-        } else if (t.rows) {
+        }
+    } else if (t.inner) {
 #pragma unroll
-            for (int a = 0; a < Q; ++a) f[push_index<Q, false>(g, n, a, t.i[w], t.j[w], t.k[w], t.c[w])] = h[w][a];
-        } else {
+        for (int a = 0; a < Q; ++a) {
+            S* p = f + push_index<Q, kInner>(g, n, a, 0, 0, 0, t.c[0]);
+            p[0] = h[0][a];
+            if (t.in[1]) p[32] = h[1][a];
+        }
+    } else {
 #pragma unroll
-            for (int a = 0; a < Q; ++a) f[push_index<Q, true>(g, n, a, t.i[w], t.j[w], t.k[w], t.c[w])] = h[w][a];
+        for (int w = 0; w < 2; ++w) {
+            if (!t.in[w]) continue;
+            if (t.rows) {
+#pragma unroll
+                for (int a = 0; a < Q; ++a)
+                    f[push_index<Q, kRows>(g, n, a, t.i[w], t.j[w], t.k[w], t.c[0] + 32 * w)] = h[w][a];
+            } else {
+#pragma unroll
+                for (int a = 0; a < Q; ++a)
+                    f[push_index<Q, kFaces>(g, n, a, t.i[w], t.j[w], t.k[w], t.c[0] + 32 * w)] = h[w][a];
+            }
         }
     }
 }

@@ -4,9 +4,12 @@
 // A warp covers 64 consecutive cells: lane l holds cells c and c + 32.  Every access of a warp is
 // a run of 32 consecutive values as in the one-cell kernels, whatever the row length (no
 // alignment to keep, no x shift to assemble), the second cell's address is the first's plus a
-// constant, and the arithmetic runs on both cells at once (f2).  The cells of a warp whose rows
-// lie off the y and z faces select for the x faces only; a warp that holds a cell of a y or z face
-// row selects for all.  Only the loads are inside that choice.
+// constant, and the arithmetic runs on both cells at once (f2).  A warp off every face reads
+// at fixed distances, one whose rows lie off the y and z faces selects for the x faces, and one that
+// holds a cell of a y or z face row selects for all.  Only the loads are inside that choice.
+// The first of the three took index arithmetic out of kernels whose integer pipe was 48% busy
+// (GB300, us per step before / after: FP16 2D 2050x1025 44.7 / 42.7, 256^3 605 / 598, 384^3 in
+// place 2195 / 2145; FP32 is bound by HBM and unchanged; 60 2D FP32 lattices together 262 / 248).
 // 32-bit indices: q * ncell < 2^31 - 64.
 #pragma once
 
@@ -19,6 +22,7 @@ struct Duo {
     bool in[2];   // whether the lane has them
     int i[2], j[2], k[2];
     bool rows;    // every cell of the warp lies on a row off the y and z faces
+    bool inner;   // every cell of the warp lies off every face
 };
 
 // Cells c0 and c0 + 32 of a lane (called by whole warps), those below `end`.  A cell beyond the
@@ -56,7 +60,9 @@ __device__ __forceinline__ Duo duo_at(const Geo& g, int c0, int end) {
         t.k[1] = OWN ? t.k[0] : g.nz - 1;
     }
     const bool off = row_off_faces(g, t.j[0], t.k[0]) && row_off_faces(g, t.j[1], t.k[1]);
+    const bool xoff = t.i[0] > 0 && t.i[0] < g.nx - 1 && t.i[1] > 0 && t.i[1] < g.nx - 1;
     t.rows = __all_sync(0xFFFFFFFFu, off);
+    t.inner = __all_sync(0xFFFFFFFFu, off && xoff);
     return t;
 }
 // The cells of block `block` of a single-lattice launch (ncell / 256 blocks of 128 threads, rounded up).
@@ -88,17 +94,30 @@ __device__ __forceinline__ float wall_value(const Geo& g, const PullRule& r, int
     return v;
 }
 
+// Where the cells of a warp lie: off every face, on rows off the y and z faces, anywhere.  In the
+// first two the second cell is the first plus 32 (the lattice's last cell lies on a face row), so
+// its values are read at a constant distance, and off the faces no index is selected.
+constexpr int kInner = 0, kRows = 1, kFaces = 2;
+
 // The Q populations of one set pulled into both cells.
-template <int Q, bool TH, bool FACES, class S, bool SWAP = false>
+template <int Q, bool TH, int AT, class S, bool SWAP = false>
 __device__ __forceinline__ void duo_pull_set(const Geo& g, const S* f, const Duo& t, f2* d) {
     const int n = (int)g.ncell;
     const PullRule r = pull_rule<TH>(g);
     decltype(ld_raw(f)) x[2][Q];
 #pragma unroll
     for (int a = 0; a < Q; ++a) {
+        if (AT == kInner) {
+            const S* p = f + (SWAP ? Lat<Q>::opp(a) : a) * n + t.c[0]
+                         - (Lat<Q>::ex(a) + g.nx * (Lat<Q>::ey(a) + g.ny * Lat<Q>::ez(a)));
+            x[0][a] = ld_raw(p);
+            x[1][a] = ld_raw(p + 32);
+            continue;
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-            x[h][a] = ld_raw(f + pull_index<Q, FACES, SWAP>(g, n, r, a, t.i[h], t.j[h], t.k[h], t.c[h]));
+            x[h][a] = ld_raw(f + pull_index<Q, AT == kFaces, SWAP>(g, n, r, a, t.i[h], t.j[h], t.k[h],
+                                                                  AT == kFaces ? t.c[h] : t.c[0] + 32 * h));
     }
 #pragma unroll
     for (int a = 0; a < Q; ++a) {
@@ -106,7 +125,7 @@ __device__ __forceinline__ void duo_pull_set(const Geo& g, const S* f, const Duo
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             v[h] = raw_value(x[h][a]);
-            if (TH) v[h] = wall_value<Q, FACES>(g, r, a, t.i[h], t.j[h], v[h]);
+            if (TH && AT != kInner) v[h] = wall_value<Q, AT == kFaces>(g, r, a, t.i[h], t.j[h], v[h]);
         }
         d[a] = make_f2(v[0], v[1]);
     }
@@ -114,12 +133,15 @@ __device__ __forceinline__ void duo_pull_set(const Geo& g, const S* f, const Duo
 template <int Q, int QT, class S>
 __device__ __forceinline__ void duo_pull(const Geo& g, const S* f, const S* gs, const Duo& t,
                                          f2* d, f2* e) {
-    if (t.rows) {
-        duo_pull_set<Q, false, false, S>(g, f, t, d);
-        duo_pull_set<QT, true, false, S>(g, gs, t, e);
+    if (t.inner) {
+        duo_pull_set<Q, false, kInner, S>(g, f, t, d);
+        duo_pull_set<QT, true, kInner, S>(g, gs, t, e);
+    } else if (t.rows) {
+        duo_pull_set<Q, false, kRows, S>(g, f, t, d);
+        duo_pull_set<QT, true, kRows, S>(g, gs, t, e);
     } else {
-        duo_pull_set<Q, false, true, S>(g, f, t, d);
-        duo_pull_set<QT, true, true, S>(g, gs, t, e);
+        duo_pull_set<Q, false, kFaces, S>(g, f, t, d);
+        duo_pull_set<QT, true, kFaces, S>(g, gs, t, e);
     }
 }
 
@@ -133,30 +155,32 @@ __device__ __forceinline__ void duo_store(float* p, const Duo& t, f2 v) {
 template <int Q>
 __device__ __forceinline__ void duo_store_pops(float* out, int n, const Duo& t, const f2* v, const PhysF&, unsigned long long,
                                                unsigned) {
-    if (t.in[1]) {
+    if (t.in[0]) {
 #pragma unroll
         for (int a = 0; a < Q; ++a) {
-            out[a * n + t.c[0]] = f2_lo(v[a]);
-            out[a * n + t.c[1]] = f2_hi(v[a]);
+            float* p = out + a * n + t.c[0];
+            p[0] = f2_lo(v[a]);
+            if (t.in[1]) p[32] = f2_hi(v[a]);
         }
-    } else if (t.in[0]) {
-#pragma unroll
-        for (int a = 0; a < Q; ++a) out[a * n + t.c[0]] = f2_lo(v[a]);
     }
 }
 template <int Q>
 __device__ __forceinline__ void duo_store_pops(__half* out, int n, const Duo& t, const f2* v, const PhysF& P,
                                                unsigned long long tick, unsigned kind) {
     float x[Q];
-    __half h[Q];
+    __half h[2][Q];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
 #pragma unroll
         for (int a = 0; a < Q; ++a) x[a] = w ? f2_hi(v[a]) : f2_lo(v[a]);
-        round_cell<Q>(x, h, P.sr != 0, sr_seed(tick, t.c[w], kind));
-        if (t.in[w]) {
+        round_cell<Q>(x, h[w], P.sr != 0, sr_seed(tick, t.c[w], kind));
+    }
+    if (t.in[0]) {
 #pragma unroll
-            for (int a = 0; a < Q; ++a) out[a * n + t.c[w]] = h[a];
+        for (int a = 0; a < Q; ++a) {
+            __half* p = out + a * n + t.c[0];
+            p[0] = h[0][a];
+            if (t.in[1]) p[32] = h[1][a];
         }
     }
 }
