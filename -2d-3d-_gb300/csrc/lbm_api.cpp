@@ -12,6 +12,8 @@
 // holds after iteration N, so stepping resumes on the same trajectory).
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <utility>
@@ -21,6 +23,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/lbm_gpu.h"
@@ -1424,6 +1427,42 @@ static double* scalar_ptr(lbm_handle* h, int field) {
     }
 }
 
+// Bring the pages of an array that is about to be written whole into memory, with a few threads.
+// A copy into a fresh allocation otherwise takes one page fault after the other (GB300 host: 27
+// GB/s, against 90 GB/s for the copy itself; lbm_get_state into fresh arrays before / after:
+// 134 MB 6.6 / 4.0 ms, 453 MB 19 / 11 ms).
+// Only whole pages inside the array are touched; where the kernel refuses (older kernels, other
+// kinds of memory), the copy faults them as before.
+static void populate_pages(void* dst, size_t bytes) {
+    // bytes a thread takes: below, starting one costs what it saves.  More than four threads wait for
+    // each other in the kernel (453 MB by 1 / 2 / 4 / 8 / 16 threads: 14.0 / 7.6 / 4.9 / 6.8 / 7.9 ms).
+    constexpr size_t kEach = size_t(4) << 20;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t b = ((uintptr_t)dst + page - 1) / page * page, e = ((uintptr_t)dst + bytes) / page * page;
+    if (e <= b || e - b < kEach) return;
+    const size_t n = std::min<size_t>({4, (e - b) / kEach, std::max(1u, std::thread::hardware_concurrency())});
+    const size_t each = ((e - b) / n + page - 1) / page * page;
+    auto part = [=](size_t t) {
+        const uintptr_t at = b + t * each;
+        if (at < e) madvise((void*)at, std::min<size_t>(each, e - at), MADV_POPULATE_WRITE);
+    };
+    std::vector<std::thread> others;
+    try {
+        others.reserve(n);
+        for (size_t t = 1; t < n; ++t) others.emplace_back(part, t);
+    } catch (...) {  // no more threads: the pages left over fault in the copy
+    }
+    part(0);
+    for (std::thread& t : others) t.join();
+}
+
+// A device array into the caller's host array, on the handle's stream; the pages are brought in
+// while the kernels before the copy run.
+static cudaError_t copy_out(lbm_handle* h, double* dst, const double* src, size_t count) {
+    populate_pages(dst, count * sizeof(double));
+    return cudaMemcpyAsync(dst, src, count * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+}
+
 static int state_io(lbm_handle* h, int field, double* dst, const double* src, size_t count) {
     NvtxRange range_("state transfer");
     if (!h || (!dst && !src)) return LBM_ERR_PARAM;
@@ -1449,7 +1488,7 @@ static int state_io(lbm_handle* h, int field, double* dst, const double* src, si
             st = fast_export(h->F, h->geo, h->phys, h->dim, field, h->d_stage, h->stream);
             if (st != LBM_OK) return fail(h, st, "field not available for this precision");
             CK_LAUNCH(h, "export");
-            CK(h, cudaMemcpyAsync(dst, h->d_stage, want * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+            CK(h, copy_out(h, dst, h->d_stage, want));
             CK(h, cudaStreamSynchronize(h->stream));
         } else {
             CK(h, cudaMemcpyAsync(h->d_stage, src, want * sizeof(double), cudaMemcpyHostToDevice, h->stream));
@@ -1469,14 +1508,14 @@ static int state_io(lbm_handle* h, int field, double* dst, const double* src, si
             aa_module_view(h->geo, qq, th, LBM_FP64, soa, th ? h->aa.gpar : h->aa.fpar, h->aa.graw, h->d_stage, false,
                            false, 0.0, 0.0, h->stream);
             CK_LAUNCH(h, "module view");
-            CK(h, cudaMemcpyAsync(dst, h->d_stage, want * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+            CK(h, copy_out(h, dst, h->d_stage, want));
         } else if (dst && h->host_direct_wr) {
             soa_to_aos(soa, dst, qq, n, h->stream);  // written straight into the caller's array
             CK_LAUNCH(h, "soa_to_aos");
         } else if (dst) {
             soa_to_aos(soa, h->d_stage, qq, n, h->stream);
             CK_LAUNCH(h, "soa_to_aos");
-            CK(h, cudaMemcpyAsync(dst, h->d_stage, want * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+            CK(h, copy_out(h, dst, h->d_stage, want));
         } else {
             if (h->host_direct) {
                 aos_to_soa(src, soa, qq, n, h->stream);  // read straight from the caller's array
@@ -1501,7 +1540,7 @@ static int state_io(lbm_handle* h, int field, double* dst, const double* src, si
         copy_doubles(dst ? d : src, dst ? dst : d, (long long)want, h->stream);
         CK_LAUNCH(h, "field copy");
     } else if (dst) {
-        CK(h, cudaMemcpyAsync(dst, d, want * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        CK(h, copy_out(h, dst, d, want));
     } else {
         CK(h, cudaMemcpyAsync(d, src, want * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     }
