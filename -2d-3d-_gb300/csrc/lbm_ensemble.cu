@@ -1,5 +1,5 @@
-// lbm_ensemble.cu - one flow launch and one thermal launch per time step for any number of
-// FP32/FP16 lattices of uneven sizes and parameters (the batched form).
+// lbm_ensemble.cu - one flow launch and one thermal launch per time step (FP32 in 2D: one launch) for
+// any number of FP32/FP16 lattices of uneven sizes and parameters (the batched form).
 //
 // A grid of about SMs x grid_mul persistent blocks walks a packed tile table: tile t is
 // (member m, first cell c0) and covers tile_cells consecutive cells of member m.  Each
@@ -14,6 +14,7 @@
 
 #include "lbm_ensemble.h"
 #include "lbm_fast_duo.cuh"
+#include "lbm_fast_tile.cuh"
 #include "lbm_launch.cuh"
 
 namespace lbm {
@@ -28,6 +29,7 @@ struct EnsMember {
     float* L[2];
     unsigned long long* tick;  // the member's step counter (stochastic rounding of FP16)
     int cur;    // buffer parity when the table was built
+    TilePlan tp;  // 2D: its tiles of the one-launch step
 };
 
 // Resident blocks of 128 threads per SM (the launch asks for half of them with 256): six, as the
@@ -163,6 +165,39 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEn
     start_next();
 }
 
+// Rows of a block of the one-launch 2D step.
+constexpr int kEnsRows = 8;
+
+// The 2D members' step in one launch (lbm_fast_tile.cuh).  FP32 only: as for one lattice, half
+// storage saves too little traffic to pay for the cells that are collided twice.  GB300, 60 members
+// of up to 1024x512: 179 us a step; 200 steps and the read-out 44.7 ms against 49.5 of two kernels.
+__global__ void __launch_bounds__(32 * kEnsRows, 32 / kEnsRows)
+    k_ens_tile(const EnsMember<float>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int flip) {
+    using S = float;
+    __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];
+    __shared__ float sf[8 * 64 * kEnsRows];
+    wait_for_previous();
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int2 tt = tiles[flip ? ntiles - 1 - t : t];  // every other step last tile first, as k_fast_tile
+        const EnsStage<S>& st = stage_member<S>(mem, tt.x, sh, [flip](const EnsMember<S>& gm, FastArgs<S>& A) {
+            const int c = gm.cur ^ flip, n = c ^ 1;
+            A.Bin0 = gm.B[c][0]; A.Bin1 = gm.B[c][1];
+            A.Bout0 = gm.B[n][0]; A.Bout1 = gm.B[n][1];
+            A.lag_in = gm.L[c];
+            A.lag_out = gm.L[n];
+            A.ticks = gm.tick;
+        });
+        const EnsMember<S>& m = st.m;
+        const int cur = m.cur ^ flip, nxt = cur ^ 1;
+        tile_step<S, kEnsRows>(m.g, m.P, m.tp, st.A, st.A, m.f[cur], m.gp[cur], m.f[nxt], m.gp[nxt], tt.y, 0ULL, sf);
+        tile_tick<S>(st.A.ticks, (unsigned)(m.tp.ntx * m.tp.nty), tt.y == 0 && threadIdx.x == 0);
+    }
+    start_next();
+}
+
+// Lists whose step is one launch.
+static bool one_launch(const EnsPlan& plan, int li) { return li == 0 && plan.precision == LBM_FP32; }
+
 template <class S>
 static cudaError_t build_typed(EnsPlan& plan, const std::vector<EnsMemberHost>& members) {
     for (int li = 0; li < kEnsLists; ++li) {
@@ -184,7 +219,9 @@ static cudaError_t build_typed(EnsPlan& plan, const std::vector<EnsMemberHost>& 
             }
             m.cur = mh.F->cur;
             const int idx = (int)hm.size();
-            const long long nt = (m.g.ncell + plan.cfg.tile_cells - 1) / plan.cfg.tile_cells;
+            m.tp = tile_plan(m.g, kEnsRows);
+            const long long nt = one_launch(plan, li) ? (long long)m.tp.ntx * m.tp.nty
+                                                      : (m.g.ncell + plan.cfg.tile_cells - 1) / plan.cfg.tile_cells;
             for (long long t = 0; t < nt; ++t) tiles.push_back(make_int2(idx, (int)t));
             plan.cells += m.g.ncell;
             hm.push_back(m);
@@ -249,6 +286,13 @@ static void step_typed(const EnsPlan& plan, int flip, cudaStream_t s) {
     for (int stage = 0; stage < 2; ++stage) {
         for (int li = 0; li < kEnsLists; ++li) {
             if (plan.ntiles[li] == 0) continue;
+            if (one_launch(plan, li)) {
+                if (stage == 1) continue;
+                const unsigned grid = (unsigned)min(plan.ntiles[li], plan.sms * plan.cfg.grid_mul);
+                launch_after(k_ens_tile, grid, 32 * kEnsRows, s, (const EnsMember<float>*)plan.d_members[li],
+                             plan.d_tiles[li], plan.ntiles[li], flip);
+                continue;
+            }
             switch (li) {
                 case 0: launch_list<2, S, false>(plan, li, stage, flip, s); break;
                 case 1: launch_list<3, S, false>(plan, li, stage, flip, s); break;

@@ -14,6 +14,7 @@
 #include "lbm_fast.h"
 #include "lbm_fast_cells.cuh"
 #include "lbm_fast_duo.cuh"
+#include "lbm_fast_tile.cuh"
 #include "lbm_fast_pairs.cuh"
 #include "lbm_launch.cuh"
 
@@ -113,6 +114,19 @@ __global__ void __launch_bounds__(128, 7) k_fast_thermal_duo(Geo g, PhysF P, Fas
     const bool one = blockIdx.x == 0 && threadIdx.x == 0;
     const unsigned long long tick = sizeof(S) == 2 || one ? thermal_tick(A.ticks, one) : 0ULL;
     thermal_duo_2k<D, S>(g, P, A, fin, gin, gout, t, tick);
+    start_next();
+}
+
+// The 2D step in one launch (lbm_fast_tile.cuh), blocks of W rows of 64 cells.
+template <class S, int W>
+__global__ void __launch_bounds__(32 * W, 32 / W) k_fast_tile(Geo g, PhysF P, TilePlan tp, FastArgs<S> Af, FastArgs<S> At,
+                                                           const S* fin, const S* gin, S* fout, S* gout, int reverse) {
+    __shared__ float sf[8 * 64 * W];
+    wait_for_previous();
+    const unsigned long long tick = sizeof(S) == 2 ? Af.ticks[0] : 0ULL;
+    // every other step runs its blocks last first: it finds what the step before touched last in L2
+    tile_step<S, W>(g, P, tp, Af, At, fin, gin, fout, gout, reverse ? last_first() : (int)blockIdx.x, tick, sf);
+    tile_tick<S>(Af.ticks, gridDim.x, blockIdx.x == 0 && threadIdx.x == 0);
     start_next();
 }
 
@@ -221,6 +235,33 @@ static void duo_step(const Geo& g, const PhysF& pf, const FastArgs<S>& Af, const
     if (th) launch_after(k_fast_thermal_duo<D, S>, nb2, 128, s, g, pf, At, fout, gin, gout);
 }
 
+// Rows of a block of the one-launch 2D step, or 0 for the two kernels.  One launch saves the way
+// from one kernel to the next, and FP32 traffic; it collides the ring of each tile twice.
+// GB300, us per step of the two kernels / with 8 rows / 4 rows:
+//   FP32 128x64 2.95 / 2.69 / 2.38, 256x128 3.29 / 2.82 / 2.69, 512x256 4.42 / 4.04 / 4.47,
+//        401x777 7.07 / 7.22 / 8.09, 1024x512 9.84 / 9.81 / 11.3, 2050x1025 55.3 / 47.8 / 53.8,
+//        4096x2048 223 / 189 / 213 (16 rows: 190);
+//   FP16 128x64 3.78 / 3.97 / 3.50, 256x128 4.23 / 3.96 / 3.97, 512x256 5.10 / 5.19 / 5.77,
+//        2050x1025 43.1 / 44.6 / 58.4, 4096x2048 171 / 177 / 226.
+// So: four rows while eight would leave SMs without a block; eight in FP32 while the blocks run at
+// once (four per SM), and where the state does not fit L2 and its traffic counts.
+static int tile_rows(const FastState& F, const Geo& g) {
+    const TilePlan tp = tile_plan(g, 8);
+    const long long blocks = (long long)tp.ntx * tp.nty;
+    if (blocks <= F.sms) return 4;
+    const bool large = g.ncell * 136 > F.l2;
+    return F.precision == LBM_FP32 && (blocks <= 4LL * F.sms || large) ? 8 : 0;
+}
+
+template <class S>
+static void tile_launch(int rows, const Geo& g, const PhysF& pf, const FastArgs<S>& Af, const FastArgs<S>& At, const S* fin,
+                        const S* gin, S* fout, S* gout, int cur, cudaStream_t s) {
+    const TilePlan tp = tile_plan(g, rows);
+    const unsigned nb = (unsigned)(tp.ntx * tp.nty);
+    if (rows == 4) launch_after(k_fast_tile<S, 4>, nb, 128, s, g, pf, tp, Af, At, fin, gin, fout, gout, cur);
+    else launch_after(k_fast_tile<S, 8>, nb, 256, s, g, pf, tp, Af, At, fin, gin, fout, gout, cur);
+}
+
 template <int D, class S>
 static void rows_step(const Geo& g, const PhysF& pf, const FastArgs<S>& Af, const FastArgs<S>& At, const S* fin,
                       const S* gin, S* fout, S* gout, cudaStream_t s, bool fl, bool th) {
@@ -323,6 +364,10 @@ void fast_tick(FastState& F, cudaStream_t s) { k_tick<<<1, 1, 0, s>>>(F.tick); }
 
 int fast_allocate(FastState& F, const lbm_params& p, const Geo& g, const AllocFn& alloc) {
     F.precision = p.precision;
+    int dev = 0, sms = 0, l2 = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) F.sms = sms;
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess && l2 > 0) F.l2 = l2;
     // x-adjacent pairs and staged rows on request (LBM_OPT_PAIRS, LBM_OPT_STAGED)
     F.tma = false;
     F.pairs = false;
@@ -344,8 +389,8 @@ int fast_allocate(FastState& F, const lbm_params& p, const Geo& g, const AllocFn
     }
     if ((st = alloc((void**)&F.err, sizeof(int))) != LBM_OK) return st;
     if (cudaMemset(F.err, 0, sizeof(int)) != cudaSuccess) return LBM_ERR_CUDA;
-    if ((st = alloc((void**)&F.tick, 2 * sizeof(unsigned long long))) != LBM_OK) return st;
-    if (cudaMemset(F.tick, 0, 2 * sizeof(unsigned long long)) != cudaSuccess) return LBM_ERR_CUDA;
+    if ((st = alloc((void**)&F.tick, 3 * sizeof(unsigned long long))) != LBM_OK) return st;
+    if (cudaMemset(F.tick, 0, 3 * sizeof(unsigned long long)) != cudaSuccess) return LBM_ERR_CUDA;
     F.sr = p.precision == LBM_FP16;
     if (F.aa) {
         // one array each, which is also the module array; the lag fields are read and
@@ -465,7 +510,9 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
             } else if (rows) {
                 rows_step<2, S>(g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
             } else if (idx32) {
-                duo_step<2, S>(g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
+                const int rows_of = fl && th ? tile_rows(F, g) : 0;
+                if (rows_of) tile_launch<S>(rows_of, g, pf, Af, At, fin, gin, fout, gout, cur, s);
+                else duo_step<2, S>(g, pf, Af, At, fin, gin, fout, gout, s, fl, th);
                 ticked = true;
             } else {
                 one_cell_step<2, false, S>(false, blocks, g, pf, Af, At, fin, gin, fout, gout, s, fl, th);

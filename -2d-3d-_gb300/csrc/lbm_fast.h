@@ -25,6 +25,8 @@ struct PhysF;
 
 struct FastState {
     int precision = LBM_FP32;  // LBM_FP32 or LBM_FP16
+    int sms = 152;             // of the device: its SMs and L2 bytes
+    long long l2 = 129LL << 20;
     int dim = 3, q = 19, qt = 7;
     size_t esize = 4;          // bytes per stored population
     void* fbuf[2] = {nullptr, nullptr};
@@ -42,7 +44,7 @@ struct FastState {
     bool single_kernel = false; // one-launch fused step (lbm_fused.cu); off: the two-kernel step is faster today
     int kchunk = 16;            // z planes per block of the fused kernel (3D)
     // Form of the non-first two-kernel step: two cells per thread with packed arithmetic
-    // (lbm_fast_duo.cuh) where 32-bit indices fit; x-adjacent pairs, staged rows
+    // (lbm_fast_duo.cuh; in 2D also one launch, lbm_fast_tile.cuh) where 32-bit indices fit; x-adjacent pairs, staged rows
     // (lbm_fast_tma.cu) or row launches on request.
     bool pairs = false;
     bool tma = false;
@@ -55,7 +57,8 @@ struct FastState {
     AAState AA;
     // FP16 storage rounds new populations stochastically (lbm_fast_math.cuh, storeS), with
     // random bits keyed on this device step counter (steps since initial; continuation
-    // records keep it).  tick[1]: its copy for the thermal kernels of lbm_fast_duo.cuh.
+    // records keep it).  tick[1]: its copy for the thermal kernels of lbm_fast_duo.cuh; tick[2]:
+    // blocks of a step that have arrived (lbm_fast_tile.cuh).
     bool sr = false;
     unsigned long long* tick = nullptr;
 };

@@ -112,12 +112,12 @@ __device__ __forceinline__ void duo_pull_set(const Geo& g, const S* f, const Duo
                          - (Lat<Q>::ex(a) + g.nx * (Lat<Q>::ey(a) + g.ny * Lat<Q>::ez(a)));
             x[0][a] = ld_raw(p);
             x[1][a] = ld_raw(p + 32);
-            continue;
-        }
+        } else {
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-            x[h][a] = ld_raw(f + pull_index<Q, AT == kFaces, SWAP>(g, n, r, a, t.i[h], t.j[h], t.k[h],
-                                                                  AT == kFaces ? t.c[h] : t.c[0] + 32 * h));
+            for (int h = 0; h < 2; ++h)
+                x[h][a] = ld_raw(f + pull_index<Q, AT == kFaces, SWAP>(g, n, r, a, t.i[h], t.j[h], t.k[h],
+                                                                      AT == kFaces ? t.c[h] : t.c[0] + 32 * h));
+        }
     }
 #pragma unroll
     for (int a = 0; a < Q; ++a) {

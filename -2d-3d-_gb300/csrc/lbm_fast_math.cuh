@@ -88,6 +88,10 @@ __device__ __forceinline__ void round_cell(const float* v, __half* h, bool sr, u
         }
     }
 }
+// A rounded population as a pull reads it back.
+__device__ __forceinline__ float stored_value(float h) { return h; }
+__device__ __forceinline__ float stored_value(__half h) { return __half2float(h); }
+
 // Rest weights (D2Q9 2DRB.F90:506-512, D3Q19 3DRB.F90:669-671).
 template <int Q>
 __host__ __device__ constexpr double wrest(int a) {

@@ -44,10 +44,6 @@ struct Tile;
 template <> struct Tile<3> { static constexpr int TX = 32, TY = 8, MINB = 2; };
 template <> struct Tile<2> { static constexpr int TX = 32, TY = 4, MINB = 4; };
 
-// A stored population as a pull reads it back (ldS).
-__device__ __forceinline__ float stored_value(float h) { return h; }
-__device__ __forceinline__ float stored_value(__half h) { return __half2float(h); }
-
 // Thermal stage at one cell: pulls, macro, thermal collision.  Returns g_post_n as the
 // next pull reads it (GP: the stored deviations, rounded to the storage type and back; halo
 // cells round with the owner's random bits, so they hold the owner's values) and the lag of
