@@ -47,6 +47,7 @@ struct lbm_handle {
     lbm_constants c;
     int dim = 3, q = 19, qt = 7;
     int device = 0;
+    int sms = 152;  // of the device
     cudaStream_t stream = nullptr;
     Geo geo{};
     PhysC phys{};
@@ -71,6 +72,7 @@ struct lbm_handle {
     PhysX px{};
     Geo xgeo{};  // geometry with the thermal wall terms of deviations
     long long *xb0 = nullptr, *xb1 = nullptr, *xb2 = nullptr, *xlag = nullptr;
+    long long* xlag1 = nullptr;  // 2D: the force of the odd buffers (cells around a tile read the old one)
     // fused passes (lbm_fixed.cu k_xfused): B_prev double-buffered, the graph of a chunk of
     // passes and the state it was captured from
     // LBM_OPT_SINGLE_KERNEL on a fixed handle.  Off by default: on GB300 the fused pass reads
@@ -390,6 +392,7 @@ static int allocate(lbm_handle* h) {
             AL(h->xb1, n);
             if (d3) AL(h->xb2, n);
             AL(h->xlag, n);
+            if (!d3) AL(h->xlag1, n);
             if (d3 && fixed_fused_supported(h->geo, h->dim)) {
                 AL(h->xb0b, n);
                 AL(h->xb1b, n);
@@ -470,7 +473,8 @@ extern "C" int lbm_create(const lbm_params* p, int device, lbm_handle** out) {
         delete h;
         return st;
     }
-    int pageable = 0;
+    int sms = 0, pageable = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) h->sms = sms;
     if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess && pageable) {
         // reads of the caller's array by the layout kernels only: writes into freshly
         // allocated host memory fault its pages in from the GPU side, measured at 3-4.5 GB/s
@@ -604,7 +608,7 @@ extern "C" int lbm_initial(lbm_handle* h) {
     return LBM_OK;
 }
 
-// The arrays the fixed-arithmetic kernels read and write.
+// The arrays that a step of the fixed arithmetic from fbuf[cur] reads and writes.
 static FixedArrays fixed_arrays(const lbm_handle* h) {
     const ExactArrays& A = h->A;
     FixedArrays X{};
@@ -625,6 +629,10 @@ static FixedArrays fixed_arrays(const lbm_handle* h) {
     X.xb1 = h->xb1;
     X.xb2 = h->xb2;
     X.xlag = h->xlag;
+    if (h->dim == 2) {
+        X.xlag_in = h->cur ? h->xlag1 : h->xlag;
+        X.xlag = h->cur ? h->xlag : h->xlag1;
+    }
     return X;
 }
 
@@ -641,7 +649,9 @@ static int materialize(lbm_handle* h, bool pops) {
     }
     if (!h->fused_valid) return LBM_OK;
     if (h->fixed) {
-        fixed_materialize(h->xgeo, h->px, fixed_arrays(h), h->dim, (const long long*)h->fbuf[h->cur],
+        FixedArrays X = fixed_arrays(h);
+        if (h->dim == 2) X.xlag = h->cur ? h->xlag1 : h->xlag;  // of the current step
+        fixed_materialize(h->xgeo, h->px, X, h->dim, (const long long*)h->fbuf[h->cur],
                           (const long long*)h->gbuf[h->cur], pops, h->stream);
         CK_LAUNCH(h, "materialize");
         return LBM_OK;
@@ -724,7 +734,7 @@ static void enqueue_one(lbm_handle* h, bool first) {
     } else if (h->p.precision == LBM_FP64 && h->fixed) {
         fixed_fused_step(h->xgeo, h->px, fixed_arrays(h), h->dim, first, (const long long*)h->fbuf[h->cur],
                          (const long long*)h->gbuf[h->cur], (long long*)h->fbuf[nxt], (long long*)h->gbuf[nxt],
-                         h->stream, 2, h->wide_index);
+                         h->stream, 2, h->wide_index, h->sms);
         h->cur = nxt;
     } else if (h->p.precision == LBM_FP64) {
         exact_fused_step(h->geo, h->phys, h->A, h->dim, first, h->fbuf[h->cur], h->gbuf[h->cur], h->fbuf[nxt],
@@ -782,7 +792,7 @@ static void x_enter(lbm_handle* h) {
     const int nxt = h->cur ^ 1;
     fixed_fused_step(h->xgeo, h->px, fixed_arrays(h), h->dim, false, (const long long*)h->fbuf[h->cur],
                      (const long long*)h->gbuf[h->cur], (long long*)h->fbuf[nxt], nullptr, h->stream, 0,
-                     h->wide_index);
+                     h->wide_index, h->sms);
     h->cur = nxt;  // f is one step ahead: fbuf[cur] = f_post_{N+1}, gbuf[cur ^ 1] = g_post_N
 }
 
@@ -801,7 +811,7 @@ static void x_pass(lbm_handle* h) {
 static void x_exit(lbm_handle* h) {
     const int c = h->cur;
     fixed_fused_step(h->xgeo, h->px, fixed_arrays(h), h->dim, false, nullptr, (const long long*)h->gbuf[c ^ 1],
-                     (long long*)h->fbuf[c], (long long*)h->gbuf[c], h->stream, 1, h->wide_index);
+                     (long long*)h->fbuf[c], (long long*)h->gbuf[c], h->stream, 1, h->wide_index, h->sms);
 }
 
 // Capture key of a chunk of fused passes: the buffer parity and which B_prev set is current.
@@ -2009,9 +2019,9 @@ extern "C" int lbm_time_kernels(lbm_handle* h, int64_t nsteps, double* ms_flow, 
             const FixedArrays X = fixed_arrays(h);
             const long long *fc = (const long long*)h->fbuf[h->cur], *gc = (const long long*)h->gbuf[h->cur];
             long long *fn = (long long*)h->fbuf[nxt], *gn = (long long*)h->gbuf[nxt];
-            fixed_fused_step(h->xgeo, h->px, X, h->dim, false, fc, gc, fn, gn, h->stream, 0, h->wide_index);
+            fixed_fused_step(h->xgeo, h->px, X, h->dim, false, fc, gc, fn, gn, h->stream, 0, h->wide_index, h->sms);
             CK(h, cudaEventRecord(ev[2 * k + 1], h->stream));
-            fixed_fused_step(h->xgeo, h->px, X, h->dim, false, fc, gc, fn, gn, h->stream, 1, h->wide_index);
+            fixed_fused_step(h->xgeo, h->px, X, h->dim, false, fc, gc, fn, gn, h->stream, 1, h->wide_index, h->sms);
             h->cur = nxt;
         } else if (h->p.precision == LBM_FP64) {
             const int nxt = h->cur ^ 1;

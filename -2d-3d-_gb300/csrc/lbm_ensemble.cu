@@ -219,7 +219,7 @@ static cudaError_t build_typed(EnsPlan& plan, const std::vector<EnsMemberHost>& 
             }
             m.cur = mh.F->cur;
             const int idx = (int)hm.size();
-            m.tp = tile_plan(m.g, kEnsRows);
+            m.tp = tile_plan(m.g, 64, kEnsRows);
             const long long nt = one_launch(plan, li) ? (long long)m.tp.ntx * m.tp.nty
                                                       : (m.g.ncell + plan.cfg.tile_cells - 1) / plan.cfg.tile_cells;
             for (long long t = 0; t < nt; ++t) tiles.push_back(make_int2(idx, (int)t));

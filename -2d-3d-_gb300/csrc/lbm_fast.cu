@@ -246,7 +246,7 @@ static void duo_step(const Geo& g, const PhysF& pf, const FastArgs<S>& Af, const
 // So: four rows while eight would leave SMs without a block; eight in FP32 while the blocks run at
 // once (four per SM), and where the state does not fit L2 and its traffic counts.
 static int tile_rows(const FastState& F, const Geo& g) {
-    const TilePlan tp = tile_plan(g, 8);
+    const TilePlan tp = tile_plan(g, 64, 8);
     const long long blocks = (long long)tp.ntx * tp.nty;
     if (blocks <= F.sms) return 4;
     const bool large = g.ncell * 136 > F.l2;
@@ -256,7 +256,7 @@ static int tile_rows(const FastState& F, const Geo& g) {
 template <class S>
 static void tile_launch(int rows, const Geo& g, const PhysF& pf, const FastArgs<S>& Af, const FastArgs<S>& At, const S* fin,
                         const S* gin, S* fout, S* gout, int cur, cudaStream_t s) {
-    const TilePlan tp = tile_plan(g, rows);
+    const TilePlan tp = tile_plan(g, 64, rows);
     const unsigned nb = (unsigned)(tp.ntx * tp.nty);
     if (rows == 4) launch_after(k_fast_tile<S, 4>, nb, 128, s, g, pf, tp, Af, At, fin, gin, fout, gout, cur);
     else launch_after(k_fast_tile<S, 8>, nb, 256, s, g, pf, tp, Af, At, fin, gin, fout, gout, cur);

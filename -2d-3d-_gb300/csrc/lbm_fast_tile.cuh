@@ -11,41 +11,20 @@
 #pragma once
 
 #include "lbm_fast_duo.cuh"
+#include "lbm_tile2d.h"
 
 namespace lbm {
 
-// Tiles of a 2D lattice: ntx x nty blocks, each owning up to tw x th cells that begin at (ox, oy)
-// among the block's 64 x (its warps) cells.  An axis that one block covers has no ring, unless it
-// is periodic (the y faces are walls).
-struct TilePlan {
-    int tw, th, ntx, nty, ox, oy;
-};
-__host__ __device__ __forceinline__ bool tile_wraps(const Geo& g) {
-    return g.bcf[0] == LBM_BC_PERIODIC || g.bct[0] == LBM_BCT_PERIODIC;
-}
-inline TilePlan tile_plan(const Geo& g, int rows) {
-    TilePlan t;
-    t.ox = g.nx > 64 || tile_wraps(g) ? 1 : 0;
-    t.oy = g.ny > rows ? 1 : 0;
-    t.tw = 64 - 2 * t.ox;
-    t.th = rows - 2 * t.oy;
-    t.ntx = (g.nx + t.tw - 1) / t.tw;
-    t.nty = (g.ny + t.th - 1) / t.th;
-    return t;
-}
-
-// The two cells of lane `lane` in row `row` of tile `tile`.  at: the first cell's index had the row
-// no end; the second's is at + 32.  A cell beyond the lattice is read as the nearest one, or as
-// the wrapped one across a periodic x face.
+// The two cells of lane `lane` in row `row` of tile `tile` (columns tile_column, tile_line).  Returns
+// the first cell's index had the row no end; the second's is 32 more.
 __host__ __device__ __forceinline__ int tile_cells(const Geo& g, const TilePlan& tp, int tile, int row, int lane, Duo& t) {
     const int ty = tile / tp.ntx, tx = tile - ty * tp.ntx;
     const int y = ty * tp.th + row - tp.oy, x = tx * tp.tw + lane - tp.ox;
-    const int j = y < 0 ? 0 : (y < g.ny ? y : g.ny - 1);
+    const int j = tile_line(g, y);
     const bool mine = row >= tp.oy && row < tp.oy + tp.th && y < g.ny;
     for (int h = 0; h < 2; ++h) {
         const int l = lane + 32 * h, xi = x + 32 * h;
-        const int over = tile_wraps(g) && xi == g.nx ? 0 : g.nx - 1;
-        t.i[h] = xi < 0 ? (tile_wraps(g) ? g.nx - 1 : 0) : (xi < g.nx ? xi : over);
+        t.i[h] = tile_column(g, xi);
         t.j[h] = j;
         t.k[h] = 0;
         t.c[h] = t.i[h] + g.nx * j;
@@ -55,17 +34,6 @@ __host__ __device__ __forceinline__ int tile_cells(const Geo& g, const TilePlan&
     t.inner = j > 0 && j < g.ny - 1 && x0 > 0 && x0 + 63 < g.nx - 1;
     t.rows = false;  // the second cell of an x-face row need not be the first plus 32
     return x + g.nx * j;
-}
-
-// Where an owned cell (i, j) at p of the block's cells pulls direction a from: pull_index's rule,
-// back standing for its own value of the opposite direction.
-template <int Q>
-__host__ __device__ __forceinline__ int tile_pull(const Geo& g, const PullRule& r, int a, int i, int j, int p, bool& back) {
-    const int ex = Lat<Q>::ex(a), ey = Lat<Q>::ey(a);
-    const bool xout = ex != 0 && (ex > 0 ? i == 0 : i == g.nx - 1);
-    const bool yout = ey != 0 && (ey > 0 ? j == 0 : j == g.ny - 1);
-    back = yout || (xout && r.wx);
-    return back ? p : (xout ? p - ex : p - ex - 64 * ey);
 }
 
 #if defined(__CUDACC__)
@@ -134,7 +102,7 @@ __device__ __forceinline__ void tile_step(const Geo& g, const PhysF& P, const Ti
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 bool back;
-                const int p = row * 64 + lane + 32 * h, from = tile_pull<9>(g, r, a, t.i[h], t.j[h], p, back);
+                const int p = row * 64 + lane + 32 * h, from = tile_pull<9, 64>(g, r, a, t.i[h], t.j[h], p, back);
                 v[h] = sf[(back ? Lat<9>::opp(a) - 1 : a - 1) * CAP + (t.in[h] ? from : p)];
             }
             d[a] = make_f2(v[0], v[1]);

@@ -9,6 +9,7 @@
 #include "lbm_fixed.h"
 #include "lbm_fixed_cell.cuh"
 #include "lbm_launch.cuh"
+#include "lbm_tile2d.h"
 
 namespace lbm {
 
@@ -114,6 +115,63 @@ __global__ void __launch_bounds__(128, kXThermalBlocks) k_xthermal_ix(Geo g, Phy
     wait_for_previous();
     if (!in) return;
     thermal_cell<D, false, 4, int>(g, X, A, fin, gin, gout, c, i, j, k, rows);
+    start_next();
+}
+
+// The 2D step of a small lattice in one launch, blocks of four rows of 32 cells (lbm_tile2d.h): the
+// flow collisions of the tile and its ring, then the thermal collisions of the tile from shared
+// memory.  Half of the cells of such a block are its ring, so it serves where the SMs have nothing
+// else to do and the way from one launch to the next is most of a step; the integer arithmetic
+// rules out collisions run twice anywhere else.  GB300, us per step of the two kernels / here:
+// 64x48 3.72 / 2.82, 128x64 4.03 / 3.18; with 64 registers 128x64 3.44, 192x96 3.71 / 4.02, 256x128 4.35 / 4.95,
+// 2050x1025 117 / 161 (eight rows: 128x64 3.53, 256x128 5.00, 2050x1025 122).
+constexpr int kXTileRows = 4;
+
+__global__ void __launch_bounds__(32 * kXTileRows, 4) k_xtile(Geo g, PhysX X, TilePlan tp, FixedArrays A,
+                                                           const long long* fin, const long long* gin, long long* fout,
+                                                           long long* gout, int reverse) {
+    constexpr int CAP = 32 * kXTileRows;
+    __shared__ long long sf[8 * CAP];
+    const int row = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31u), n = (int)g.ncell;
+    const int tile = reverse ? last_first() : (int)blockIdx.x;  // every other step last tile first (L2)
+    const int ty = tile / tp.ntx, tx = tile - ty * tp.ntx;
+    const int x = tx * tp.tw + lane - tp.ox, y = ty * tp.th + row - tp.oy;
+    const int i = tile_column(g, x), j = tile_line(g, y), c = i + g.nx * j;
+    const bool own = lane >= tp.ox && lane < tp.ox + tp.tw && x < g.nx && row >= tp.oy && row < tp.oy + tp.th && y < g.ny;
+    wait_for_previous();
+    q60 d[9], dp[9], e[5], ep[5], rho, P[3], U[3], F, ts = Qb(0);
+    pull_cell<2>(g, fin, gin, c, i, j, 0, j > 0 && j < g.ny - 1, d, e);
+    q60 B[3] = {Qb(A.xb0[c]), Qb(A.xb1[c]), Qb(0)};
+#pragma unroll
+    for (int a = 0; a < 5; ++a) ts = ts + e[a];
+    macro<2>(d, Qb(A.xlag_in[c]), X, rho, P, U, F);
+    const q60 Fy = collide_trt_2d(d, rho, P, U, F, ts, X, dp);
+    if (own) {
+        A.xlag[c] = Fy.s();
+#pragma unroll
+        for (int a = 0; a < 9; ++a) fout[a * n + c] = dp[a].s();
+    }
+#pragma unroll
+    for (int a = 1; a < 9; ++a) sf[(a - 1) * CAP + (int)threadIdx.x] = dp[a].s();
+    __syncthreads();
+    if (own) {
+        const PullRule r = pull_rule<false>(g);
+        d[0] = dp[0];
+#pragma unroll
+        for (int a = 1; a < 9; ++a) {
+            bool back;
+            const int p = tile_pull<9, 32>(g, r, a, i, j, (int)threadIdx.x, back);
+            d[a] = Qb(sf[(back ? Lat<9>::opp(a) - 1 : a - 1) * CAP + p]);
+        }
+        macro<2>(d, Fy, X, rho, P, U, F);
+        collideT_2d(e, U, ts, B, X, ep);
+        if (X.use_g) {
+            A.xb0[c] = B[0].s();
+            A.xb1[c] = B[1].s();
+        }
+#pragma unroll
+        for (int a = 0; a < 5; ++a) gout[a * n + c] = ep[a].s();
+    }
     start_next();
 }
 
@@ -377,10 +435,19 @@ void fixed_fused_pass(const Geo& g, const PhysX& X, const long long* fin, const 
 template <int D>
 static void steady_step(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fprev,
                         const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, bool fl, bool th,
-                        bool wide) {
+                        bool wide, int sms) {
     constexpr int Q = D == 3 ? 19 : 9;
     if (!wide && (long long)Q * g.ncell < (1LL << 31)) {
         const unsigned nb = (unsigned)((g.ncell + 127) / 128);
+        if (D == 2 && fl && th) {
+            const TilePlan tp = tile_plan(g, 32, kXTileRows);
+            const long long blocks = (long long)tp.ntx * tp.nty;
+            if (2 * blocks <= 3 * sms) {
+                launch_after(k_xtile, (unsigned)blocks, 32 * kXTileRows, s, g, X, tp, A, fprev, gprev, fnext, gnext,
+                             fnext < fprev ? 1 : 0);
+                return;
+            }
+        }
         if (fl) launch_after(k_xflow_ix<D>, nb, 128, s, g, X, A, fprev, gprev, fnext);
         if (th) launch_after(k_xthermal_ix<D>, nb, 128, s, g, X, A, fnext, gprev, gnext);
         return;
@@ -402,7 +469,7 @@ static void steady_step(const Geo& g, const PhysX& X, const FixedArrays& A, cons
 }
 
 void fixed_fused_step(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, bool first, const long long* fprev,
-                      const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, int part, bool wide) {
+                      const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, int part, bool wide, int sms) {
     const int bs = 128;
     const unsigned nb = xblocks(g.ncell, bs);
     const bool fl = part != 1, th = part != 0;
@@ -411,14 +478,14 @@ void fixed_fused_step(const Geo& g, const PhysX& X, const FixedArrays& A, int di
             if (fl) k_xflow<2, true><<<nb, bs, 0, s>>>(g, X, A, fprev, gprev, fnext);
             if (th) k_xthermal<2, true><<<nb, bs, 0, s>>>(g, X, A, fnext, gprev, gnext);
         } else {
-            steady_step<2>(g, X, A, fprev, gprev, fnext, gnext, s, fl, th, wide);
+            steady_step<2>(g, X, A, fprev, gprev, fnext, gnext, s, fl, th, wide, sms);
         }
     } else {
         if (first) {
             if (fl) k_xflow<3, true><<<nb, bs, 0, s>>>(g, X, A, fprev, gprev, fnext);
             if (th) k_xthermal<3, true><<<nb, bs, 0, s>>>(g, X, A, fnext, gprev, gnext);
         } else {
-            steady_step<3>(g, X, A, fprev, gprev, fnext, gnext, s, fl, th, wide);
+            steady_step<3>(g, X, A, fprev, gprev, fnext, gnext, s, fl, th, wide, sms);
         }
     }
 }

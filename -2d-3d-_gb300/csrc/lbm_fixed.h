@@ -9,10 +9,10 @@ namespace lbm {
 
 // One fused step (part 0: flow kernel, 1: thermal kernel, 2: both) on q60 fused buffers.
 // first: the inputs are the FP64 module arrays.  g: deviation geometry (deviation_geo).
-// wide: 64-bit cell indices in the interior-row kernels even where 32-bit ones fit.
+// wide: 64-bit cell indices in the interior-row kernels even where 32-bit ones fit.  sms: the device's.
 void fixed_fused_step(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, bool first, const long long* fprev,
-                      const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, int part = 2,
-                      bool wide = false);
+                      const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, int part, bool wide,
+                      int sms);
 // The FP64 module arrays of the current step from the q60 fused buffers and the lag; pops: the
 // populations as well as the scalar fields.
 void fixed_materialize(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, const long long* fcur,

@@ -664,6 +664,7 @@ __device__ __forceinline__ void collideT_2d(const q60* e, const q60* U, q60 tdev
 struct FixedArrays {
     double *f, *g, *rho, *u, *v, *w, *T, *Bx, *By, *Bz, *Tlag, *Fx, *Fy;
     long long *xb0, *xb1, *xb2, *xlag;
+    const long long* xlag_in;  // what the flow half reads, where that is not xlag (2D)
 };
 
 namespace fxa {
@@ -739,7 +740,7 @@ __device__ __forceinline__ void flow_cell(const Geo& g, const PhysX& X, const Fi
             for (int a = 0; a < QT; ++a) ts = ts + pull_thermal<QT, q60>(g, a, i, j, k, c, lg);
         }
         tdev = ts;
-        macro<D>(d, Qb(A.xlag[ci]), X, rho, P, U, F);
+        macro<D>(d, Qb((D == 2 && A.xlag_in ? A.xlag_in : A.xlag)[ci]), X, rho, P, U, F);
     }
     if (D == 2) {
         const q60 Fy = FIRST ? collide_2d(d, rho, P, U, tdev, X, dp) : collide_trt_2d(d, rho, P, U, F, tdev, X, dp);
