@@ -740,10 +740,12 @@ void exact_stage(int stage, const Geo& g, const PhysC& P, const ExactArrays& A, 
     }
 }
 
-// Threads per block of the fused step kernels: 128, or 32 on lattices below 65,536 cells,
-// where 128-thread blocks leave a few blocks per SM and the step waits for the SMs that
-// hold one block more than the others (the FP64 kernels are bound by each SM's FP64 pipe).
-static inline int step_block(const Geo& g) { return g.ncell < 65536 ? 32 : 128; }
+// Threads per block of the fused step kernels: 128, or 32 on lattices below 400,000 cells, where
+// 128-thread blocks leave few blocks per SM and the step waits for the SMs that hold one block
+// more than the others (the FP64 kernels are bound by each SM's FP64 pipe).  GB300, us per step
+// with 128 / 32: 256x128 19.7 / 18.2, 512x256 63.0 / 61.5, 401x777 148.6 / 145.4, 48^3 128.0 / 127.3,
+// 64^3 293.6 both, 128^3 2231 both.
+static inline int step_block(const Geo& g) { return g.ncell < 400000 ? 32 : 128; }
 
 template <int D>
 static void fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, bool first, const double* fprev,
