@@ -72,13 +72,13 @@ struct lbm_handle {
     PhysX px{};
     Geo xgeo{};  // geometry with the thermal wall terms of deviations
     long long *xb0 = nullptr, *xb1 = nullptr, *xb2 = nullptr, *xlag = nullptr;
-    long long* xlag1 = nullptr;  // 2D: the force of the odd buffers (cells around a tile read the old one)
+    long long* xlag1 = nullptr;  // one-launch 2D step: the odd buffers' force (cells around a tile read the old one)
     // fused passes (lbm_fixed.cu k_xfused): B_prev double-buffered, the graph of a chunk of
     // passes and the state it was captured from
     // LBM_OPT_SINGLE_KERNEL on a fixed handle.  Off by default: on GB300 the fused pass reads
     // a third less DRAM but executes about 1.4x the integer instructions (the thermal halo is
-    // recomputed with 64-bit products) and runs at half the two-kernel rate (256^3: 4.08 ms
-    // against 2.14 ms per step).
+    // recomputed with 64-bit products) and runs at well under half the two-kernel rate (256^3:
+    // 4.08 ms per step when measured, against 1.64 ms).
     bool xfused = false;
     long long *xb0b = nullptr, *xb1b = nullptr, *xb2b = nullptr;
     cudaGraph_t xgraph = nullptr;
@@ -392,7 +392,7 @@ static int allocate(lbm_handle* h) {
             AL(h->xb1, n);
             if (d3) AL(h->xb2, n);
             AL(h->xlag, n);
-            if (!d3) AL(h->xlag1, n);
+            if (fixed_one_launch(h->geo, h->dim, h->sms)) AL(h->xlag1, n);
             if (d3 && fixed_fused_supported(h->geo, h->dim)) {
                 AL(h->xb0b, n);
                 AL(h->xb1b, n);
@@ -467,14 +467,15 @@ extern "C" int lbm_create(const lbm_params* p, int device, lbm_handle** out) {
         delete h;
         return LBM_ERR_CUDA;
     }
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) h->sms = sms;
     int st = allocate(h);
     if (st != LBM_OK) {
         release(h);
         delete h;
         return st;
     }
-    int sms = 0, pageable = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) h->sms = sms;
+    int pageable = 0;
     if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess && pageable) {
         // reads of the caller's array by the layout kernels only: writes into freshly
         // allocated host memory fault its pages in from the GPU side, measured at 3-4.5 GB/s
@@ -629,7 +630,7 @@ static FixedArrays fixed_arrays(const lbm_handle* h) {
     X.xb1 = h->xb1;
     X.xb2 = h->xb2;
     X.xlag = h->xlag;
-    if (h->dim == 2) {
+    if (h->xlag1) {
         X.xlag_in = h->cur ? h->xlag1 : h->xlag;
         X.xlag = h->cur ? h->xlag : h->xlag1;
     }
@@ -650,7 +651,7 @@ static int materialize(lbm_handle* h, bool pops) {
     if (!h->fused_valid) return LBM_OK;
     if (h->fixed) {
         FixedArrays X = fixed_arrays(h);
-        if (h->dim == 2) X.xlag = h->cur ? h->xlag1 : h->xlag;  // of the current step
+        if (h->xlag1) X.xlag = h->cur ? h->xlag1 : h->xlag;  // of the current step
         fixed_materialize(h->xgeo, h->px, X, h->dim, (const long long*)h->fbuf[h->cur],
                           (const long long*)h->gbuf[h->cur], pops, h->stream);
         CK_LAUNCH(h, "materialize");
@@ -2141,7 +2142,7 @@ extern "C" int lbm_footprint(const lbm_params* p, size_t* bytes) {
     if (p->precision == LBM_FP64) {
         b += 8 * n * (aa ? q + qt : 3 * q + 3 * qt);         // AA: f, g | f_post A/B, g_post A/B, f, g
         b += 8 * n * (p->dim == 3 ? 16 : 13);                // rho u v T Bx By up vp Tp jx jy (+w Bz wp Tlag jz | Fx Fy)
-        if (p->arith == LBM_ARITH_FIXED) b += 8 * n * (p->dim == 3 ? 4 : 3);  // q60 B_prev and lag
+        if (p->arith == LBM_ARITH_FIXED) b += 8 * n * (p->dim == 3 || n < 16384 ? 4 : 3);  // q60 B_prev and lag
     } else {
         const size_t nb = aa ? 1 : 2;
         b += es * n * (aa ? q + qt : 3 * q + 3 * qt);        // AA: f, g | F A/B, G A/B, f, g (module)

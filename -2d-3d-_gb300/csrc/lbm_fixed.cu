@@ -175,6 +175,11 @@ __global__ void __launch_bounds__(32 * kXTileRows, 4) k_xtile(Geo g, PhysX X, Ti
     start_next();
 }
 
+bool fixed_one_launch(const Geo& g, int dim, int sms) {
+    const TilePlan tp = tile_plan(g, 32, kXTileRows);
+    return dim == 2 && 2LL * tp.ntx * tp.nty <= 3LL * sms;
+}
+
 template <int D>
 __global__ void k_xmaterialize(Geo g, PhysX X, FixedArrays A, const long long* __restrict__ fin,
                                const long long* __restrict__ gin) {
@@ -439,14 +444,11 @@ static void steady_step(const Geo& g, const PhysX& X, const FixedArrays& A, cons
     constexpr int Q = D == 3 ? 19 : 9;
     if (!wide && (long long)Q * g.ncell < (1LL << 31)) {
         const unsigned nb = (unsigned)((g.ncell + 127) / 128);
-        if (D == 2 && fl && th) {
+        if (D == 2 && fl && th && fixed_one_launch(g, D, sms)) {
             const TilePlan tp = tile_plan(g, 32, kXTileRows);
-            const long long blocks = (long long)tp.ntx * tp.nty;
-            if (2 * blocks <= 3 * sms) {
-                launch_after(k_xtile, (unsigned)blocks, 32 * kXTileRows, s, g, X, tp, A, fprev, gprev, fnext, gnext,
-                             fnext < fprev ? 1 : 0);
-                return;
-            }
+            launch_after(k_xtile, (unsigned)(tp.ntx * tp.nty), 32 * kXTileRows, s, g, X, tp, A, fprev, gprev, fnext, gnext,
+                         fnext < fprev ? 1 : 0);
+            return;
         }
         if (fl) launch_after(k_xflow_ix<D>, nb, 128, s, g, X, A, fprev, gprev, fnext);
         if (th) launch_after(k_xthermal_ix<D>, nb, 128, s, g, X, A, fnext, gprev, gnext);

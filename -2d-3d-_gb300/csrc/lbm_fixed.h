@@ -13,6 +13,9 @@ namespace lbm {
 void fixed_fused_step(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, bool first, const long long* fprev,
                       const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, int part, bool wide,
                       int sms);
+// The 2D step of this lattice is one launch with 32-bit indices: at most one and a half blocks per
+// SM (k_xtile; both sides measured there).  A.xlag_in is then not A.xlag.
+bool fixed_one_launch(const Geo& g, int dim, int sms);
 // The FP64 module arrays of the current step from the q60 fused buffers and the lag; pops: the
 // populations as well as the scalar fields.
 void fixed_materialize(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, const long long* fcur,
