@@ -1451,6 +1451,15 @@ static void populate_pages(void* dst, size_t bytes) {
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     const uintptr_t b = ((uintptr_t)dst + page - 1) / page * page, e = ((uintptr_t)dst + bytes) / page * page;
     if (e <= b || e - b < kEach) return;
+    // an array that is in memory already needs nothing (17 MB: 0.11 ms, 0.21 with the threads): look
+    // at a few of its pages
+    int absent = 0;
+    for (int k = 0; k < 8; ++k) {
+        unsigned char in = 0;
+        if (mincore((void*)(b + (e - b - page) / 7 * k / page * page), page, &in) != 0) return;
+        absent += !(in & 1);
+    }
+    if (absent == 0) return;
     const size_t n = std::min<size_t>({4, (e - b) / kEach, std::max(1u, std::thread::hardware_concurrency())});
     const size_t each = ((e - b) / n + page - 1) / page * page;
     auto part = [=](size_t t) {
