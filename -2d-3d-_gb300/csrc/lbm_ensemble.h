@@ -1,9 +1,9 @@
-// lbm_ensemble.h - batched time stepping of many FP32/FP16 lattices in one launch per stage.
+// lbm_ensemble.h - batched time stepping of many FP32/FP16 lattices in one or two launches per step.
 //
 // Members keep their own buffers (each is an ordinary handle); the ensemble builds a
 // device table of member descriptors (geometry, constants, buffer pointers, buffer
 // parity) and a packed tile table (member, first cell) per member list, and advances every
-// member with one flow and one thermal launch per list and step.  Lists: 2D and 3D members
+// member with one flow and one thermal launch per list and step (2D FP32: one launch).  Lists: 2D and 3D members
 // taken two cells per thread with packed arithmetic, and those whose cell indices need 64 bits,
 // taken one cell per thread.
 #pragma once
@@ -24,7 +24,7 @@ struct EnsMemberHost {
 };
 
 struct EnsLaunchCfg {
-    int block = 128;        // threads per block
+    int block = 128;        // threads per block (64-bit indices)
     int tile_cells = 1024;  // cells per tile (a multiple of `block`)
     int grid_mul = 32;      // grid = min(tiles, SMs * grid_mul)
     int pairs = 1;          // kept for callers: every member takes two cells per thread now

@@ -1,10 +1,11 @@
 // lbm_fast.cu - the reduced-storage forms: FP32 or FP16 populations (deviations from the
 // rest state), FP32 arithmetic, FMA contraction allowed.
 //
-// This unit holds the two-kernel step (used for the first step after `initial` or a
-// state load, and to enter the single-kernel mode of lbm_fused.cu), the materialisation
-// of the module arrays, and the conversions to and from the reference's FP64 layout.
-// The moment space is the reference's: the forward transform is its integer matrix
+// This unit holds the steps of the two-buffer pattern (two cells per thread, in 2D also the whole
+// step in one launch; one cell per thread for the first step after `initial` or a state load and
+// for 64-bit indices; rows and pairs on request), the materialisation of the module arrays, and
+// the conversions to and from the reference's FP64 layout.
+// The moment space is the reference's: in the first step the forward transform is its integer matrix
 // applied to the deviations, the relaxation acts on non-equilibrium moments
 // m_k - meq_k = M_k d - (meq_k(rho,u) - meq_k(1,0)), and the inverse transform is its
 // M^-1 with the divisions by constants turned into multiplications.

@@ -41,7 +41,7 @@ struct FastState {
     int cur = 0;
     bool fused_valid = false;   // the fused buffers hold the current state
     bool ahead = false;         // single-kernel phase: F[cur^1] already holds f_post_{N+1}
-    bool single_kernel = false; // one-launch fused step (lbm_fused.cu); off: the two-kernel step is faster today
+    bool single_kernel = false; // marching fused step (lbm_fused.cu); off: the other forms are faster
     int kchunk = 16;            // z planes per block of the fused kernel (3D)
     // Form of the non-first two-kernel step: two cells per thread with packed arithmetic
     // (lbm_fast_duo.cuh; in 2D also one launch, lbm_fast_tile.cuh) where 32-bit indices fit; x-adjacent pairs, staged rows

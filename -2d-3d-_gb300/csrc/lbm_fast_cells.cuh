@@ -1,5 +1,5 @@
-// lbm_fast_cells.cuh - per-cell bodies of the two-kernel FP32/FP16 step, shared by the
-// single-lattice kernels (lbm_fast.cu) and the batched many-lattice kernels
+// lbm_fast_cells.cuh - one-cell bodies of the two-kernel FP32/FP16 step (first step, 64-bit
+// indices, rows), shared by the single-lattice kernels (lbm_fast.cu) and the batched many-lattice kernels
 // (lbm_ensemble.cu), so both run the same arithmetic.
 #pragma once
 
@@ -31,8 +31,7 @@ struct FastArgs {
 
 // Flow collision of step n: f_post_n from f_post_{n-1} (or the module arrays when FIRST).
 // Reads lag_in (3D: T_{n-2}; 2D: F_y,n-1); writes lag_out (2D: F_y,n).  INNER: cells off
-// the lattice's faces pull at fixed offsets without the boundary tests (the batched kernels
-// leave it off: their persistent loops would carry both paths' registers).
+// the lattice's faces pull at fixed offsets without the boundary tests.
 // I: index type of the cell's own accesses and of the fixed-offset pulls (int where every
 // array index fits in 32 bits; the values do not depend on it).
 template <int D, bool FIRST, class S, bool INNER = true, class I = long long>

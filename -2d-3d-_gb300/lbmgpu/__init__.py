@@ -115,8 +115,8 @@ LBM_OPT_KCHUNK = 2
 LBM_OPT_PAIRS = 3
 LBM_OPT_STAGED = 4
 LBM_OPT_FP16_ROUNDING = 5  # FP16 storage: 1 stochastic rounding (default), 0 nearest
-LBM_OPT_WIDE_INDEX = 8     # fixed arithmetic: 64-bit indices in every kernel (1) or 32-bit ones where they fit (0)
-LBM_OPT_ROWS = 7           # FP32/FP16 two-buffer steps: interior-row and face-row launches (1) or one cell per thread
+LBM_OPT_WIDE_INDEX = 8     # 64-bit indices in every kernel (1) or 32-bit ones where they fit (0)
+LBM_OPT_ROWS = 7           # FP32/FP16 two-buffer steps: interior-row and face-row launches (1) or the default forms
 LBM_OPT_HOST_DIRECT = 6    # state transfer on the caller's host arrays: bit 0 set_state reads, bit 1 get_state writes
 
 _lib = None
@@ -379,8 +379,8 @@ class Lattice:
 
 
 class Ensemble:
-    """Many FP32/FP16 lattices advanced together: one flow and one thermal launch per step
-    over a packed tile table of all members (the batched form)."""
+    """Many FP32/FP16 lattices advanced together: one flow and one thermal launch per step (2D
+    FP32: one launch) over a packed tile table of all members (the batched form)."""
 
     def __init__(self, device=0):
         self.lib = load_library()
@@ -426,8 +426,8 @@ class Ensemble:
         return self.launch()
 
     def configure(self, block=128, tile_cells=1024, grid_per_sm=8, pairs=1):
-        """Set the launch configuration (pairs: bit 0 pairs 2D members with even nx, bit 1
-        3D members); the values do not depend on it."""
+        """Set the launch configuration (pairs is kept, without effect); the values do not depend
+        on it."""
         self._ck(self.lib.lbm_ensemble_configure(self._h, int(block), int(tile_cells), int(grid_per_sm), int(pairs)),
                  "lbm_ensemble_configure")
 

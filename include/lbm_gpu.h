@@ -218,11 +218,11 @@ int lbm_RBcalc_Nu_wall_avg(lbm_handle* h, lbm_nu_wall* out);
 int lbm_get_state(lbm_handle* h, int field, double* host, size_t count);
 int lbm_set_state(lbm_handle* h, int field, const double* host, size_t count);
 
-/* ---- batched form: many lattices in one launch per stage (no counterpart in the
+/* ---- batched form: many lattices in one or two launches per step (no counterpart in the
  *      reference, which runs one case per executable) ---------------------------------------
  * An ensemble advances any number of FP32/FP16 handles (one storage precision, any mix of
- * sizes, Ra, Pr, 2D and 3D) with one flow and one thermal launch per step over a packed
- * tile table, replayed from captured CUDA graphs.  Members stay ordinary handles: their
+ * sizes, Ra, Pr, 2D and 3D) with one flow and one thermal launch per step (2D FP32: one
+ * launch) over a packed tile table, replayed from captured CUDA graphs.  Members stay ordinary handles: their
  * diagnostics and state transfer work as usual (the handle's stream waits for the
  * ensemble's work).  A member that is not yet in the fused form (after lbm_initial or
  * lbm_set_state) takes that first step alone at the next lbm_ensemble_step. */
@@ -239,11 +239,12 @@ const char* lbm_ensemble_last_error(const lbm_ensemble* e);
 /* Tile/block autotuner: times `nsteps` steps of each launch configuration and keeps the
  * fastest (members advance by those steps); outputs may be NULL. */
 int lbm_ensemble_autotune(lbm_ensemble* e, int nsteps, int* best_block, int* best_tile, int* best_grid);
-/* Launch configuration of the batched step: threads per block (128 or 256), cells per tile
- * (a positive multiple of the block), grid = min(tiles, SMs x grid_mul) with grid_mul in
- * 1..64, and pairs (bit 0: 2D members with even nx take two x-adjacent cells per thread with
- * 2-element vector loads and stores; bit 1: the same for 3D members).  Every configuration
- * gives the same values bit for bit; lbm_ensemble_autotune picks one by timing.
+/* Launch configuration of the batched step: threads per block (128 or 256; members with
+ * 64-bit indices only, the others take their kernels' own), cells per tile (a positive multiple
+ * of the block; 2D FP32 members have tiles of their own), grid = min(tiles, SMs x grid_mul) with
+ * grid_mul in 1..64, and pairs (0..3; kept, without effect: every member takes two cells per
+ * thread).  Every configuration gives the same values bit for bit; lbm_ensemble_autotune picks
+ * one by timing.
  * LBM_ERR_PARAM for values out of range.  get_launch: outputs may be NULL. */
 int lbm_ensemble_configure(lbm_ensemble* e, int block, int tile_cells, int grid_mul, int pairs);
 int lbm_ensemble_get_launch(const lbm_ensemble* e, int* block, int* tile_cells, int* grid_mul, int* pairs);
@@ -252,8 +253,8 @@ int lbm_ensemble_get_launch(const lbm_ensemble* e, int* block, int* tile_cells, 
 int lbm_footprint(const lbm_params* p, size_t* bytes);
 
 /* ---- execution options (no counterpart in the reference) --------------------------------
- * LBM_OPT_SINGLE_KERNEL: FP32/FP16 handles advance with one fused kernel per step (1) or
- *   with the two-kernel form (0, default, three times faster on GB300).  Both run the same
+ * LBM_OPT_SINGLE_KERNEL: FP32/FP16 handles advance with one marching fused kernel per step (1)
+ *   or with the default forms (0, default, more than three times faster on GB300).  Both run the same
  *   arithmetic; T and the thermal populations agree bit for bit, the flow populations to
  *   their last bits (the collision's multiply-adds may fuse differently).  On a 3D FP64
  *   handle with the fixed arithmetic (nx <= 512) it selects the fused pass, which runs the
@@ -262,15 +263,16 @@ int lbm_footprint(const lbm_params* p, size_t* bytes);
  *   default, faster on GB300); both give the same values bit for bit.
  * LBM_OPT_KCHUNK: z planes marched by one block of the fused 3D kernel (default 16).
  * LBM_OPT_PAIRS: the two-kernel FP32/FP16 step moves populations as 2-cell vectors, two
- *   x-adjacent cells per thread (1; used when nx is even) or one cell per thread (0).
+ *   x-adjacent cells per thread (1; used when nx is even) or takes two cells 32 apart per
+ *   thread, in 2D also in one launch per step (0, default).
  * LBM_OPT_STAGED: the two-kernel FP32/FP16 step stages tiles of x-rows in shared memory
  *   with bulk asynchronous copies (1; used when nx is a multiple of 8; takes precedence
  *   over LBM_OPT_PAIRS) or pulls every value from global memory (0).  A staged kernel
  *   whose bounded wait for its copies gives up sets a device flag: the next lbm_sync or
  *   diagnostic returns LBM_ERR_TIMEOUT.
- * All forms give the same values bit for bit.  Defaults (fastest on GB300): one cell per
- * thread, except two cells per thread for 2D FP32; in the in-place pattern (LBM_PATTERN_AA)
- * the even flow sweep, whose accesses are all the cell's own slots, is always paired when
+ * All forms give the same values bit for bit.  Defaults (fastest on GB300): two cells 32 apart
+ * per thread; in the in-place pattern (LBM_PATTERN_AA) with periodic faces one cell per thread,
+ * but for the even flow sweep, whose accesses are all the cell's own slots: it is paired when
  * nx is even, and the options select the paired or staged form for the other sweeps.
  * LBM_OPT_FP16_ROUNDING: how FP16 storage rounds the new populations of a step.  Stochastic
  *   (1, default): up with probability equal to the dropped fraction, with random bits keyed
@@ -293,15 +295,13 @@ int lbm_footprint(const lbm_params* p, size_t* bytes);
 #define LBM_OPT_HOST_DIRECT   6
 /* LBM_OPT_ROWS: FP32/FP16 two-buffer steps launch interior rows (only x can leave the
  *   lattice there: the x rule by selects, no cell-index division) and face rows (the full
- *   boundary rule) as separate kernels (1), or one cell per thread in lattice order (0).  Two
- *   cells per thread, where chosen, takes precedence.  Same values either way. */
+ *   boundary rule) as separate kernels (1), or the default forms (0).  LBM_OPT_PAIRS, where
+ *   chosen, takes precedence.  Same values either way. */
 #define LBM_OPT_ROWS          7
 /* LBM_OPT_WIDE_INDEX: fixed-arithmetic and FP32/FP16 handles index their arrays with 64-bit
  *   integers in every kernel (1), the form lattices of q * ncell >= 2^31 take, or with 32-bit
- *   indices in the main step kernels (the fixed arithmetic's interior rows, the FP16
- *   one-cell kernels and the FP32 thermal kernel, where they measured faster on GB300) where
- *   every index fits (0, default: half the address arithmetic and 32-bit divisions of the
- *   cell index).  Same values either way. */
+ *   indices where every index fits (0, default: the boundary rules are selects on the index,
+ *   and the FP32/FP16 kernels take two cells per thread).  Same values either way. */
 #define LBM_OPT_WIDE_INDEX    8
 int lbm_set_option(lbm_handle* h, int option, int value);
 
