@@ -32,9 +32,10 @@ struct EnsMember {
     TilePlan tp;  // 2D: its tiles of the one-launch step
 };
 
-// Resident blocks of 128 threads per SM (the launch asks for half of them with 256): six, as the
-// single-lattice duo kernels; the one-cell kernels (64-bit indices) take six as well.
-constexpr int kEnsBlocks = 6;
+// Resident blocks per SM: of 128 threads with two cells each, or of 256 with one (wide: 64-bit
+// indices).  GB300, us per step of 30 members with 5 / 6 / 7 / 8 blocks: 2D FP16 93.5 / 91.9 / 91.4 /
+// 85.8 (10: 94.4), 3D FP32 2492 / 2553 / 2627 / 2778, 3D FP16 2000 / 2049 / 2051 / 2163 (4: 2121).
+constexpr int ens_blocks(int dim, bool wide) { return wide ? 3 : (dim == 2 ? 8 : 5); }
 
 // Cell coordinates of a thread's cells in a tile, stepped instead of divided: one division
 // at the thread's first cell, then (i, j, k) advance by `stride` cells with carries (i by
@@ -93,7 +94,7 @@ __device__ __forceinline__ const EnsStage<S>& stage_member(const EnsMember<S>* _
 // WIDE: one cell per thread with 64-bit indices (members too large for 32-bit ones); otherwise two
 // cells per thread (lbm_fast_duo.cuh), a block taking 2 * blockDim.x cells of its tile at a time.
 template <int D, class S, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEnsBlocks))
+__global__ void __launch_bounds__(WIDE ? 256 : 128, ens_blocks(D, WIDE))
     k_ens_flow(const EnsMember<S>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int tile_cells, int flip) {
     __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];
     wait_for_previous();
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEn
 }
 
 template <int D, class S, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 256 : 128, (WIDE ? kEnsBlocks / 2 : kEnsBlocks))
+__global__ void __launch_bounds__(WIDE ? 256 : 128, ens_blocks(D, WIDE))
     k_ens_thermal(const EnsMember<S>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int tile_cells,
                   int flip) {
     __shared__ __align__(16) unsigned sh[(sizeof(EnsStage<S>) + 3) / 4];

@@ -92,13 +92,14 @@ __global__ void __launch_bounds__(128, (OneCellBlocks<S, true>::value)) k_fast_t
     thermal_cell_2k<D, FIRST, S, true, I>(g, P, A, fin, gin, gout, c, i, j, k);
 }
 
-// Two cells per thread, 32 apart (lbm_fast_duo.cuh): the default of the steady-state step.  Six
-// (flow) and seven (thermal) resident blocks per SM: 80 and 72 registers.  GB300, us per step at
-// 256^3 with 5 / 6 / 7 / 8 blocks of both: FP32 818 / 814 / 814 / 824, FP16 659 / 630 / 642 / 660.
-// Against one cell per thread with branches in its pulls: 256^3 FP32 979 / 810 (6.5 TB/s on 313 B
-// per cell: bound by HBM), FP16 955 / 607; 96^3 FP16 89 / 34; 2D 2050x1025 FP32 75 / 63.
+// Two cells per thread, 32 apart (lbm_fast_duo.cuh): the default of the steady-state step.  Seven
+// resident blocks per SM (72 registers).  GB300, us per step with 5 and 6 / 6 and 7 / 7 and 7 / 8 and
+// 8 blocks of the flow and the thermal kernel: 256^3 FP16 621 / 598 / 589 / 596, FP32 804 / 803 /
+// 803 / 808; 96^3 FP16 34.0 / 33.8 / 33.6 / 34.5.
+// Against one cell per thread with branches in its pulls: 256^3 FP32 979 / 803 (6.5 TB/s on 313 B
+// per cell: bound by HBM), FP16 955 / 589; 96^3 FP16 89 / 34.
 template <int D, class S>
-__global__ void __launch_bounds__(128, 6) k_fast_flow_duo(Geo g, PhysF P, FastArgs<S> A, const S* fin,
+__global__ void __launch_bounds__(128, 7) k_fast_flow_duo(Geo g, PhysF P, FastArgs<S> A, const S* fin,
                                                        const S* gin, S* fout) {
     const Duo t = duo_cells(g, (int)blockIdx.x);
     wait_for_previous();

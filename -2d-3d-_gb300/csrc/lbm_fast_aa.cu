@@ -406,10 +406,11 @@ __global__ void __launch_bounds__(128) k_aa_thermal_p(Geo g, PhysF P, FastArgs<S
     }
 }
 
-// Two cells per thread, 32 apart (lbm_fast_aa_duo.cuh): resident blocks as for the two-buffer
-// kernels (lbm_fast.cu).
+// Two cells per thread, 32 apart (lbm_fast_aa_duo.cuh).  GB300, us per step with 6 / 7 / 8 resident
+// blocks of the flow kernel: 384^3 FP16 2148 / 2130 / 2213, 256^3 FP32 814 / 819 / 856; thermal with
+// 8 instead of 7: 2203 and 827.
 template <int D, class S, bool ODD>
-__global__ void __launch_bounds__(128, 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs<S> A, S* f, const S* gs,
+__global__ void __launch_bounds__(128, sizeof(S) == 2 ? 7 : 6) k_aa_flow_duo(Geo g, PhysF P, FastArgs<S> A, S* f, const S* gs,
                                                      int raw) {
     const Duo t = duo_cells<true>(g, (int)blockIdx.x);
     wait_for_previous();
