@@ -32,8 +32,8 @@ __device__ __forceinline__ void duo_own_set(const Geo& g, const S* f, const Duo&
     decltype(ld_raw(f)) x[2][Q];
 #pragma unroll
     for (int a = 0; a < Q; ++a) {
-        x[0][a] = ld_raw(f + a * n + t.c[0]);
-        x[1][a] = ld_raw(f + a * n + t.c[1]);
+        x[0][a] = ld_raw(cell_ptr<Q>(f, a * n, t.c[0]));
+        x[1][a] = ld_raw(cell_ptr<Q>(f, a * n, t.c[1]));
     }
     PullRule r = pull_rule<TH>(g);
     if (!raw) r.cx = r.cy = false;
@@ -89,12 +89,12 @@ __device__ __forceinline__ void duo_aa_store(const Geo& g, S* f, const Duo& t, c
         for (int w = 0; w < 2; ++w) {
             if (!t.in[w]) continue;
 #pragma unroll
-            for (int a = 0; a < Q; ++a) f[Lat<Q>::opp(a) * n + t.c[w]] = h[w][a];
+            for (int a = 0; a < Q; ++a) *cell_ptr<Q>(f, Lat<Q>::opp(a) * n, t.c[w]) = h[w][a];
         }
     } else if (t.inner) {
 #pragma unroll
         for (int a = 0; a < Q; ++a) {
-            S* p = f + push_index<Q, kInner>(g, n, a, 0, 0, 0, t.c[0]);
+            S* p = cell_ptr<Q>(f, push_index<Q, kInner>(g, n, a, 0, 0, 0, 0), t.c[0]);
             p[0] = h[0][a];
             if (t.in[1]) p[32] = h[1][a];
         }
