@@ -137,14 +137,17 @@ __device__ __forceinline__ q60 mul4(q60 a4, q60 b4) {
 // 1/rho for rho in (1/2, 4): an FP32 reciprocal of the leading bits (24 correct bits), then two
 // steps of Newton's iteration r <- r + r (1 - rho r).  The first needs its residual to 2^-52 only
 // and the second's residual fits 32 bits, so both corrections are single 32 x 32 -> 64-bit
-// products; only rho r of the second step is a full product.
+// products; only rho r of the second step is a full product.  Each factor stays below 2^31 next to
+// rho = 1/2, where r comes up to 2: the seed's conversion saturates at 2 - 2^-30, and the second
+// correction takes r in units of 2^-29.
 __device__ __forceinline__ q60 recip(q60 rho) {
     float x = (float)(int)(rho.s() >> 32) * 0x1p-28f;
     x = x < 0.5f ? 0.5f : (x > 4.0f ? 4.0f : x);
 #ifdef __CUDA_ARCH__
-    const unsigned r0 = __float2uint_rz(__frcp_rn(x) * 0x1p30f);
+    const unsigned r0 = (unsigned)__float2int_rz(__frcp_rn(x) * 0x1p30f);
 #else
-    const unsigned r0 = (unsigned)((1.0f / x) * 0x1p30f);
+    const float seed = (1.0f / x) * 0x1p30f;
+    const unsigned r0 = seed < 0x1p31f ? (unsigned)seed : 0x7FFFFFFFu;
 #endif
     // rho r0 with r0 in units of 2^-30
     const unsigned long long t = (((rho.u >> 32) * r0) << 2) + (((rho.u & 0xFFFFFFFFULL) * r0) >> 30);
@@ -152,7 +155,7 @@ __device__ __forceinline__ q60 recip(q60 rho) {
     const q60 r1 = Qb((long long)((unsigned long long)r0 << 30)) +
                    Qb(((long long)(int)r0 * (long long)(int)(e1.s() >> 8)) >> 22);
     const q60 e2 = Qb(kOne) - mul(rho, r1);
-    return r1 + Qb(((long long)(int)(r1.s() >> 30) * (long long)(int)e2.s()) >> 30);
+    return r1 + Qb(((long long)(int)(r1.s() >> 31) * (long long)(int)e2.s()) >> 29);
 }
 
 __device__ __forceinline__ double quiet_nan() {
