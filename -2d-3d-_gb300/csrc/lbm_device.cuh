@@ -243,6 +243,13 @@ __device__ __forceinline__ T pull_thermal_xrow(const Geo& g, int a, int i, I c, 
     return v;
 }
 
+// Whether 32-bit indices serve every kernel that takes them (pull_index, the two-cell kernels, the
+// tiles), q directions per set: besides the array's own q * ncell values, an index that a select then
+// drops lies up to a plane and a row beyond them, and that of a lane past the lattice up to 63.
+__host__ __device__ __forceinline__ bool narrow_index(const Geo& g, int q) {
+    return q * g.ncell + (g.nz > 1 ? (long long)g.nx * g.ny : 0) + g.nx + 64 < (1LL << 31);
+}
+
 // The lattice's boundary switches as the index rules take them: whether an x (z) face of the set is
 // a wall, and for the thermal set which axes hold constant-temperature walls.
 struct PullRule {

@@ -207,7 +207,7 @@ static cudaError_t build_typed(EnsPlan& plan, const std::vector<EnsMemberHost>& 
         std::vector<EnsMember<S>> hm;
         std::vector<int2> tiles;
         for (const EnsMemberHost& mh : members) {
-            if (mh.dim != dim || ((dim == 3 ? 19LL : 9LL) * mh.geo.ncell >= (1LL << 31) - 64) != wide) continue;
+            if (mh.dim != dim || narrow_index(mh.geo, dim == 3 ? 19 : 9) == wide) continue;
             EnsMember<S> m{};
             m.g = dev_geo(mh.geo, mh.phys);
             m.P = fast_physf(*mh.F, mh.phys);

@@ -753,7 +753,7 @@ static void fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, bool 
     const int bs = step_block(g);
     const unsigned nb = nblocks(g.ncell, bs);
     const bool fl = part != 1, th = part != 0;
-    const bool narrow = (D == 3 ? 19LL : 9LL) * g.ncell < (1LL << 31);
+    const bool narrow = narrow_index(g, D == 3 ? 19 : 9);
     if (first) {
         if (fl) k_flow<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
         if (th) k_thermal<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
@@ -829,7 +829,7 @@ void exact_reconstruct(const Geo& g, const PhysC& P, const ExactArrays& A, int d
 void exact_materialize(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, const double* fcur,
                        const double* gcur, cudaStream_t s) {
     const unsigned nb = nblocks(g.ncell, 128);
-    const bool narrow = (dim == 3 ? 19LL : 9LL) * g.ncell < (1LL << 31);
+    const bool narrow = narrow_index(g, dim == 3 ? 19 : 9);
     if (dim == 2 && narrow) k_materialize<2, true><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
     else if (dim == 2) k_materialize<2, false><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
     else if (narrow) k_materialize<3, true><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);

@@ -488,7 +488,7 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
     const unsigned blocks = nb(g.ncell, 128);
     const bool paired = F.pairs && g.nx % 2 == 0;
     const bool rows = F.rows && !paired && row_launch_supported(g);
-    const bool idx32 = !F.wide && (long long)F.q * g.ncell < (1LL << 31) - 64;
+    const bool idx32 = !F.wide && narrow_index(g, F.q);
     bool ticked = false;  // the step's kernels advance the step counter themselves
     dim3 pgrid, pblock;
     pair_launch(g, pgrid, pblock);
@@ -554,7 +554,7 @@ static void materialize(const FastState& F, const Geo& g, const PhysF& pf, bool 
     const S* gin = (const S*)F.gbuf[F.cur];
     const FastArgs<S> A = args_for<S>(F, F.cur, F.cur, F.cur, F.cur);
     const unsigned n = nb(g.ncell, 128);
-    if ((long long)F.q * g.ncell >= (1LL << 31)) k_fast_materialize<D, S, true, false><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
+    if (!narrow_index(g, F.q)) k_fast_materialize<D, S, true, false><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
     else if (pops) k_fast_materialize<D, S, true, true><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
     else k_fast_materialize<D, S, false, true><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
 }

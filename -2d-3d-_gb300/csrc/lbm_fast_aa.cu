@@ -473,7 +473,7 @@ static bool aa_step_launch(FastState& F, const Geo& g, const PhysF& pf, cudaStre
     // two x-adjacent cells per thread (even nx) and every other sweep one (LBM_OPT_PAIRS /
     // LBM_OPT_STAGED select the paired or staged form for them).
     if (!FIRST && !F.pairs && !F.tma && !F.wide && !any_face(st.face_f) && !any_face(st.face_g) &&
-        (long long)F.q * g.ncell < (1LL << 31) - 64 && (part == 1 ? st.fpar != st.gpar : st.fpar == st.gpar)) {
+        narrow_index(g, F.q) && (part == 1 ? st.fpar != st.gpar : st.fpar == st.gpar)) {
         const unsigned nb2 = (unsigned)((g.ncell + 255) / 256);
         if (part != 1) {
             if (st.fpar) launch_after(k_aa_flow_duo<D, S, true>, nb2, 128, s, g, pf, A, f, gg, raw);
@@ -547,7 +547,7 @@ static void aa_materialize(const FastState& F, const Geo& g, const PhysF& pf, cu
     const int raw = st.graw ? 1 : 0;
     const FastArgs<S> A = aa_args<S>(F);
     const S *f = (const S*)F.fbuf[0], *gg = (const S*)F.gbuf[0];
-    if ((long long)F.q * g.ncell < (1LL << 31))
+    if (narrow_index(g, F.q))
         k_aa_materialize_f<D, S, true><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
     else
         k_aa_materialize_f<D, S, false><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);

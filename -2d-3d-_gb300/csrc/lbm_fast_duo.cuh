@@ -10,7 +10,7 @@
 // The first of the three took index arithmetic out of kernels whose integer pipe was 48% busy
 // (GB300, us per step before / after: FP16 2D 2050x1025 44.7 / 42.7, 256^3 605 / 598, 384^3 in
 // place 2195 / 2145; FP32 is bound by HBM and unchanged; 60 2D FP32 lattices together 262 / 248).
-// 32-bit indices: q * ncell < 2^31 - 64.
+// 32-bit indices: narrow_index.
 #pragma once
 
 #include "lbm_fast_cells.cuh"

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(128) k_xthermal_face(Geo g, PhysX X, FixedArra
 }
 
 // Steady-state step, one cell per thread in lattice order, every boundary rule as selects on the
-// load indices (32-bit: q * ncell < 2^31).  The kernels are bound by HBM: with branches between
+// load indices (32-bit: narrow_index).  The kernels are bound by HBM: with branches between
 // the loads a warp waited for some of them one after the other, and rows at the lattice's faces
 // took a launch of their own.  GB300, us per step against interior and face kernels: 2D 128x64
 // 4.4 / 10.4, 2050x1025 123 / 154; 3D 64^3 27 / 46, 128^3 215 / 259, 161x97x131 214 / 310, 256^3
@@ -441,8 +441,7 @@ template <int D>
 static void steady_step(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fprev,
                         const long long* gprev, long long* fnext, long long* gnext, cudaStream_t s, bool fl, bool th,
                         bool wide, int sms) {
-    constexpr int Q = D == 3 ? 19 : 9;
-    if (!wide && (long long)Q * g.ncell < (1LL << 31)) {
+    if (!wide && narrow_index(g, D == 3 ? 19 : 9)) {
         const unsigned nb = (unsigned)((g.ncell + 127) / 128);
         if (D == 2 && fl && th && fixed_one_launch(g, D, sms)) {
             const TilePlan tp = tile_plan(g, 32, kXTileRows);
@@ -496,7 +495,7 @@ template <int D>
 static void materialize(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fcur, const long long* gcur,
                         bool pops, cudaStream_t s) {
     const unsigned nb = xblocks(g.ncell, 128);
-    if ((D == 3 ? 19LL : 9LL) * g.ncell >= (1LL << 31)) k_xmaterialize<D><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
+    if (!narrow_index(g, D == 3 ? 19 : 9)) k_xmaterialize<D><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
     else if (pops) k_xmaterialize_ix<D, true><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
     else k_xmaterialize_ix<D, false><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
 }
