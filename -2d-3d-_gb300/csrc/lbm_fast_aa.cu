@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(128) k_aa_flow_p(Geo g, PhysF P, FastArgs<S> A
     if (!aa_pair_cell(g, c0, i0, j, k)) return;
     constexpr int Q = (D == 2) ? 9 : 19, QT = (D == 2) ? 5 : 7;
     const long long n = g.ncell;
+    const float2 lag = ld2<float, true>(A.lag_in, c0);  // first, as in aa_flow_cell
     f2 d[Q];
     if (ODD) {
         auto lf = [&](int b, long long cc) { return ldA(f, Lat<Q>::opp(b) * n + cc); };
@@ -336,7 +337,6 @@ __global__ void __launch_bounds__(128) k_aa_flow_p(Geo g, PhysF P, FastArgs<S> A
             ts = vadd(ts, make_f2(e.x, e.y));
         }
     }
-    const float2 lag = ld2<float, true>(A.lag_in, c0);
     const f2 Fy = steady_flow<D>(d, steady_lag<D>(make_f2(lag.x, lag.y), P), ts, P);
     if (D == 2) stf2(A.lag_out, c0, f2_lo(Fy), f2_hi(Fy));
     S h0[Q], h1[Q];
