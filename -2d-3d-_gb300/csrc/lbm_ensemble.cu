@@ -1,12 +1,12 @@
-// lbm_ensemble.cu - one flow launch and one thermal launch per time step (FP32 in 2D: one launch) for
+// lbm_ensemble.cu - one flow launch and one thermal launch per time step (most FP32 in 2D: one launch) for
 // any number of FP32/FP16 lattices of uneven sizes and parameters (the batched form).
 //
 // A grid of about SMs x grid_mul persistent blocks walks a packed tile table: tile t is
 // (member m, first cell c0) and covers tile_cells consecutive cells of member m.  Each
 // block reads the member's descriptor (geometry, relaxation rates, buffer pointers and
 // parity), then runs the same per-cell bodies as the single-lattice two-kernel step
-// (lbm_fast_duo.cuh, or lbm_fast_cells.cuh for members beyond 32-bit indices) on its cells.  Small lattices therefore fill the GPU together instead of one launch
-// each.
+// (lbm_fast_duo.cuh, or lbm_fast_cells.cuh for members beyond 32-bit indices) on its cells.  Small
+// lattices therefore fill the GPU together instead of one launch each.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, ens_blocks(D, WIDE))
 // Rows of a block of the one-launch 2D step.
 constexpr int kEnsRows = 8;
 
-// The 2D members' step in one launch (lbm_fast_tile.cuh).  FP32 only: as for one lattice, half
+// The step of 2D members in one launch (lbm_fast_tile.cuh), those that TileRule picks.  FP32 only: as for one lattice, half
 // storage saves too little traffic to pay for the cells that are collided twice.  GB300, 60 members
 // of up to 1024x512: 179 us a step; 200 steps and the read-out 44.7 ms against 49.5 of two kernels.
 __global__ void __launch_bounds__(32 * kEnsRows, 32 / kEnsRows)
@@ -196,18 +196,43 @@ __global__ void __launch_bounds__(32 * kEnsRows, 32 / kEnsRows)
     start_next();
 }
 
-// Lists whose step is one launch.
-static bool one_launch(const EnsPlan& plan, int li) { return li == 0 && plan.precision == LBM_FP32; }
+// Which 2D FP32 members take the one-launch step: those whose blocks own two fifths of the cells they
+// hold (72% of a wide and tall member's; a member narrower than a block leaves columns idle, one a little
+// wider than a block nearly a whole one), and the others as long as their blocks run in about two
+// waves (four per SM), where the launch that is saved is most of the step.  GB300, us per step of one
+// launch / two, with the share owned: 50 of 124x300 (73%) 49.9 / 59.2, 64 of 48x400 (56%) 38.6 /
+// 39.9, 50 of 66x500 (38%) 66.4 / 54.8, 50 of 33x300 (39%) 21.2 / 16.9, 50 of 8x2000 (9%) 117.6 / 25.3;
+// few blocks: 100 of 70x20 (34%) 8.2 / 12.9, 200 of 10x10 (10%) 4.8 / 6.1.
+struct TileRule {
+    bool sparse = false;  // members that own less take it as well
+    static bool takes_tiles(const EnsMemberHost& mh, int precision) {
+        return mh.dim == 2 && precision == LBM_FP32 && narrow_index(mh.geo, 9);
+    }
+    static long long blocks(const EnsMemberHost& mh) {
+        const TilePlan tp = tile_plan(mh.geo, 64, kEnsRows);
+        return (long long)tp.ntx * tp.nty;
+    }
+    static bool owns_enough(const EnsMemberHost& mh) { return 5 * mh.geo.ncell >= 2 * 64 * kEnsRows * blocks(mh); }
+    TileRule(const std::vector<EnsMemberHost>& members, int precision, int sms) {
+        long long n = 0;
+        for (const EnsMemberHost& mh : members)
+            if (takes_tiles(mh, precision) && !owns_enough(mh)) n += blocks(mh);
+        sparse = n <= 8LL * sms;
+    }
+    int list_of(const EnsMemberHost& mh, int precision) const {
+        if (takes_tiles(mh, precision) && (sparse || owns_enough(mh))) return kEnsTiles;
+        return (mh.dim == 3 ? 1 : 0) + (narrow_index(mh.geo, mh.dim == 3 ? 19 : 9) ? 0 : 2);
+    }
+};
 
 template <class S>
 static cudaError_t build_typed(EnsPlan& plan, const std::vector<EnsMemberHost>& members) {
+    const TileRule rule(members, plan.precision, plan.sms);
     for (int li = 0; li < kEnsLists; ++li) {
-        const int dim = (li & 1) ? 3 : 2;
-        const bool wide = (li & 2) != 0;
         std::vector<EnsMember<S>> hm;
         std::vector<int2> tiles;
         for (const EnsMemberHost& mh : members) {
-            if (mh.dim != dim || narrow_index(mh.geo, dim == 3 ? 19 : 9) == wide) continue;
+            if (rule.list_of(mh, plan.precision) != li) continue;
             EnsMember<S> m{};
             m.g = dev_geo(mh.geo, mh.phys);
             m.P = fast_physf(*mh.F, mh.phys);
@@ -221,7 +246,7 @@ static cudaError_t build_typed(EnsPlan& plan, const std::vector<EnsMemberHost>& 
             m.cur = mh.F->cur;
             const int idx = (int)hm.size();
             m.tp = tile_plan(m.g, 64, kEnsRows);
-            const long long nt = one_launch(plan, li) ? (long long)m.tp.ntx * m.tp.nty
+            const long long nt = li == kEnsTiles ? (long long)m.tp.ntx * m.tp.nty
                                                       : (m.g.ncell + plan.cfg.tile_cells - 1) / plan.cfg.tile_cells;
             for (long long t = 0; t < nt; ++t) tiles.push_back(make_int2(idx, (int)t));
             plan.cells += m.g.ncell;
@@ -287,7 +312,7 @@ static void step_typed(const EnsPlan& plan, int flip, cudaStream_t s) {
     for (int stage = 0; stage < 2; ++stage) {
         for (int li = 0; li < kEnsLists; ++li) {
             if (plan.ntiles[li] == 0) continue;
-            if (one_launch(plan, li)) {
+            if (li == kEnsTiles) {
                 if (stage == 1) continue;
                 const unsigned grid = (unsigned)min(plan.ntiles[li], plan.sms * plan.cfg.grid_mul);
                 launch_after(k_ens_tile, grid, 32 * kEnsRows, s, (const EnsMember<float>*)plan.d_members[li],

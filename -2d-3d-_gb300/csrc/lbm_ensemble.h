@@ -3,9 +3,9 @@
 // Members keep their own buffers (each is an ordinary handle); the ensemble builds a
 // device table of member descriptors (geometry, constants, buffer pointers, buffer
 // parity) and a packed tile table (member, first cell) per member list, and advances every
-// member with one flow and one thermal launch per list and step (2D FP32: one launch).  Lists: 2D and 3D members
-// taken two cells per thread with packed arithmetic, and those whose cell indices need 64 bits,
-// taken one cell per thread.
+// member with one flow and one thermal launch per list and step.  Lists: 2D and 3D members taken two
+// cells per thread with packed arithmetic, those whose cell indices need 64 bits, taken one cell
+// per thread, and the 2D FP32 members whose step is one launch (TileRule, lbm_ensemble.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -30,8 +30,9 @@ struct EnsLaunchCfg {
     int pairs = 1;          // kept for callers: every member takes two cells per thread now
 };
 
-// Member lists of a plan: index (dim == 3) + 2 * wide (64-bit cell indices).
-constexpr int kEnsLists = 4;
+// Member lists of a plan: index (dim == 3) + 2 * wide (64-bit cell indices), and the 2D FP32 members
+// whose step is one launch.
+constexpr int kEnsTiles = 4, kEnsLists = 5;
 
 struct EnsPlan {
     int precision = LBM_FP32;

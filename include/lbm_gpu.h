@@ -221,8 +221,8 @@ int lbm_set_state(lbm_handle* h, int field, const double* host, size_t count);
 /* ---- batched form: many lattices in one or two launches per step (no counterpart in the
  *      reference, which runs one case per executable) ---------------------------------------
  * An ensemble advances any number of FP32/FP16 handles (one storage precision, any mix of
- * sizes, Ra, Pr, 2D and 3D) with one flow and one thermal launch per step (2D FP32: one
- * launch) over a packed tile table, replayed from captured CUDA graphs.  Members stay ordinary handles: their
+ * sizes, Ra, Pr, 2D and 3D) with one flow and one thermal launch per step (most 2D FP32
+ * members: one launch) over a packed tile table, replayed from captured CUDA graphs.  Members stay ordinary handles: their
  * diagnostics and state transfer work as usual (the handle's stream waits for the
  * ensemble's work).  A member that is not yet in the fused form (after lbm_initial or
  * lbm_set_state) takes that first step alone at the next lbm_ensemble_step. */
