@@ -2103,6 +2103,7 @@ extern "C" int lbm_set_option(lbm_handle* h, int option, int value) {
         case LBM_OPT_PAIRS:
             if (h->p.precision == LBM_FP64) return fail(h, LBM_ERR_STATE, "the plain FP64 method has no paired form");
             h->F.pairs = value != 0;
+            h->F.pairs_set = true;
             break;
         case LBM_OPT_WIDE_INDEX:
             if (h->p.precision == LBM_FP64 && !h->fixed)

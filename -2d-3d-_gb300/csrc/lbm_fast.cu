@@ -487,7 +487,11 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
     }
     const unsigned blocks = nb(g.ncell, 128);
     const bool paired = F.pairs && g.nx % 2 == 0;
-    const bool rows = F.rows && !paired && row_launch_supported(g);
+    // 2D FP32 (even nx) runs two cells per thread unless LBM_OPT_PAIRS says no: rows are slower there
+    // (GB300, us per step with rows / x-adjacent pairs / the default forms: 512x256 12.4 / 8.1 / 4.0,
+    // 2048x1024 90.6 / 73.3 / 48.3)
+    const bool two_cells = dim == 2 && F.precision == LBM_FP32 && g.nx % 2 == 0 && !F.pairs_set;
+    const bool rows = F.rows && !paired && !two_cells && row_launch_supported(g);
     const bool idx32 = !F.wide && narrow_index(g, F.q);
     bool ticked = false;  // the step's kernels advance the step counter themselves
     dim3 pgrid, pblock;

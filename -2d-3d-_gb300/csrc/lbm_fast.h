@@ -47,6 +47,7 @@ struct FastState {
     // (lbm_fast_duo.cuh; in 2D also one launch, lbm_fast_tile.cuh) where 32-bit indices fit; x-adjacent pairs, staged rows
     // (lbm_fast_tma.cu) or row launches on request.
     bool pairs = false;
+    bool pairs_set = false;     // LBM_OPT_PAIRS was given
     bool tma = false;
     bool rows = false;          // interior-row and face-row launches (LBM_OPT_ROWS)
     bool wide = false;          // 64-bit cell indices where 32-bit ones fit (LBM_OPT_WIDE_INDEX)

@@ -296,7 +296,8 @@ int lbm_footprint(const lbm_params* p, size_t* bytes);
 /* LBM_OPT_ROWS: FP32/FP16 two-buffer steps launch interior rows (only x can leave the
  *   lattice there: the x rule by selects, no cell-index division) and face rows (the full
  *   boundary rule) as separate kernels (1), or the default forms (0).  LBM_OPT_PAIRS, where
- *   chosen, takes precedence.  Same values either way. */
+ *   chosen, takes precedence, and so do the default forms of 2D FP32 lattices with even nx unless
+ *   LBM_OPT_PAIRS was set to 0.  Same values either way. */
 #define LBM_OPT_ROWS          7
 /* LBM_OPT_WIDE_INDEX: fixed-arithmetic and FP32/FP16 handles index their arrays with 64-bit
  *   integers in every kernel (1), the form lattices of q * ncell >= 2^31 take, or with 32-bit
