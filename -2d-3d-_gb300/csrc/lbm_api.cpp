@@ -118,7 +118,7 @@ struct lbm_handle {
     bool host_access = false;   // the device can
     bool host_direct = false;   // and lbm_set_state reads the caller's array so (LBM_OPT_HOST_DIRECT bit 0)
     bool host_direct_wr = false;  // and lbm_get_state writes it so (bit 1)
-    bool wide_index = false;      // fixed arithmetic: 64-bit cell indices everywhere (LBM_OPT_WIDE_INDEX)
+    bool wide_index = false;      // 64-bit cell indices where 32-bit ones fit (LBM_OPT_WIDE_INDEX; FP32/FP16: F.wide)
 };
 
 // ------------------------------------------------------------------------------------
@@ -653,7 +653,7 @@ static int materialize(lbm_handle* h, bool pops) {
         FixedArrays X = fixed_arrays(h);
         if (h->xlag1) X.xlag = h->cur ? h->xlag1 : h->xlag;  // of the current step
         fixed_materialize(h->xgeo, h->px, X, h->dim, (const long long*)h->fbuf[h->cur],
-                          (const long long*)h->gbuf[h->cur], pops, h->stream);
+                          (const long long*)h->gbuf[h->cur], pops, h->stream, h->wide_index);
         CK_LAUNCH(h, "materialize");
         return LBM_OK;
     }
@@ -663,7 +663,7 @@ static int materialize(lbm_handle* h, bool pops) {
         CK_LAUNCH(h, "materialize");
         return LBM_OK;
     }
-    exact_materialize(h->geo, h->phys, h->A, h->dim, h->fbuf[h->cur], h->gbuf[h->cur], h->stream);
+    exact_materialize(h->geo, h->phys, h->A, h->dim, h->fbuf[h->cur], h->gbuf[h->cur], h->stream, h->wide_index);
     CK_LAUNCH(h, "materialize");
     h->A.fpost = h->fbuf[h->cur];
     h->A.gpost = h->gbuf[h->cur];
@@ -739,7 +739,7 @@ static void enqueue_one(lbm_handle* h, bool first) {
         h->cur = nxt;
     } else if (h->p.precision == LBM_FP64) {
         exact_fused_step(h->geo, h->phys, h->A, h->dim, first, h->fbuf[h->cur], h->gbuf[h->cur], h->fbuf[nxt],
-                         h->gbuf[nxt], h->stream);
+                         h->gbuf[nxt], h->stream, 2, h->wide_index);
         h->cur = nxt;
     } else if (first || !use_single(h)) {
         fast_step(h->F, h->geo, h->phys, h->dim, first, h->stream);
@@ -2036,10 +2036,10 @@ extern "C" int lbm_time_kernels(lbm_handle* h, int64_t nsteps, double* ms_flow, 
         } else if (h->p.precision == LBM_FP64) {
             const int nxt = h->cur ^ 1;
             exact_fused_step(h->geo, h->phys, h->A, h->dim, false, h->fbuf[h->cur], h->gbuf[h->cur], h->fbuf[nxt],
-                             h->gbuf[nxt], h->stream, 0);
+                             h->gbuf[nxt], h->stream, 0, h->wide_index);
             CK(h, cudaEventRecord(ev[2 * k + 1], h->stream));
             exact_fused_step(h->geo, h->phys, h->A, h->dim, false, h->fbuf[h->cur], h->gbuf[h->cur], h->fbuf[nxt],
-                             h->gbuf[nxt], h->stream, 1);
+                             h->gbuf[nxt], h->stream, 1, h->wide_index);
             h->cur = nxt;
         } else if (use_single(h)) {
             // one kernel per step: its time goes to the first slot, the second is empty
@@ -2074,6 +2074,8 @@ extern "C" int lbm_time_kernels(lbm_handle* h, int64_t nsteps, double* ms_flow, 
     return LBM_OK;
 }
 
+static void ens_changed(lbm_ensemble* e);
+
 extern "C" int lbm_set_option(lbm_handle* h, int option, int value) {
     if (!h) return LBM_ERR_PARAM;
     switch (option) {
@@ -2106,10 +2108,9 @@ extern "C" int lbm_set_option(lbm_handle* h, int option, int value) {
             h->F.pairs_set = true;
             break;
         case LBM_OPT_WIDE_INDEX:
-            if (h->p.precision == LBM_FP64 && !h->fixed)
-                return fail(h, LBM_ERR_STATE, "the plain FP64 method indexes with 64-bit integers only");
             h->wide_index = value != 0;  // the captured chunk is dropped below
             h->F.wide = value != 0;
+            if (h->ensemble) ens_changed(h->ensemble);
             break;
         case LBM_OPT_ROWS:
             if (h->p.precision == LBM_FP64) return fail(h, LBM_ERR_STATE, "the FP64 forms choose their own launches");
@@ -2188,6 +2189,9 @@ struct lbm_ensemble {
     cudaGraphExec_t graph_exec = nullptr;
     std::string err;
 };
+
+// A member's launches changed: the plan is built again at the next step.
+static void ens_changed(lbm_ensemble* e) { e->dirty = true; }
 
 static int efail(lbm_ensemble* e, int st, const std::string& m) {
     if (e) e->err = m;

@@ -205,8 +205,9 @@ __global__ void __launch_bounds__(32 * kEnsRows, 32 / kEnsRows)
 // few blocks: 100 of 70x20 (34%) 8.2 / 12.9, 200 of 10x10 (10%) 4.8 / 6.1.
 struct TileRule {
     bool sparse = false;  // members that own less take it as well
+    static bool narrow(const EnsMemberHost& mh) { return !mh.F->wide && narrow_index(mh.geo, mh.dim == 3 ? 19 : 9); }
     static bool takes_tiles(const EnsMemberHost& mh, int precision) {
-        return mh.dim == 2 && precision == LBM_FP32 && narrow_index(mh.geo, 9);
+        return mh.dim == 2 && precision == LBM_FP32 && narrow(mh);
     }
     static long long blocks(const EnsMemberHost& mh) {
         const TilePlan tp = tile_plan(mh.geo, 64, kEnsRows);
@@ -221,7 +222,7 @@ struct TileRule {
     }
     int list_of(const EnsMemberHost& mh, int precision) const {
         if (takes_tiles(mh, precision) && (sparse || owns_enough(mh))) return kEnsTiles;
-        return (mh.dim == 3 ? 1 : 0) + (narrow_index(mh.geo, mh.dim == 3 ? 19 : 9) ? 0 : 2);
+        return (mh.dim == 3 ? 1 : 0) + (narrow(mh) ? 0 : 2);
     }
 };
 

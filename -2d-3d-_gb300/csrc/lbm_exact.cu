@@ -749,11 +749,11 @@ static inline int step_block(const Geo& g) { return g.ncell < 400000 ? 32 : 128;
 
 template <int D>
 static void fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, bool first, const double* fprev,
-                       const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part) {
+                       const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part, bool wide) {
     const int bs = step_block(g);
     const unsigned nb = nblocks(g.ncell, bs);
     const bool fl = part != 1, th = part != 0;
-    const bool narrow = narrow_index(g, D == 3 ? 19 : 9);
+    const bool narrow = !wide && narrow_index(g, D == 3 ? 19 : 9);
     if (first) {
         if (fl) k_flow<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fprev, gprev, fnext);
         if (th) k_thermal<D, true, false><<<nb, bs, 0, s>>>(g, P, A, fnext, gprev, gnext);
@@ -767,9 +767,9 @@ static void fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, bool 
 }
 
 void exact_fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, bool first, const double* fprev,
-                      const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part) {
-    if (dim == 2) fused_step<2>(g, P, A, first, fprev, gprev, fnext, gnext, s, part);
-    else fused_step<3>(g, P, A, first, fprev, gprev, fnext, gnext, s, part);
+                      const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part, bool wide) {
+    if (dim == 2) fused_step<2>(g, P, A, first, fprev, gprev, fnext, gnext, s, part, wide);
+    else fused_step<3>(g, P, A, first, fprev, gprev, fnext, gnext, s, part, wide);
 }
 
 static AAFace<double> aa_faces(void* const face[3]) {
@@ -827,9 +827,9 @@ void exact_reconstruct(const Geo& g, const PhysC& P, const ExactArrays& A, int d
 }
 
 void exact_materialize(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, const double* fcur,
-                       const double* gcur, cudaStream_t s) {
+                       const double* gcur, cudaStream_t s, bool wide) {
     const unsigned nb = nblocks(g.ncell, 128);
-    const bool narrow = narrow_index(g, dim == 3 ? 19 : 9);
+    const bool narrow = !wide && narrow_index(g, dim == 3 ? 19 : 9);
     if (dim == 2 && narrow) k_materialize<2, true><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
     else if (dim == 2) k_materialize<2, false><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);
     else if (narrow) k_materialize<3, true><<<nb, 128, 0, s>>>(g, P, A, fcur, gcur);

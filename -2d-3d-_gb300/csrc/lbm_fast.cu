@@ -558,7 +558,7 @@ static void materialize(const FastState& F, const Geo& g, const PhysF& pf, bool 
     const S* gin = (const S*)F.gbuf[F.cur];
     const FastArgs<S> A = args_for<S>(F, F.cur, F.cur, F.cur, F.cur);
     const unsigned n = nb(g.ncell, 128);
-    if (!narrow_index(g, F.q)) k_fast_materialize<D, S, true, false><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
+    if (F.wide || !narrow_index(g, F.q)) k_fast_materialize<D, S, true, false><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
     else if (pops) k_fast_materialize<D, S, true, true><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
     else k_fast_materialize<D, S, false, true><<<n, 128, 0, s>>>(g, pf, A, fin, gin);
 }

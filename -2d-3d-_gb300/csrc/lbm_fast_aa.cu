@@ -547,7 +547,7 @@ static void aa_materialize(const FastState& F, const Geo& g, const PhysF& pf, cu
     const int raw = st.graw ? 1 : 0;
     const FastArgs<S> A = aa_args<S>(F);
     const S *f = (const S*)F.fbuf[0], *gg = (const S*)F.gbuf[0];
-    if (narrow_index(g, F.q))
+    if (!F.wide && narrow_index(g, F.q))
         k_aa_materialize_f<D, S, true><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);
     else
         k_aa_materialize_f<D, S, false><<<nb, 128, 0, s>>>(g, pf, A, f, gg, st.fpar, st.gpar, raw);

@@ -493,17 +493,17 @@ void fixed_fused_step(const Geo& g, const PhysX& X, const FixedArrays& A, int di
 
 template <int D>
 static void materialize(const Geo& g, const PhysX& X, const FixedArrays& A, const long long* fcur, const long long* gcur,
-                        bool pops, cudaStream_t s) {
+                        bool pops, cudaStream_t s, bool wide) {
     const unsigned nb = xblocks(g.ncell, 128);
-    if (!narrow_index(g, D == 3 ? 19 : 9)) k_xmaterialize<D><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
+    if (wide || !narrow_index(g, D == 3 ? 19 : 9)) k_xmaterialize<D><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
     else if (pops) k_xmaterialize_ix<D, true><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
     else k_xmaterialize_ix<D, false><<<nb, 128, 0, s>>>(g, X, A, fcur, gcur);
 }
 
 void fixed_materialize(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, const long long* fcur,
-                       const long long* gcur, bool pops, cudaStream_t s) {
-    if (dim == 2) materialize<2>(g, X, A, fcur, gcur, pops, s);
-    else materialize<3>(g, X, A, fcur, gcur, pops, s);
+                       const long long* gcur, bool pops, cudaStream_t s, bool wide) {
+    if (dim == 2) materialize<2>(g, X, A, fcur, gcur, pops, s, wide);
+    else materialize<3>(g, X, A, fcur, gcur, pops, s, wide);
 }
 
 void fixed_post_to_double(const PhysX& X, long long* fbuf, long long* gbuf, long long n, int q, int qt,

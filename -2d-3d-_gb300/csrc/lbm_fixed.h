@@ -19,7 +19,7 @@ bool fixed_one_launch(const Geo& g, int dim, int sms);
 // The FP64 module arrays of the current step from the q60 fused buffers and the lag; pops: the
 // populations as well as the scalar fields.
 void fixed_materialize(const Geo& g, const PhysX& X, const FixedArrays& A, int dim, const long long* fcur,
-                       const long long* gcur, bool pops, cudaStream_t s);
+                       const long long* gcur, bool pops, cudaStream_t s, bool wide);
 // Convert the q60 fused buffers in place to the FP64 post-collision populations of the
 // plain method's layout (the handle then continues from its module arrays).
 void fixed_post_to_double(const PhysX& X, long long* fbuf, long long* gbuf, long long n, int q, int qt,

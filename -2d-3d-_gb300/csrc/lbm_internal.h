@@ -156,11 +156,12 @@ void aa_module_view(const Geo& g, int q, bool thermal, int precision, const void
 // ---- exact FP64 kernels (lbm_exact.cu) ------------------------------------------------
 void exact_initial(const Geo& g, const PhysC& P, const InitC& I, const ExactArrays& A, int dim, cudaStream_t s);
 void exact_stage(int stage, const Geo& g, const PhysC& P, const ExactArrays& A, int dim, cudaStream_t s);
-// part: 0 = flow kernel only, 1 = thermal kernel only, 2 = both (one full step)
+// part: 0 = flow kernel only, 1 = thermal kernel only, 2 = both (one full step).  wide: 64-bit indices
+// where 32-bit ones fit.
 void exact_fused_step(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, bool first, const double* fprev,
-                      const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part = 2);
+                      const double* gprev, double* fnext, double* gnext, cudaStream_t s, int part, bool wide);
 void exact_materialize(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, const double* fcur,
-                       const double* gcur, cudaStream_t s);
+                       const double* gcur, cudaStream_t s, bool wide);
 
 // In-place pattern: part 0 = flow sweep, 1 = thermal sweep, 2 = both; flips the parities.
 void exact_aa_step(const Geo& g, const PhysC& P, const ExactArrays& A, int dim, bool first, AAState& S,

@@ -299,8 +299,9 @@ int lbm_footprint(const lbm_params* p, size_t* bytes);
  *   chosen, takes precedence, and so do the default forms of 2D FP32 lattices with even nx unless
  *   LBM_OPT_PAIRS was set to 0.  Same values either way. */
 #define LBM_OPT_ROWS          7
-/* LBM_OPT_WIDE_INDEX: fixed-arithmetic and FP32/FP16 handles index their arrays with 64-bit
- *   integers in every kernel (1), the form lattices of q * ncell >= 2^31 take, or with 32-bit
+/* LBM_OPT_WIDE_INDEX: the handle's arrays are indexed with 64-bit integers in every kernel of the
+ *   step, of the module arrays' rebuild and of the ensemble it is in (1), the form lattices of
+ *   about 2^31 / q cells and more take, or with 32-bit
  *   indices where every index fits (0, default: the boundary rules are selects on the index,
  *   and the FP32/FP16 kernels take two cells per thread).  Same values either way. */
 #define LBM_OPT_WIDE_INDEX    8
