@@ -471,6 +471,21 @@ int fast_take_error(FastState& F, cudaStream_t s) {
     return LBM_ERR_TIMEOUT;
 }
 
+static bool paired_cells(const FastState& F, const Geo& g) { return F.pairs && g.nx % 2 == 0; }
+
+// 2D FP32 (even nx) runs two cells per thread unless LBM_OPT_PAIRS says no: rows are slower there
+// (GB300, us per step with rows / x-adjacent pairs / the default forms: 512x256 12.4 / 8.1 / 4.0,
+// 2048x1024 90.6 / 73.3 / 48.3).
+static bool row_launches(const FastState& F, const Geo& g) {
+    const bool two_cells = F.dim == 2 && F.precision == LBM_FP32 && g.nx % 2 == 0 && !F.pairs_set;
+    return F.rows && !paired_cells(F, g) && !two_cells && row_launch_supported(g);
+}
+
+bool fast_one_launch(const FastState& F, const Geo& g) {
+    return F.dim == 2 && !F.aa && !F.wide && narrow_index(g, F.q) && !paired_cells(F, g) && !row_launches(F, g) &&
+           !(F.tma && fast_tma_supported(g, F.dim, F.precision)) && tile_rows(F, g) != 0;
+}
+
 void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first, cudaStream_t s, int part) {
     const PhysF pf = fast_physf(F, P);
     const Geo g = dev_geo(g0, P);
@@ -486,12 +501,8 @@ void fast_step(FastState& F, const Geo& g0, const PhysC& P, int dim, bool first,
         return;
     }
     const unsigned blocks = nb(g.ncell, 128);
-    const bool paired = F.pairs && g.nx % 2 == 0;
-    // 2D FP32 (even nx) runs two cells per thread unless LBM_OPT_PAIRS says no: rows are slower there
-    // (GB300, us per step with rows / x-adjacent pairs / the default forms: 512x256 12.4 / 8.1 / 4.0,
-    // 2048x1024 90.6 / 73.3 / 48.3)
-    const bool two_cells = dim == 2 && F.precision == LBM_FP32 && g.nx % 2 == 0 && !F.pairs_set;
-    const bool rows = F.rows && !paired && !two_cells && row_launch_supported(g);
+    const bool paired = paired_cells(F, g);
+    const bool rows = row_launches(F, g);
     const bool idx32 = !F.wide && narrow_index(g, F.q);
     bool ticked = false;  // the step's kernels advance the step counter themselves
     dim3 pgrid, pblock;

@@ -71,6 +71,8 @@ void fast_initial(FastState& F, const Geo& g, const PhysC& P, const InitC& I, in
 // Two-kernel step (flow collision, then thermal).  first: read the module arrays.
 // part: 0 = flow kernel only, 1 = thermal kernel only, 2 = both.
 void fast_step(FastState& F, const Geo& g, const PhysC& P, int dim, bool first, cudaStream_t s, int part = 2);
+// Both parts of a steady-state step are one launch (lbm_fast_tile.cuh).
+bool fast_one_launch(const FastState& F, const Geo& g);
 // Single-kernel mode: enter (one flow collision ahead), then one launch per step.
 void fast_enter(FastState& F, const Geo& g, const PhysC& P, int dim, cudaStream_t s);
 void fast_fused_step(FastState& F, const Geo& g, const PhysC& P, int dim, cudaStream_t s);

@@ -324,7 +324,8 @@ class Lattice:
         self._ck(self.lib.lbm_set_option(self._h, int(option), int(value)), "lbm_set_option")
 
     def time_kernels(self, nsteps):
-        """Mean device ms per launch of the (flow, thermal) fused kernels over nsteps steps."""
+        """Mean device ms per launch of the (flow, thermal) fused kernels over nsteps steps; a step
+        that is one launch is all in the first figure."""
         a, b = C.c_double(), C.c_double()
         self._ck(self.lib.lbm_time_kernels(self._h, int(nsteps), C.byref(a), C.byref(b)), "lbm_time_kernels")
         return a.value, b.value

@@ -312,7 +312,9 @@ int lbm_set_option(lbm_handle* h, int option, int value);
 /* The handle's CUDA stream (a cudaStream_t), for callers that record their own events. */
 int lbm_get_stream(lbm_handle* h, void** stream);
 /* Advance nsteps fused steps without graph replay, recording CUDA events around each
- * kernel; returns the mean device time per launch of the flow and thermal kernels. */
+ * kernel; returns the mean device time per launch of the flow and thermal kernels.  Where a step is
+ * one launch (2D lattices whose default form is; LBM_OPT_SINGLE_KERNEL), ms_flow is the whole step's
+ * and ms_thermal 0. */
 int lbm_time_kernels(lbm_handle* h, int64_t nsteps, double* ms_flow, double* ms_thermal);
 /* Self-test (no counterpart in the reference): the plain method divides by the reference's
  * integer constants (x/19, x/2394, ...) with a 3-operation correctly rounded sequence; this
