@@ -12,8 +12,6 @@
 // holds after iteration N, so stepping resumes on the same trajectory).
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
-#include <sys/mman.h>
-#include <unistd.h>
 
 #include <algorithm>
 #include <utility>
@@ -23,7 +21,6 @@
 #include <cstring>
 #include <new>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/lbm_gpu.h"
@@ -31,6 +28,7 @@
 #include "lbm_fast.h"
 #include "lbm_fixed.h"
 #include "lbm_internal.h"
+#include "lbm_pages.h"
 #include "lbm_records.h"
 
 using namespace lbm;
@@ -1442,44 +1440,6 @@ static double* scalar_ptr(lbm_handle* h, int field) {
         case LBM_FIELD_FY: return d3 ? nullptr : A.Fy;
         default: return nullptr;
     }
-}
-
-// Bring the pages of an array that is about to be written whole into memory, with a few threads.
-// A copy into a fresh allocation otherwise takes one page fault after the other (GB300 host: 27
-// GB/s, against 90 GB/s for the copy itself; lbm_get_state into fresh arrays before / after:
-// 134 MB 6.6 / 4.0 ms, 453 MB 19 / 11 ms).
-// Only whole pages inside the array are touched; where the kernel refuses (older kernels, other
-// kinds of memory), the copy faults them as before.
-static void populate_pages(void* dst, size_t bytes) {
-    // bytes a thread takes: below, starting one costs what it saves.  More than four threads wait for
-    // each other in the kernel (453 MB by 1 / 2 / 4 / 8 / 16 threads: 14.0 / 7.6 / 4.9 / 6.8 / 7.9 ms).
-    constexpr size_t kEach = size_t(4) << 20;
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    const uintptr_t b = ((uintptr_t)dst + page - 1) / page * page, e = ((uintptr_t)dst + bytes) / page * page;
-    if (e <= b || e - b < kEach) return;
-    // an array that is in memory already needs nothing (17 MB: 0.11 ms, 0.21 with the threads): look
-    // at a few of its pages
-    int absent = 0;
-    for (int k = 0; k < 8; ++k) {
-        unsigned char in = 0;
-        if (mincore((void*)(b + (e - b - page) / 7 * k / page * page), page, &in) != 0) return;
-        absent += !(in & 1);
-    }
-    if (absent == 0) return;
-    const size_t n = std::min<size_t>({4, (e - b) / kEach, std::max(1u, std::thread::hardware_concurrency())});
-    const size_t each = ((e - b) / n + page - 1) / page * page;
-    auto part = [=](size_t t) {
-        const uintptr_t at = b + t * each;
-        if (at < e) madvise((void*)at, std::min<size_t>(each, e - at), MADV_POPULATE_WRITE);
-    };
-    std::vector<std::thread> others;
-    try {
-        others.reserve(n);
-        for (size_t t = 1; t < n; ++t) others.emplace_back(part, t);
-    } catch (...) {  // no more threads: the pages left over fault in the copy
-    }
-    part(0);
-    for (std::thread& t : others) t.join();
 }
 
 // A device array into the caller's host array, on the handle's stream; the pages are brought in
