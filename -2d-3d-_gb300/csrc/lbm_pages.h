@@ -41,11 +41,12 @@ inline void populate_pages(void* dst, size_t bytes) {
     const uintptr_t b = ((uintptr_t)dst + page - 1) / page * page, e = ((uintptr_t)dst + bytes) / page * page;
     if (e <= b || e - b < kEach) return;
     // an array that is in memory already needs nothing (17 MB: 0.11 ms, 0.21 with the threads): look
-    // at a few of its pages
+    // at its first, middle and last page.  Each look costs such an array about 0.4 us (7 MB without / with
+    // three / with eight: 50.2 / 52.1 / 53.8 us).
     int absent = 0;
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < 3; ++k) {
         unsigned char in = 0;
-        if (mincore((void*)(b + (e - b - page) / 7 * k / page * page), page, &in) != 0) return;
+        if (mincore((void*)(b + (e - b - page) / 2 * k / page * page), page, &in) != 0) return;
         absent += !(in & 1);
     }
     if (absent == 0) return;
