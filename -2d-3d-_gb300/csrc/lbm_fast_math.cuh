@@ -243,9 +243,13 @@ __device__ __forceinline__ f2 vneg(f2 a) {
 template <class V> __device__ __forceinline__ V vfma(float a, V b, V c) { return vfma(vset<V>(a), b, c); }
 template <class V> __device__ __forceinline__ V vmul(float a, V b) { return vmul(vset<V>(a), b); }
 __device__ __forceinline__ float rcp_seed(float x) {
+#if defined(__CUDACC__)
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+#else  // the tests' host build
+    return 1.0f / x;
+#endif
 }
 __device__ __forceinline__ float vrcp_seed(float x) { return rcp_seed(x); }
 __device__ __forceinline__ f2 vrcp_seed(f2 x) { return make_f2(rcp_seed(f2_lo(x)), rcp_seed(f2_hi(x))); }
@@ -366,22 +370,26 @@ __device__ __forceinline__ V steady_flow(V* d, V lag, V ts, const PhysF& P) {
         k[8] = vfma(-P.q12, j[2], jy);
     }
     // The axis pairs' odd parts are what the momentum j + F_y leaves after the diagonals', and the
-    // rest population what the mass leaves: constants that do not sum to one in FP32 would scale
-    // both a little in every step.  The momentum passes through fcollide's own FP32 factor (1/6,
-    // 1/10; 3e-8 and 1.5e-8 from exact), so that long runs stay with those of the moment form.
+    // rest population what the mass leaves.  The half of the momentum is taken as a rounded product
+    // (3D 9 * (1/18)f, 2D 5 * 0.1f) that gains 0.9e-8 (2D 1.8e-8) per step: less than the moment form's
+    // 1.4e-8 to 1.6e-8 (2D 2.8e-8; tests/test_cpu_steady_momentum.py), so velocities are nearer to 64
+    // bits than that form's.  An exact half gains nothing, but puts velocities after 1000 steps up to
+    // 2.9e-5 from those of the moment form's gain; with these they are within 1.2e-5, and FP32 results
+    // are held to 2e-5 from one version to the next.
+    constexpr float kPart = D == 3 ? 1.0f / 18.0f : 0.1f, kTimes = D == 3 ? 9.0f : 5.0f;
 #pragma unroll
     for (int b = 0; b < NP; ++b) E[b] = vfma(P.ce, E[b], g[b]);
 #pragma unroll
     for (int b = D; b < NP; ++b) O[b] = vfma(P.co, O[b], k[b]);
     const V jf = vfma(gr, ts, j[1]);
     if (D == 2) {
-        O[0] = vfma(3.0f, vmul(1.0f / 6.0f, j[0]), vsub(O[3], O[2]));
-        O[1] = vfma(3.0f, vmul(1.0f / 6.0f, jf), vneg(vadd(O[2], O[3])));
+        O[0] = vfma(kTimes, vmul(kPart, j[0]), vsub(O[3], O[2]));
+        O[1] = vfma(kTimes, vmul(kPart, jf), vneg(vadd(O[2], O[3])));
         d[0] = vfma(-2.0f, vadd(vadd(E[0], E[1]), vadd(E[2], E[3])), dr);
     } else {
-        O[0] = vfma(5.0f, vmul(0.1f, j[0]), vadd(vsub(O[4], O[3]), vsub(O[6], O[5])));
-        O[1] = vfma(5.0f, vmul(0.1f, jf), vneg(vadd(vadd(O[3], O[4]), vadd(O[7], O[8]))));
-        O[2] = vfma(5.0f, vmul(0.1f, j[2]), vsub(vsub(O[8], O[7]), vadd(O[5], O[6])));
+        O[0] = vfma(kTimes, vmul(kPart, j[0]), vadd(vsub(O[4], O[3]), vsub(O[6], O[5])));
+        O[1] = vfma(kTimes, vmul(kPart, jf), vneg(vadd(vadd(O[3], O[4]), vadd(O[7], O[8]))));
+        O[2] = vfma(kTimes, vmul(kPart, j[2]), vsub(vsub(O[8], O[7]), vadd(O[5], O[6])));
         d[0] = vfma(-2.0f, vadd(vadd(vadd(vadd(E[0], E[1]), E[2]), vadd(E[3], E[4])), vadd(vadd(E[5], E[6]), vadd(E[7], E[8]))), dr);
     }
 #pragma unroll
