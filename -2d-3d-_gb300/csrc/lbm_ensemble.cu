@@ -169,9 +169,10 @@ __global__ void __launch_bounds__(WIDE ? 256 : 128, ens_blocks(D, WIDE))
 // Rows of a block of the one-launch 2D step.
 constexpr int kEnsRows = 8;
 
-// The step of 2D members in one launch (lbm_fast_tile.cuh), those that TileRule picks.  FP32 only: as for one lattice, half
-// storage saves too little traffic to pay for the cells that are collided twice.  GB300, 60 members
-// of up to 1024x512: 179 us a step; 200 steps and the read-out 44.7 ms against 49.5 of two kernels.
+// The step of 2D members in one launch (lbm_fast_tile.cuh), those that TileRule picks.  FP32 only: as
+// for one lattice, half storage saves too little traffic to pay for the cells that are collided
+// twice.  GB300, 60 members of up to 1024x512: 179 us a step; 200 steps and the read-out 44.7 ms
+// against 49.5 of two kernels.
 __global__ void __launch_bounds__(32 * kEnsRows, 32 / kEnsRows)
     k_ens_tile(const EnsMember<float>* __restrict__ mem, const int2* __restrict__ tiles, int ntiles, int flip) {
     using S = float;
